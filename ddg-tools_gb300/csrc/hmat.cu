@@ -11,7 +11,7 @@
 //
 // Per product (C channels per element: 9 gradient + 3 average per input vector for faces, 3
 // per vector for vertices):
-//   prologue    m = M x per element (FP32), element-major [n][C]
+//   prologue    m = M x per element (float pairs), element-major [n][C], a plane per vector
 //   upward      up[node] = sum_{q in node} a_q m_q, bottom-up (the second child to arrive adds)
 //   far         farx[node] = sum_{b in far(node)} h(node, b) up[b]            (warp per node)
 //   rows        per leaf (warp): near sums over the chain's near blocks with H~a accumulated
@@ -29,6 +29,7 @@
 #include <type_traits>
 #include <vector>
 
+#include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
 #include "block_tree.hpp"
@@ -40,13 +41,16 @@
 namespace rsg {
 
 constexpr int FACE = 0, VERTEX = 1;
-// Which of the two kernels a channel uses: FACE_CH (vector q owns channels 12q..12q+11, the
-// last three of them the averages, kernel 1), VERTEX_CH (kernel 0 throughout), ONES (channel
-// c uses kernel c: the two-channel pass that forms the far part of H~a).
+// Which of the two kernels a channel uses: FACE_CH (12 channels per vector, the last three of
+// them the averages, kernel 1), VERTEX_CH (4 per vector, the last one padding; kernel 0
+// throughout), ONES (channel c uses kernel c: the two-channel pass that forms the far part of
+// H~a from m = 1).
 constexpr int FACE_CH = 0, VERTEX_CH = 1, ONES = 2;
 template <int SEL>
+constexpr int kChannels = SEL == FACE_CH ? 12 : (SEL == VERTEX_CH ? 4 : 2);
+template <int SEL>
 __device__ __forceinline__ bool uses_k1(int c) {
-  return SEL == FACE_CH ? (c % 12) >= 9 : (SEL == ONES ? c == 1 : false);
+  return SEL == FACE_CH ? c >= 9 : (SEL == ONES ? c == 1 : false);
 }
 
 struct HDev {
@@ -62,17 +66,20 @@ struct HDev {
   const double2 *leaf_farA;  // per leaf: far sums of psi = a (k_0, k_1) along its chain, the far part of H~a
   double *leafsum;           // per leaf: C channel far sums along its chain
   const uint32_t *colidx;    // near columns of every leaf's chain, flattened, leaf by leaf
-  const uint4 *items;        // per work item: leaf ordinal, column-range begin / end, weight base
-  const void *wts;           // near weights per item: rows x (columns padded to 32), see NearW
+  const uint4 *items;        // per work item: leaf ordinal, column-range begin / end, weight base (in 8 float2)
+  const float2 *wts;         // near weights per item: [kernel][row pair][column], see hm_weights_kernel
   const uint32_t *item_off;  // per leaf: its work items [item_off[k], item_off[k + 1])
+  const uint32_t *sched;     // work items by the leaf's rows, then most columns first
+  uint32_t sched_off[9];     // those of leaves of i rows: [sched_off[i - 1], sched_off[i])
   double *up;                // per node: C channel sums of a m (FP64)
   float2 *up2;               // the same sums as float pairs (hi, lo), read by the far sums
   double *farx;              // per node: C channel far sums (FP64)
   float2 *part;              // per work item: 8 rows x C near sums as float pairs
   uint32_t *count;           // per node: arrival counter of the upward pass
-  const float2 *m;           // [n][C] channel values as float pairs (hi, lo)
+  const float *m;            // channel values as float pairs: [n] records of 2 C floats, see m_get
   float2 *z;                 // [n][C] results as float pairs
-  int n_nodes, n_leaves, n_el, n_items, n_far_items, C;
+  // (the buffers with C channels hold one such plane per vector, vector by vector)
+  int n_nodes, n_leaves, n_el, n_items, n_far_items;
   float neg_s;               // kernel exponent e applied to r^2: r2^e
   int pw_mode, pw_k;         // e = pw_k / pw_mode for pw_mode 2 or 3 (exact roots), else powf
 };
@@ -84,18 +91,22 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &t) {
   t = (a - (s - bv)) + (b - bv);
 }
 
-// (h, l) += (oh, ol) for float pairs.
-// Layout of the channel values m: per element, C channels as float pairs (hi, lo), stored by
-// channel pairs as (hi_2i, hi_2i+1, lo_2i, lo_2i+1) so that the near field reads the hi parts
-// (and the lo parts) of two channels as one packed operand.
-__device__ __forceinline__ int m_hi(int c) { return (c >> 1) * 4 + (c & 1); }
-__device__ __forceinline__ float2 m_get(const float2 *row, int c) {
-  const float *f = reinterpret_cast<const float *>(row);
-  return make_float2(f[m_hi(c)], f[m_hi(c) + 2]);
+// Layout of the channel values of one element: the hi parts, then the lo parts (12 and 12 floats
+// for faces; 4 and 4, the last of them zero, for vertices).
+template <int SEL>
+__device__ __forceinline__ float2 m_get(const float *f, int c) {
+  if (SEL == ONES) return make_float2(1.f, 0.f);
+  return make_float2(f[c], f[kChannels<SEL> + c]);
 }
-__device__ __forceinline__ void m_set(float2 *row, int c, float2 v) {
-  float *f = reinterpret_cast<float *>(row);
-  f[m_hi(c)] = v.x, f[m_hi(c) + 2] = v.y;
+// the values v[0 .. C) of one element
+template <int C>
+__device__ __forceinline__ void m_store(float *f, const float2 (&v)[C]) {
+  float4 *o = reinterpret_cast<float4 *>(f);
+#pragma unroll
+  for (int i = 0; i < C; i += 4) {
+    o[i / 4] = make_float4(v[i].x, v[i + 1].x, v[i + 2].x, v[i + 3].x);
+    o[(C + i) / 4] = make_float4(v[i].y, v[i + 1].y, v[i + 2].y, v[i + 3].y);
+  }
 }
 
 // Two FP32 values in one 64-bit register (first in the low half) and the packed FP32 pair
@@ -139,6 +150,7 @@ __device__ __forceinline__ float2 to_pair(double v) {
   return make_float2(h, (float)(v - (double)h));
 }
 
+// (h, l) += (oh, ol) for float pairs.
 __device__ __forceinline__ void pair_add(float &h, float &l, float oh, float ol) {
   float s, t;
   two_sum(h, oh, s, t);
@@ -193,55 +205,36 @@ __device__ __forceinline__ void near_kernel(const HDev &d, float d0, float d1, f
 // left + right (fixed order, no waiting). The far field is FP64 end to end (upward, far sums, chain push-down): its sums
 // cancel against m_p H~a for a smooth input just as the near sums do, and at O(nodes) and
 // O(far blocks) work the FP64 rate costs little.
-template <int CC>
+template <int SEL>
 __global__ void hm_upward_kernel(HDev d) {
-  // one warp per leaf, lane l holding channels l, l + 32, ...
-  constexpr int NPL = (CC + 31) / 32;
+  // one warp per leaf and vector, lane l holding channel l
+  constexpr int CC = kChannels<SEL>;
   const int k = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, c = lane;
+  const size_t pn = blockIdx.y * (size_t)d.n_nodes;
   if (k >= d.n_leaves) return;
   const uint32_t leaf = d.leaves[k];
-  double u[NPL];
-#pragma unroll
-  for (int i = 0; i < NPL; ++i) u[i] = 0.0;
-  for (uint32_t p = d.start[leaf]; p < d.end[leaf]; ++p) {
-    const double a = d.xh[p].w;
-    const float2 *mp = d.m + (size_t)p * CC;
-#pragma unroll
-    for (int i = 0; i < NPL; ++i) {
-      const int c = lane + 32 * i;
-      if (c < CC) {
-        const float2 v = m_get(mp, c);
-        u[i] = fma(a, (double)v.x + (double)v.y, u[i]);
-      }
+  double u = 0.0;
+  if (c < CC)
+    for (uint32_t p = d.start[leaf]; p < d.end[leaf]; ++p) {
+      const double a = d.xh[p].w;
+      const float2 v = m_get<SEL>(d.m + (blockIdx.y * (size_t)d.n_el + p) * (2 * CC), c);
+      u = fma(a, (double)v.x + (double)v.y, u);
     }
-  }
-  double *o = d.up + (size_t)leaf * CC;
-  float2 *o2 = d.up2 + (size_t)leaf * CC;
-#pragma unroll
-  for (int i = 0; i < NPL; ++i)
-    if (lane + 32 * i < CC) o[lane + 32 * i] = u[i], o2[lane + 32 * i] = to_pair(u[i]);
+  if (c < CC) d.up[(pn + leaf) * CC + c] = u, d.up2[(pn + leaf) * CC + c] = to_pair(u);
   uint32_t n = leaf;
   while (n != 0) {
     const uint32_t par = d.parent[n];
     __threadfence();  // this warp's sums of n, before the arrival is counted
     __syncwarp();
     unsigned old = 0u;
-    if (lane == 0) old = atomicAdd(&d.count[par], 1u);
+    if (lane == 0) old = atomicAdd(&d.count[pn + par], 1u);
     old = __shfl_sync(0xffffffffu, old, 0);
     if ((old & 1u) == 0u) return;  // first child to arrive: the sibling's warp adds
     __threadfence();
-    const double *l = d.up + (size_t)(par + 1) * CC;
-    const double *r = d.up + (size_t)d.right[par] * CC;
-    double *op = d.up + (size_t)par * CC;
-    float2 *op2 = d.up2 + (size_t)par * CC;
-#pragma unroll
-    for (int i = 0; i < NPL; ++i) {
-      const int c = lane + 32 * i;
-      if (c < CC) {
-        const double v = __ldcg(l + c) + __ldcg(r + c);
-        op[c] = v, op2[c] = to_pair(v);
-      }
+    if (c < CC) {
+      const double v = __ldcg(d.up + (pn + par + 1) * CC + c) + __ldcg(d.up + (pn + d.right[par]) * CC + c);
+      d.up[(pn + par) * CC + c] = v, d.up2[(pn + par) * CC + c] = to_pair(v);
     }
     n = par;
   }
@@ -251,10 +244,10 @@ __global__ void hm_upward_kernel(HDev d) {
 // 564-578) in double-float arithmetic: the coefficients and the node sums are float pairs
 // (about 48 bits), each product is formed exactly to that width (FMA) and added by error-free
 // transformations; the result is handed on in FP64. GB300 issues FP32 at many times its FP64
-// rate. One warp per (node, group of at most twelve channels): lane = sub CG + c holds channel
-// c of the group and takes the node's far blocks sub, sub + 2, ... (sub = 0, 1); the two
-// partial sums are then added. The operations do not depend on the channel count, so the pass
-// over psi = a (two channels) and a product pass add the same terms in the same order.
+// rate. One warp per (item, vector): lane = sub C + c holds channel c and takes the item's far
+// blocks sub, sub + 2, ... (sub = 0, 1); the two partial sums are then added. The operations
+// do not depend on the channel count, so the pass over psi = a (two channels) and a product
+// pass add the same terms in the same order.
 __device__ __forceinline__ void df_fma(float &ah, float &al, float kh, float kl, float uh, float ul) {
   const float ph = kh * uh;
   float pe = fmaf(kh, uh, -ph);
@@ -267,17 +260,15 @@ __device__ __forceinline__ void df_fma(float &ah, float &al, float kh, float kl,
   al = se - (ah - sh);
 }
 
-template <int SEL, int CC>
+template <int SEL>
 __global__ void hm_far_kernel(HDev d) {
-  constexpr int CG = CC < 12 ? CC : 12;
-  static_assert(CC % CG == 0 && 2 * CG <= 32, "channel groups");
-  constexpr int NG = CC / CG;
-  const int wg = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-  const int w = wg / NG, grp = wg - w * NG;
+  constexpr int CC = kChannels<SEL>;
+  static_assert(2 * CC <= 32, "two blocks at a time");
+  const int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
   if (w >= d.n_far_items) return;
   const uint4 it = d.far_items[w];
-  const int lane = threadIdx.x & 31, sub = lane / CG, c = lane - sub * CG;
-  const int ch = grp * CG + c;
+  const int lane = threadIdx.x & 31, sub = lane / CC, ch = lane - sub * CC;
+  const float2 *up2 = d.up2 + blockIdx.y * (size_t)d.n_nodes * CC;
   float ah = 0.f, al = 0.f;
   if (sub < 2) {
     const bool k1 = uses_k1<SEL>(ch);
@@ -289,7 +280,7 @@ __global__ void hm_far_kernel(HDev d) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         kk[i] = d.far_coef[q + 2 * i];
-        u[i] = d.up2[(size_t)d.far_col[q + 2 * i] * CC + ch];
+        u[i] = up2[(size_t)d.far_col[q + 2 * i] * CC + ch];
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -297,13 +288,13 @@ __global__ void hm_far_kernel(HDev d) {
     }
     for (; q < it.z; q += 2) {
       const float4 k = d.far_coef[q];
-      const float2 u = d.up2[(size_t)d.far_col[q] * CC + ch];
+      const float2 u = up2[(size_t)d.far_col[q] * CC + ch];
       df_fma(ah, al, k1 ? k.z : k.x, k1 ? k.w : k.y, u.x, u.y);
     }
   }
-  const float oh = __shfl_down_sync(0xffffffffu, ah, CG), ol = __shfl_down_sync(0xffffffffu, al, CG);
+  const float oh = __shfl_down_sync(0xffffffffu, ah, CC), ol = __shfl_down_sync(0xffffffffu, al, CC);
   pair_add(ah, al, oh, ol);
-  if (sub == 0) d.fpart[(size_t)w * CC + ch] = make_float2(ah, al);
+  if (sub == 0) d.fpart[(blockIdx.y * (size_t)d.n_far_items + w) * CC + ch] = make_float2(ah, al);
 }
 
 // farx[a][c]: the node's item partials added in item order as float pairs, handed on in FP64
@@ -315,11 +306,12 @@ __global__ void hm_far_final_kernel(HDev d) {
   const size_t a = t / CC;
   const int c = (int)(t - a * CC);
   float h = 0.f, l = 0.f;
+  const float2 *fp = d.fpart + blockIdx.y * (size_t)d.n_far_items * CC;
   for (uint32_t i = d.far_item_off[a]; i < d.far_item_off[a + 1]; ++i) {
-    const float2 v = d.fpart[(size_t)i * CC + c];
+    const float2 v = fp[(size_t)i * CC + c];
     pair_add(h, l, v.x, v.y);
   }
-  d.farx[t] = (double)h + (double)l;
+  d.farx[blockIdx.y * (size_t)d.n_nodes * CC + t] = (double)h + (double)l;
 }
 
 // Far coefficients (k_0, k_1) of every far block, FP64, as float pairs (hi, lo): d the centroid
@@ -350,17 +342,53 @@ __global__ void hm_far_coef_kernel(const uint4 *__restrict__ items, int n_items,
   }
 }
 
-// Near weights of an element pair as the rows kernel applies them: faces (w_0, w_1) =
-// a_q (k_0, k_1), vertices w_0 = a_q k_0; zero on the diagonal (q = p). Stored per work item
-// as [row][column], rows padded to a multiple of 32 columns so that each 32-column slice
-// starts on a 128-byte boundary.
-template <int KIND>
-using NearW = typename std::conditional<KIND == FACE, float2, float>::type;
-constexpr int kTileW = 36;          // shared-memory row stride of a weight tile (bank spread)
+// How a warp takes work items of the near field (slices of a leaf's near columns): an item has
+// LPI lanes (column residue j, row group rg, channel group cg), so that a warp takes 32 / LPI
+// items side by side. For a leaf of NS rows the columns fall into G = 32 / NS residue classes,
+// whose sums are kept apart and added in order at the end; lane (j, rg, cg) takes the columns
+// j, j + G, ... for NPL of the leaf's NP = ceil(NS / 2) row pairs and CPL channels. The columns
+// pass through shared memory in tiles of T (a multiple of G).
+// The error-free sums are bound by the FP32 pipe: they take small tiles of registers (more warps);
+// the plain sums by shared-memory reads: larger tiles, fewer bytes per product. Faces take one
+// vector (NV = 1) per warp; vertices, whose vectors have three channels only, all of them.
+template <int KIND, int NS, bool PLAIN, int NV>
+struct NearLanes {
+  static constexpr bool F = KIND == FACE;
+  static constexpr int G = 32 / NS, NP = (NS + 1) / 2;
+  static constexpr int CPL = !F ? 3 * NV : (NS == 1 ? 12 : NS == 2 ? 6 : NS == 3 ? 4 : NS == 6 ? (PLAIN ? 4 : 2) : 3);
+  static constexpr int NCG = F ? 12 / CPL : 1;
+  static constexpr int RG = !F ? NP : (NS >= 7 && !PLAIN ? 2 : 1), NPL = NP / RG;
+  static constexpr int LPI = F && NS >= 6 && PLAIN ? 16 : 32;
+  static constexpr int IPW = 32 / LPI;                 // items per warp
+  static constexpr int T = NS == 1 ? 32 : NS == 3 ? 20 : NS == 5 ? 18
+                         : NS == 6 ? (F && PLAIN ? 10 : 20) : F && NS >= 7 && PLAIN ? 8 : 16;  // columns of a tile
+  static constexpr int K = F ? 2 : 1;                  // kernels
+  // a tile in shared memory: the hi parts of the columns (C floats each), the lo parts, the weight
+  // planes; the offsets keep the lanes of a load (and of a copy) on different banks
+  static constexpr int C = F ? 12 : 4 * NV;
+  static constexpr int LO = T * C + (20 - T * C % 32 + 32) % 32;
+  static constexpr int W = LO + T * C;
+  static constexpr int PLANE = NP * T * 2 + (K == 2 ? (16 - NP * T * 2 % 32 + 32) % 32 : 0);
+  static constexpr int FLOATS = W + K * PLANE;
+  static_assert(T % G == 0 && T % 2 == 0 && T <= 32 && G * RG * NCG <= LPI && NPL * RG == NP, "lane mapping");
+};
+constexpr int kNearStages = 3;  // tiles of a warp in shared memory: one in use, two in flight
+template <int KIND, int NV>
+constexpr int kStageFloats = KIND == FACE ? 960 : 256 * NV + 96;  // of all the items of a warp
 constexpr uint32_t kFarChunk = 64;  // far blocks per far work item
 
+// float2 weights of an item of ns rows and ncol columns, a multiple of 8
 template <int KIND>
-__global__ void hm_weights_kernel(HDev d, size_t total) {
+__host__ __device__ __forceinline__ uint32_t near_weights(uint32_t ns, uint32_t ncol) {
+  return ((KIND == FACE ? 2u : 1u) * ((ns + 1) / 2) * ((ncol + 1) & ~1u) + 7u) & ~7u;
+}
+
+// Near weights of an element pair as the rows kernel applies them: faces (w_0, w_1) =
+// a_q (k_0, k_1), vertices w_0 = a_q k_0; zero on the diagonal (q = p) and in the padding.
+// Stored per work item as planes [kernel][row pair][column] of float2 (the weights of rows 2i
+// and 2i + 1: a packed operand), columns padded to an even number.
+template <int KIND>
+__global__ void hm_weights_kernel(HDev d) {
   // one warp per (item, row); lanes strided over the item's columns
   const size_t wr = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -368,17 +396,17 @@ __global__ void hm_weights_kernel(HDev d, size_t total) {
   const uint32_t w = (uint32_t)(wr >> 3), r = (uint32_t)(wr & 7);
   const uint4 it = d.items[w];
   const uint32_t leaf = d.leaves[it.x];
-  const uint32_t s0 = d.start[leaf], ns = d.end[leaf] - s0;
-  if (r >= ns) return;
-  const uint32_t p = s0 + r, ncol = it.z - it.y, npad = (ncol + 31) & ~31u;
+  const uint32_t s0 = d.start[leaf], ns = d.end[leaf] - s0, np2 = (ns + 1) / 2;
+  if (r >= 2 * np2) return;  // the second row of the last pair may be padding
+  const uint32_t p = s0 + min(r, ns - 1), ncol = it.z - it.y, npad = (ncol + 1) & ~1u;
   const float4 ph = d.xh[p], pl = d.xl[p];
   const float4 np = KIND == FACE ? d.nrm[p] : make_float4(0.f, 0.f, 0.f, 0.f);
-  NearW<KIND> *out = reinterpret_cast<NearW<KIND> *>(const_cast<void *>(d.wts)) + it.w + (size_t)r * npad;
+  float *out = reinterpret_cast<float *>(const_cast<float2 *>(d.wts) + 8 * (size_t)it.w + (size_t)(r >> 1) * npad) + (r & 1);
   for (uint32_t k = lane; k < npad; k += 32) {
     float w0 = 0.f, w1 = 0.f;
     if (k < ncol) {
       const uint32_t q = d.colidx[it.y + k];
-      if (q != p) {
+      if (q != p && r < ns) {
         const float4 qh = d.xh[q], ql = d.xl[q];
         const float d0 = (ph.x - qh.x) + (pl.x - ql.x);
         const float d1 = (ph.y - qh.y) + (pl.y - ql.y);
@@ -388,25 +416,17 @@ __global__ void hm_weights_kernel(HDev d, size_t total) {
         w0 = k0 * qh.w, w1 = k1 * qh.w;
       }
     }
-    if constexpr (KIND == FACE) out[k] = make_float2(w0, w1);
-    else out[k] = w0;
+    out[2 * k] = w0;
+    if (KIND == FACE) out[2 * ((size_t)np2 * npad + k)] = w1;
   }
-  (void)total;
 }
 
-// One tile of a work item in shared memory: the channel values of 32 columns (per channel
-// pair the 16 bytes (hi, hi, lo, lo) of the paired layout), channel pair major (consecutive columns in consecutive 16-byte slots, so that the lanes of a
-// load phase reading up to 8 columns meet no bank twice), and the near weights of up to
-// 8 rows x 32 columns.
-template <int KIND, int CC>
-struct alignas(16) RowsTile {
-  float4 m[CC / 2][32];
-  NearW<KIND> w[8][kTileW];
-};
-
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+// 16 bytes global -> shared, asynchronous, `bytes` (16 or 0) of them read and the rest zero
+__device__ __forceinline__ void cp_async16(unsigned smem, const void *gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(smem), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async16_l2(unsigned smem, const void *gmem, unsigned bytes) {  // not kept in L1
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem), "l"(gmem), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -414,143 +434,225 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// Near sums of one work item (a slice of the flattened near columns of a leaf's root-to-leaf
-// chain) in difference form: sum_q w_pq (m_p - m_q) for channels [c0, c0 + CC) of the row's
-// element p. One warp per item; the leaf's ns rows (3 to 8) each take G = 32 / ns lanes
-// (lane = r G + j), lane j of a row taking every G-th column, so that small leaves keep the
-// warp busy. The weights w_pq were evaluated once per set-up (hm_weights_kernel) and are
-// applied to the CC channels. m_p - m_q is formed exactly from the float pairs (their hi
-// parts share a grid), each product w (m_p - m_q) is split exactly too, and the terms are
-// summed as float pairs: the high parts by error-free additions (two_sum), whose errors gather
-// with the low parts in a second float. (Kahan summation would leave an error of eps times
-// each lane's partial sum, a first-order quantity.) The G partial sums of a row are then added
-// in lane order as float pairs (through shared memory). The columns of an item pass through
-// shared memory in tiles of 32 (channel values and the weights of the tile, copied by cp.async
-// while the previous tile is being used). For a smooth input the terms are first-order
-// quantities that cancel to a second-order result, and the output stage (M^T, a discrete
-// divergence) cancels once more, so plain FP32 sums of H~a m and H~(a m) would lose about
-// four digits.
-template <int KIND, int CC, bool PLAIN>
-__global__ void __launch_bounds__(128, 5) hm_rows_kernel(HDev d, int c0) {
-  static_assert(CC <= 12 && CC % 2 == 0, "at most twelve channels per pass");
-  using WT = NearW<KIND>;
-  constexpr int kChunkW = 16 / (int)sizeof(WT);   // weights per 16-byte copy
-  constexpr int kChunksRow = 32 / kChunkW;         // copies per 32-column weight row
-  // per warp: two tiles (double buffer filled by cp.async); the lane-sum table of the end
-  // reuses the warp's tiles
-  __shared__ RowsTile<KIND, CC> tiles[4][2];
-  static_assert(sizeof(tiles[0]) >= 32 * CC * sizeof(float2), "reduction table fits a warp's tiles");
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (w >= d.n_items) return;
-  const uint4 it = d.items[w];  // leaf ordinal, flat column range [y, z), weight base
-  const uint32_t leaf = d.leaves[it.x];
-  const uint32_t s0 = d.start[leaf], ns = d.end[leaf] - s0;
-  const int G = 32 / (int)ns;
-  const int r = lane / G, j = lane - r * G;
-  const bool act = (uint32_t)r < ns;
-  const uint32_t p = s0 + (act ? r : 0);
-  const int C = d.C;
-  // channel pairs c2: hi parts mh, lo parts ml of the row, sums (ks, kc)
-  f32x2 mh[CC / 2], ml[CC / 2], ks[CC / 2], kc[CC / 2];
-  {
-    const ulonglong2 *mp = reinterpret_cast<const ulonglong2 *>(d.m + (size_t)p * C + c0);
+// N consecutive floats from shared memory (8- or 16-byte aligned when N is even or a multiple of 4)
+template <int N>
+__device__ __forceinline__ void lds_floats(const float *p, float (&v)[N]) {
+  if constexpr (N % 4 == 0) {
 #pragma unroll
-    for (int c2 = 0; c2 < CC / 2; ++c2) {
-      const ulonglong2 v = mp[c2];
-      mh[c2] = v.x, ml[c2] = v.y, ks[c2] = 0ull, kc[c2] = 0ull;
+    for (int i = 0; i < N; i += 4) {
+      const float4 t = *reinterpret_cast<const float4 *>(p + i);
+      v[i] = t.x, v[i + 1] = t.y, v[i + 2] = t.z, v[i + 3] = t.w;
+    }
+  } else if constexpr (N % 2 == 0) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+      const float2 t = *reinterpret_cast<const float2 *>(p + i);
+      v[i] = t.x, v[i + 1] = t.y;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = p[i];
+  }
+}
+
+// Near sums of one work item in difference form: sum_q w_pq (m_p - m_q) for the rows p of the
+// leaf. m_p - m_q is formed exactly from the float pairs (their hi parts share a grid), each
+// product w (m_p - m_q) is split exactly too, and the terms are summed as float pairs: the high
+// parts by error-free additions (two_sum), whose errors gather with the low parts in a second
+// float. (Kahan summation would leave an error of eps times each lane's partial sum, a
+// first-order quantity.) The G residue classes of the columns are then added in order as float
+// pairs. For a smooth input the terms are first-order quantities that cancel to a second-order
+// result, and the output stage (M^T, a discrete divergence) cancels once more, so plain FP32
+// sums of H~a m and H~(a m) would lose about four digits.
+//
+// A lane keeps its rows' values and sums in registers, so that a column's values are read from
+// shared memory once for all the rows it is applied to (with a lane per row the reads of the
+// column values, four wavefronts per 16 bytes of a warp, bounded the kernel). Packed operands
+// run over row pairs, as the stored weights do. The tiles (column records gathered by index,
+// contiguous weights) are copied by cp.async two tiles ahead.
+template <int KIND, int NS, bool PLAIN, int NV>
+__device__ __forceinline__ void rows_items(const HDev &d, float *st, uint32_t w, uint32_t nb) {
+  using L = NearLanes<KIND, NS, PLAIN, NV>;
+  constexpr int CC = KIND == FACE ? 12 : 4, CV = L::C, NP = L::NP, NPL = L::NPL, CPL = L::CPL, T = L::T, LPI = L::LPI, IPW = L::IPW;
+  constexpr int F4 = CV / 2;  // 16-byte parts of a column record (of all its vectors)
+  constexpr int CHM = (T * F4 + LPI - 1) / LPI, CHW = (L::K * NP * T / 2 + LPI - 1) / LPI;
+  constexpr int SF = IPW == 1 ? kStageFloats<KIND, NV> : kStageFloats<KIND, NV> / IPW / 32 * 32 - 16;  // floats of an item's tile
+  static_assert(L::FLOATS <= SF, "the tile fits");
+  // warp w of the leaves of NS rows: items [IPW p, IPW p + IPW) of them in d.sched, vector q (of nb
+  // passes); the vectors of an item in consecutive warps, so that its weights come from DRAM once
+  const uint32_t p = w / nb, q = w - p * nb;
+  const int wl = threadIdx.x & 31, sub = wl / LPI, lane = wl - sub * LPI;
+  const uint32_t pos = d.sched_off[NS - 1] + p * IPW + sub;
+  const bool have = pos < d.sched_off[NS];
+  const uint32_t item = d.sched[have ? pos : d.sched_off[NS] - 1];
+  const uint4 it = d.items[item];  // leaf ordinal, flat column range [y, z), weight base
+  const uint32_t s0 = d.start[d.leaves[it.x]];
+  const uint32_t ncol = it.z - it.y, npad = (ncol + 1) & ~1u;
+  const uint32_t *ci = d.colidx + it.y;
+  const float2 *wg = d.wts + 8 * (size_t)it.w;
+  if (q == 0 && lane == 0 && have && ncol > 0)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(wg),
+                 "r"(near_weights<KIND>(NS, ncol) * (uint32_t)sizeof(float2))
+                 : "memory");
+  const float *m = d.m + (size_t)q * d.n_el * (2 * CC);
+  st += sub * SF;
+  const bool act = lane < L::G * L::RG * L::NCG;
+  const int la = act ? lane : 0, cg = la % L::NCG, rg = (la / L::NCG) % L::RG, j = la / (L::NCG * L::RG);
+  f32x2 mh[NPL][CPL], ml[NPL][CPL], ks[NPL][CPL], kc[NPL][CPL];
+  const size_t plane = (size_t)d.n_el * (2 * CC);  // from vector to vector (vertices)
+#pragma unroll
+  for (int i = 0; i < NPL; ++i) {
+    const int r0 = 2 * (rg * NPL + i), r1 = min(r0 + 1, NS - 1);
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) {
+      const float *u = m + (size_t)(s0 + r0) * (2 * CC) + (KIND == FACE ? cg * CPL + c : c / 3 * plane + c % 3);
+      const float *v = m + (size_t)(s0 + r1) * (2 * CC) + (KIND == FACE ? cg * CPL + c : c / 3 * plane + c % 3);
+      mh[i][c] = f2_pack(u[0], v[0]), ml[i][c] = f2_pack(u[CC], v[CC]);
+      ks[i][c] = kc[i][c] = 0ull;
     }
   }
-  const uint32_t ncol = it.z - it.y, ntiles = (ncol + 31) / 32, npad = ntiles * 32;
-  const WT *wg = reinterpret_cast<const WT *>(d.wts) + it.w;
-  // lane l copies the channel values of column t0 + l and its share of the weight rows
-  auto stage = [&](int buf, uint32_t t0) {
-    RowsTile<KIND, CC> &tl = tiles[wib][buf];
-    if ((uint32_t)lane < ncol - t0) {
-      const uint32_t q = d.colidx[it.y + t0 + lane];
-      const float4 *mq = reinterpret_cast<const float4 *>(d.m + (size_t)q * C + c0);
+  // tiles of the item, and of the longest item of the warp (the others add zero-weight columns)
+  const uint32_t nt = (ncol + T - 1) / T;
+  uint32_t ntw = nt;
 #pragma unroll
-      for (int c2 = 0; c2 < CC / 2; ++c2) cp_async16(&tl.m[c2][lane], mq + c2);
-    }
+  for (int o = LPI; o < 32; o <<= 1) ntw = max(ntw, __shfl_xor_sync(0xffffffffu, ntw, o));
+  // the columns of tile t by lane (past the end the last column, with zero weights)
+  auto index = [&](uint32_t t) { return ncol > 0 ? __ldg(ci + min(t * T + lane, ncol - 1)) : s0; };
+  auto stage = [&](uint32_t t, uint32_t x) {
+    if (t < ntw) {
+      float *sg = st + (t % kNearStages) * kStageFloats<KIND, NV>;
+      const unsigned sm = (unsigned)__cvta_generic_to_shared(sg), sw = sm + 4 * L::W;
 #pragma unroll
-    for (int i = 0; i < 8 * kChunksRow / 32; ++i) {
-      const int id = lane + 32 * i, row = id / kChunksRow, ch = id - row * kChunksRow;
-      if ((uint32_t)row < ns) cp_async16(&tl.w[row][ch * kChunkW], wg + (size_t)row * npad + t0 + ch * kChunkW);
+      for (int i = 0; i < CHM; ++i) {
+        const int c = lane + LPI * i, col = c / F4, part4 = c - col * F4;
+        const uint32_t qc = __shfl_sync(0xffffffffu, x, col, LPI);
+        if (T * F4 % LPI == 0 || c < T * F4)
+          // faces: three parts of hi, three of lo; vertices: (hi, lo) of every vector
+          if constexpr (KIND == FACE)
+            cp_async16(sm + 4 * (col * CV + 4 * part4 + (part4 >= 3 ? L::LO - CV : 0)), m + (size_t)qc * 24 + 4 * part4);
+          else
+            cp_async16(sm + 4 * (col * CV + 4 * (part4 >> 1) + (part4 & 1 ? L::LO : 0)),
+                       m + (part4 >> 1) * plane + (size_t)qc * 8 + 4 * (part4 & 1));
+      }
+#pragma unroll
+      for (int i = 0; i < CHW; ++i) {
+        const int c = lane + LPI * i, row = c / (T / 2);
+        const uint32_t k = t * T + 2 * (c - row * (T / 2));
+        if (L::K * NP * T / 2 % LPI == 0 || c < L::K * NP * T / 2)
+          cp_async16_l2(sw + 16 * c + (L::K == 2 && row >= NP ? 4 * (L::PLANE - NP * T * 2) : 0), wg + (k < npad ? (size_t)row * npad + k : 0), k < npad ? 16u : 0u);
+      }
     }
-    cp_async_commit();
+    cp_async_commit();  // one group per tile, empty past the end
   };
-  if (ntiles > 0) stage(0, 0);
-  for (uint32_t ti = 0; ti < ntiles; ++ti) {
-    const int buf = ti & 1;
-    if (ti + 1 < ntiles) {
-      stage(buf ^ 1, (ti + 1) * 32);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncwarp();
-    const uint32_t t0 = ti * 32, nt = min(32u, ncol - t0);
-    const RowsTile<KIND, CC> &tl = tiles[wib][buf];
-    // lane j of a row takes the item's columns j, j + G, ... (in order): here the local
-    // indices k with (t0 + k) = j mod G
-    if (act)
-      for (uint32_t k = ((uint32_t)j + (uint32_t)G - t0 % (uint32_t)G) % (uint32_t)G; k < nt; k += G) {
-        // packed weights of the channel pairs: (w0, w0), (w0, w1) (the pair of channels 8, 9),
-        // (w1, w1), and their negatives
-        f32x2 W[3];
-        if constexpr (KIND == FACE) {
-          const f32x2 ww = *reinterpret_cast<const f32x2 *>(&tl.w[r][k]);
-          const float2 wf = f2_unpack(ww);
-          W[0] = f2_pack(wf.x, wf.x), W[1] = ww, W[2] = f2_pack(wf.y, wf.y);
-        } else {
-          const float w0 = tl.w[r][k];
-          W[0] = W[1] = W[2] = f2_pack(w0, w0);
-        }
 #pragma unroll
-        for (int c2 = 0; c2 < CC / 2; ++c2) {
-          const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(&tl.m[c2][k]);  // (hi pair, lo pair)
-          const int wi = KIND == FACE ? (2 * c2 + 1 < 9 ? 0 : (2 * c2 >= 9 ? 2 : 1)) : 0;
+  for (int t = 0; t < kNearStages - 1; ++t) stage(t, index(t));
+  uint32_t qn = index(kNearStages - 1);
+  // the planes of the first and of the last channel of the lane: channels below kTh use the first
+  constexpr int kTh = KIND == VERTEX ? CPL : CPL == 12 ? 9 : CPL == 6 ? 3 : CPL == 3 ? 3 : 1;
+  const int wa = rg * NPL * T + (KIND == FACE && cg * CPL >= 9 ? L::PLANE / 2 : 0);
+  const int wb = rg * NPL * T + (KIND == FACE && cg * CPL + CPL > 9 ? L::PLANE / 2 : 0);
+  for (uint32_t t = 0; t < ntw; ++t) {
+    cp_async_wait<kNearStages - 2>();
+    __syncwarp();  // tile t is there for every lane, tile t - 1 done with by every lane
+    stage(t + kNearStages - 1, qn);
+    qn = index(t + kNearStages);
+    const float *sg = st + (t % kNearStages) * kStageFloats<KIND, NV>;
+    const f32x2 *sw = reinterpret_cast<const f32x2 *>(sg + L::W);
+#pragma unroll 2
+    for (int k0 = 0; k0 < T; k0 += L::G) {
+      const int k = k0 + j;
+      constexpr int CR = KIND == FACE ? CPL : CV;
+      float vh[CR], vl[CR];
+      lds_floats<CR>(sg + k * CV + cg * CPL, vh);
+      lds_floats<CR>(sg + L::LO + k * CV + cg * CPL, vl);
+      f32x2 qh[CPL], ql[CPL];
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        const int x = KIND == FACE ? c : c / 3 * 4 + c % 3;
+        qh[c] = f2_pack(vh[x], vh[x]), ql[c] = f2_pack(vl[x], vl[x]);
+      }
+#pragma unroll
+      for (int i = 0; i < NPL; ++i) {
+        const f32x2 w0 = sw[wa + i * T + k], w1 = kTh >= CPL ? w0 : sw[wb + i * T + k];
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+          const f32x2 w = c < kTh ? w0 : w1;
+          // dh = mh_p - mh_q is exact (the hi parts share a grid)
+          const f32x2 dh = f2_sub(mh[i][c], qh[c]), dl = f2_sub(ml[i][c], ql[c]);
           if constexpr (PLAIN) {
             // the inner operator: w (m_p - m_q) from the same exact differences, summed in plain
             // FP32 (no error-free transformations)
-            const f32x2 t = f2_add(f2_sub(mh[c2], v.x), f2_sub(ml[c2], v.y));
-            ks[c2] = f2_fma(W[wi], t, ks[c2]);
+            ks[i][c] = f2_fma(w, f2_add(dh, dl), ks[i][c]);
             continue;
           }
-          const f32x2 w = W[wi], wn = W[wi] ^ kF2Sign;
-          // w (m_p - m_q) = pr + pe + w dl up to eps^2 terms: dh = mh_p - mh_q is exact (the
-          // hi parts share a grid), dl = ml_p - ml_q, w dh = pr + pe (FMA), so no rounding that
-          // depends on the input reaches the sum above eps^2. npr = -pr (exact); the
-          // error-free sum ks + pr = s + err: bb = s - ks, err = (ks - (s - bb)) + (pr - bb).
-          const f32x2 dh = f2_sub(mh[c2], v.x);
-          const f32x2 dl = f2_sub(ml[c2], v.y);
-          const f32x2 npr = f2_mul(wn, dh);
+          // w (m_p - m_q) = pr + pe + w dl up to eps^2 terms: w dh = pr + pe (FMA), so no
+          // rounding that depends on the input reaches the sum above eps^2. npr = -pr (exact);
+          // the error-free sum ks + pr = s + err: bb = s - ks, err = (ks - (s - bb)) + (pr - bb).
+          const f32x2 npr = f2_mul(w ^ kF2Sign, dh);
           const f32x2 lo = f2_fma(w, dl, f2_fma(w, dh, npr));
-          const f32x2 sn = f2_sub(ks[c2], npr);
-          const f32x2 bb = f2_sub(sn, ks[c2]);
-          const f32x2 err = f2_sub(f2_sub(ks[c2], f2_sub(sn, bb)), f2_add(npr, bb));
-          ks[c2] = sn;
-          kc[c2] = f2_add(kc[c2], f2_add(err, lo));
+          const f32x2 sn = f2_sub(ks[i][c], npr);
+          const f32x2 bb = f2_sub(sn, ks[i][c]);
+          const f32x2 err = f2_sub(f2_sub(ks[i][c], f2_sub(sn, bb)), f2_add(npr, bb));
+          ks[i][c] = sn;
+          kc[i][c] = f2_add(kc[i][c], f2_add(err, lo));
         }
       }
-    __syncwarp();
+    }
   }
-  // the G lanes of a row: partial sums (s, t) added in lane order as float pairs
-  float2(*red)[CC] = reinterpret_cast<float2(*)[CC]>(&tiles[wib][0]);
-#pragma unroll
-  for (int c2 = 0; c2 < CC / 2; ++c2) {
-    const float2 s2 = f2_unpack(ks[c2]), k2 = f2_unpack(kc[c2]);
-    red[lane][2 * c2] = make_float2(s2.x, k2.x), red[lane][2 * c2 + 1] = make_float2(s2.y, k2.y);
-  }
+  // the G residue classes of a row added in order as float pairs, through shared memory
+  constexpr int CO = KIND == FACE ? 12 : 3 * NV;  // channels written
+  static_assert(L::G * NS * CO * 2 * IPW <= kNearStages * kStageFloats<KIND, NV>, "the sums fit the warp's tiles");
+  cp_async_wait<0>();
   __syncwarp();
-  if (!act || j != 0) return;
-  float2 *o = d.part + ((size_t)w * 8 + r) * C + c0;
+  float2 *red = reinterpret_cast<float2 *>(st - sub * SF) + sub * (L::G * NS * CO);
+  if (act)
 #pragma unroll
-  for (int c = 0; c < CC; ++c) {
-    float h = red[lane][c].x, l = red[lane][c].y;
-    for (int g = 1; g < G; ++g) pair_add(h, l, red[lane + g][c].x, red[lane + g][c].y);
-    o[c] = make_float2(h, l);
-  }
+    for (int i = 0; i < NPL; ++i)
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        const int r = 2 * (rg * NPL + i), o = (j * NS + r) * CO + cg * CPL + c;
+        const float2 s2 = f2_unpack(ks[i][c]), k2 = f2_unpack(kc[i][c]);
+        red[o] = make_float2(s2.x, k2.x);
+        if (r + 1 < NS) red[o + CO] = make_float2(s2.y, k2.y);
+      }
+  __syncwarp();
+  float2 *part = d.part + ((size_t)q * d.n_items + item) * 8 * CC;
+  if (have)
+#pragma unroll 2
+    for (int o = lane; o < NS * CO; o += LPI) {
+      float2 v = red[o];
+#pragma unroll
+      for (int g = 1; g < L::G; ++g) {
+        const float2 u = red[g * NS * CO + o];
+        pair_add(v.x, v.y, u.x, u.y);
+      }
+      if constexpr (KIND == FACE) {
+        part[o] = v;
+      } else {
+        const int r = o / CO, c = o - r * CO;
+        part[(size_t)(c / 3) * d.n_items * 8 * CC + r * CC + c % 3] = v;
+      }
+    }
+}
+
+// Warps [warps[i + 1], warps[i]) take the items of the leaves of i rows (warps[9] = 0).
+struct RowsGrid {
+  uint32_t warps[10];
+};
+template <int KIND, bool PLAIN, int NV>
+__global__ void __launch_bounds__(128, 4) hm_rows_kernel(HDev d, RowsGrid gr, uint32_t nb) {
+  __shared__ __align__(16) float stages[4][kNearStages * kStageFloats<KIND, NV>];
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  float *st = stages[threadIdx.x >> 5];
+  // longest first: the leaves of 8 rows have the lowest blocks
+  if (w < gr.warps[8]) rows_items<KIND, 8, PLAIN, NV>(d, st, w, nb);
+  else if (w < gr.warps[7]) rows_items<KIND, 7, PLAIN, NV>(d, st, w - gr.warps[8], nb);
+  else if (w < gr.warps[6]) rows_items<KIND, 6, PLAIN, NV>(d, st, w - gr.warps[7], nb);
+  else if (w < gr.warps[5]) rows_items<KIND, 5, PLAIN, NV>(d, st, w - gr.warps[6], nb);
+  else if (w < gr.warps[4]) rows_items<KIND, 4, PLAIN, NV>(d, st, w - gr.warps[5], nb);
+  else if (w < gr.warps[3]) rows_items<KIND, 3, PLAIN, NV>(d, st, w - gr.warps[4], nb);
+  else if (w < gr.warps[2]) rows_items<KIND, 2, PLAIN, NV>(d, st, w - gr.warps[3], nb);
+  else if (w < gr.warps[1]) rows_items<KIND, 1, PLAIN, NV>(d, st, w - gr.warps[2], nb);
 }
 
 // Per (leaf, channel): the far sums along the leaf's chain (root to leaf), FP64, shared by the
@@ -561,36 +663,41 @@ __global__ void hm_chain_sum_kernel(HDev d, const double *__restrict__ src, doub
   if (t >= (size_t)d.n_leaves * CC) return;
   const int k = (int)(t / CC), c = (int)(t % CC);
   double s = 0.0;
+  src += blockIdx.y * (size_t)d.n_nodes * CC;
   for (uint32_t ci = d.chain_off[k]; ci < d.chain_off[k + 1]; ++ci) s += src[(size_t)d.chain[ci] * CC + c];
-  dst[t] = s;
+  dst[blockIdx.y * (size_t)d.n_leaves * CC + t] = s;
 }
 
 // Per (row, channel): z = near + (m_p H~a_far - H~(a m)_far), the near sums of the leaf's
 // items (in item order, as float pairs) plus the leaf's chain sums of the far field (FP64,
 // hm_chain_sum_kernel). The far part of H~a was summed with the same operations from psi = a,
 // so m = 1 gives z = 0 exactly.
-template <int SEL, int CC>
+template <int SEL>
 __global__ void hm_epilogue_kernel(HDev d) {
+  constexpr int CC = kChannels<SEL>;
   const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const size_t row = t / CC;
   const int c = (int)(t - row * CC);
   const uint32_t k = (uint32_t)(row >> 3), r = (uint32_t)(row & 7);
   if (k >= (uint32_t)d.n_leaves) return;
+  if (SEL == VERTEX_CH && c == 3) return;  // padding
   const uint32_t leaf = d.leaves[k];
   const uint32_t s0 = d.start[leaf];
   if (r >= d.end[leaf] - s0) return;
-  const uint32_t p = s0 + r;
+  const size_t p = blockIdx.y * (size_t)d.n_el + s0 + r;
+  const float2 *part = d.part + blockIdx.y * (size_t)d.n_items * 8 * CC;
   float nh = 0.f, nl = 0.f;
   for (uint32_t i = d.item_off[k]; i < d.item_off[k + 1]; ++i) {
-    const float2 v = d.part[((size_t)i * 8 + r) * CC + c];
+    const float2 v = part[((size_t)i * 8 + r) * CC + c];
     pair_add(nh, nl, v.x, v.y);
   }
   const double2 fa = d.leaf_farA[k];
-  const float2 mv = m_get(d.m + (size_t)p * CC, c);
-  const double far = ((double)mv.x + (double)mv.y) * (uses_k1<SEL>(c) ? fa.y : fa.x) - d.leafsum[(size_t)k * CC + c];
+  const float2 mv = m_get<SEL>(d.m + p * (2 * CC), c);
+  const double far = ((double)mv.x + (double)mv.y) * (uses_k1<SEL>(c) ? fa.y : fa.x) -
+                     d.leafsum[(blockIdx.y * (size_t)d.n_leaves + k) * CC + c];
   const double zz = ((double)nh + (double)nl) + far;
   const float zh = (float)zz;
-  d.z[(size_t)p * CC + c] = make_float2(zh, (float)(zz - (double)zh));
+  d.z[p * CC + c] = make_float2(zh, (float)(zz - (double)zh));
 }
 
 // ------------------------------------------------------------------ face prologue / epilogue
@@ -629,55 +736,55 @@ __device__ __forceinline__ float2 split_q(double v, unsigned long long qbits) {
 
 // pass 0: the channels' largest magnitudes (a warp maximum of the high words, then one atomic
 // per warp and channel; every lane of the warp takes part, `act` false contributing 0);
-// pass 1: the split values
-__device__ __forceinline__ void emit(float2 *mp, int c, double v, unsigned long long *qmax, int pass, bool act) {
+// pass 1: the split value
+__device__ __forceinline__ void emit(float2 &o, int c, double v, unsigned long long *qmax, int pass, bool act) {
   if (pass == 0) {
     unsigned a = act ? (unsigned)((unsigned long long)__double_as_longlong(fabs(v)) >> 32) : 0u;
     a = __reduce_max_sync(0xffffffffu, a);
     if ((threadIdx.x & 31) == 0 && a != 0u) atomicMax(qmax + c, (unsigned long long)a << 32);
   } else if (act) {
-    m_set(mp, c, split_q(v, qmax[c]));
+    o = split_q(v, qmax[c]);
   }
 }
 
 // m per face in BVH order (FaceMetricTree::product, hierarchical.rs:711-746), in FP64 and
-// stored as float pairs; vector q owns channels 12q + (3k + r) = sum_c x[3 t_c + k] g_c[r]
-// (gradient) and 12q + 9 + k = (x_0 + x_1 + x_2)/3 for axis k (average; the division by 3 is
-// a product with the rounded 1/3, within an FP64 unit of the quotient, far below the float
-// pairs' resolution).
-__global__ void face_m_kernel(FaceOps o, const double *__restrict__ xs, size_t ldx, int nb, int C,
-                              float2 *m, unsigned long long *qmax, int pass) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// stored as float pairs; channels 3k + r = sum_c x[3 t_c + k] g_c[r] (gradient) and 9 + k =
+// (x_0 + x_1 + x_2)/3 for axis k (average; the division by 3 is a product with the rounded 1/3,
+// within an FP64 unit of the quotient, far below the float pairs' resolution). blockIdx.y is
+// the vector.
+__global__ void face_m_kernel(FaceOps o, const double *__restrict__ xs, size_t ldx, float *m, unsigned long long *qmax,
+                              int pass) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
   const bool act = p < o.nf;  // the whole warp runs the loops (warp maxima in pass 0)
   const uint32_t f = act ? o.order[p] : 0;
   const uint32_t *t = o.faces + 3 * (size_t)f;
   const double *g = o.g + 9 * (size_t)f;
-  float2 *mp = m + (size_t)(act ? p : 0) * C;
-  for (int q = 0; q < nb; ++q) {
-    const double *x = xs + q * ldx;
-    for (int k = 0; k < 3; ++k) {
-      const double x0 = x[3 * (size_t)t[0] + k], x1 = x[3 * (size_t)t[1] + k], x2 = x[3 * (size_t)t[2] + k];
-      for (int r = 0; r < 3; ++r)
-        emit(mp, 12 * q + 3 * k + r, x0 * g[r] + x1 * g[3 + r] + x2 * g[6 + r], qmax, pass, act);
-      emit(mp, 12 * q + 9 + k, ((x0 + x1) + x2) * (1.0 / 3.0), qmax, pass, act);
-    }
+  const double *x = xs + q * ldx;
+  float2 v[12];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double x0 = x[3 * (size_t)t[0] + k], x1 = x[3 * (size_t)t[1] + k], x2 = x[3 * (size_t)t[2] + k];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+      emit(v[3 * k + r], 12 * q + 3 * k + r, x0 * g[r] + x1 * g[3 + r] + x2 * g[6 + r], qmax, pass, act);
+    emit(v[9 + k], 12 * q + 9 + k, ((x0 + x1) + x2) * (1.0 / 3.0), qmax, pass, act);
   }
-  if (pass == 1 && act)
-    for (int c = 12 * nb; c < C; ++c) m_set(mp, c, make_float2(0.f, 0.f));
+  if (pass == 1 && act) m_store<12>(m + ((size_t)q * o.nf + p) * 24, v);
 }
 
 // y_v = 2 sum_{S ni v} a_S (w_hi g_c . z_hi + w_lo z_lo / 3) in FP64 (hierarchical.rs:779-811).
-__global__ void face_gather_kernel(FaceOps o, const float2 *__restrict__ z, int nb, int C,
-                                   double w_hi, double w_lo, double *__restrict__ ys, size_t ldy) {
+__global__ void face_gather_kernel(FaceOps o, const float2 *__restrict__ z, double w_hi, double w_lo,
+                                   double *__restrict__ ys, size_t ldy) {
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= o.nv) return;
-  for (int q = 0; q < nb; ++q) {
+  {
+    const int q = blockIdx.y;
     double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
     for (uint32_t e = o.inc_off[v]; e < o.inc_off[v + 1]; ++e) {
       uint32_t fc = o.inc[e], f = fc >> 2, c = fc & 3;
       double a = o.area[f];
       const double *g = o.g + 9 * (size_t)f + 3 * c;
-      const float2 *zs = z + (size_t)o.position[f] * C + 12 * q;
+      const float2 *zs = z + ((size_t)q * o.nf + o.position[f]) * 12;
       double acc[3];
       for (int k = 0; k < 3; ++k) {
         const float2 *zh = zs + 3 * k;
@@ -695,32 +802,32 @@ __global__ void face_gather_kernel(FaceOps o, const float2 *__restrict__ z, int 
 
 // ------------------------------------------------------------------ vertex prologue / epilogue
 
-// psi channels of the vertex operator: m = x per axis (psi = a x in the upward sums), vector q
-// at channels 4q + k (4q + 3 is padding).
-__global__ void vertex_m_kernel(const uint32_t *order, const double *__restrict__ xs, size_t ldx,
-                                int nv, int nb, int C, float2 *m, unsigned long long *qmax, int pass) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// Channels of the vertex operator: m = x per axis (psi = a x in the upward sums); blockIdx.y is
+// the vector.
+__global__ void vertex_m_kernel(const uint32_t *order, const double *__restrict__ xs, size_t ldx, int nv, float *m,
+                                unsigned long long *qmax, int pass) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
   const bool act = p < nv;  // the whole warp runs the loops (warp maxima in pass 0)
   const uint32_t v = act ? order[p] : 0;
-  float2 *mp = m + (size_t)(act ? p : 0) * C;
-  if (pass == 1 && act)
-    for (int c = 0; c < C; ++c) m_set(mp, c, make_float2(0.f, 0.f));
-  for (int q = 0; q < nb; ++q)
-    for (int k = 0; k < 3; ++k) emit(mp, 4 * q + k, xs[q * ldx + 3 * (size_t)v + k], qmax, pass, act);
+  float2 mv[4];
+  mv[3] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) emit(mv[k], 3 * q + k, xs[q * ldx + 3 * (size_t)v + k], qmax, pass, act);
+  if (pass == 1 && act) m_store<4>(m + ((size_t)q * nv + p) * 8, mv);
 }
 
 // y = 2 a (H~a x - H~(a x)) = 2 a z (hierarchical.rs:1330-1343).
-__global__ void vertex_out_kernel(const uint32_t *order, const float4 *el, const float2 *z, int nv,
-                                  int nb, int C, double scale, double *__restrict__ ys, size_t ldy) {
+__global__ void vertex_out_kernel(const uint32_t *order, const float4 *el, const float2 *z, int nv, double scale,
+                                  double *__restrict__ ys, size_t ldy) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= nv) return;
+  const int q = blockIdx.y;
   uint32_t v = order[p];
   double a = el[p].w;
-  for (int q = 0; q < nb; ++q)
-    for (int k = 0; k < 3; ++k) {
-      const float2 zz = z[(size_t)p * C + 4 * q + k];
-      ys[q * ldy + 3 * (size_t)v + k] = scale * 2.0 * a * ((double)zz.x + zz.y);
-    }
+  for (int k = 0; k < 3; ++k) {
+    const float2 zz = z[((size_t)q * nv + p) * 4 + k];
+    ys[q * ldy + 3 * (size_t)v + k] = scale * 2.0 * a * ((double)zz.x + zz.y);
+  }
 }
 
 // Element records: positions as float pairs (hi + lo), weights, normals; FP64 in.
@@ -792,15 +899,45 @@ __global__ void near_fill_kernel(uint32_t nl, const uint32_t *__restrict__ leave
   }
 }
 
-// the weight count of every work item: its rows times its columns padded to 32
+// the weight count of every work item, in blocks of 8 float2 (kernels x row pairs x padded columns),
+// and the total of rows x columns padded to 32 (the size the near field is limited by)
+template <int KIND>
 __global__ void item_weights_kernel(uint32_t n_items, const uint4 *__restrict__ items, const uint32_t *__restrict__ leaves,
                                     const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
-                                    unsigned long long *w) {
+                                    unsigned long long *w, unsigned long long *total) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned long long entries = 0;
+  if (i < n_items) {
+    const uint4 it = items[i];
+    const uint32_t leaf = leaves[it.x], ns = end[leaf] - start[leaf], ncol = it.z - it.y;
+    w[i] = near_weights<KIND>(ns, ncol) / 8;
+    entries = (unsigned long long)ns * ((ncol + 31) & ~31u);
+  }
+  for (int o = 16; o > 0; o >>= 1) entries += __shfl_down_sync(0xffffffffu, entries, o);
+  if ((threadIdx.x & 31) == 0 && entries) atomicAdd(total, entries);
+}
+// sort key of every work item: the leaf's rows, then most columns first
+__global__ void item_key_kernel(uint32_t n_items, const uint4 *__restrict__ items, const uint32_t *__restrict__ leaves,
+                                const uint32_t *__restrict__ start, const uint32_t *__restrict__ end, uint32_t *key,
+                                uint32_t *idx) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_items) return;
   const uint4 it = items[i];
   const uint32_t leaf = leaves[it.x];
-  w[i] = (unsigned long long)(end[leaf] - start[leaf]) * ((it.z - it.y + 31) & ~31u);
+  key[i] = ((end[leaf] - start[leaf]) << 16) | (0xffffu - (it.z - it.y));
+  idx[i] = i;
+}
+// off[i] = the first of the sorted keys of more than i rows, i = 0 .. 8
+__global__ void sched_off_kernel(uint32_t n, const uint32_t *__restrict__ key, uint32_t *off) {
+  const uint32_t i = threadIdx.x;
+  if (i > 8) return;
+  uint32_t a = 0, b = n;
+  while (a < b) {
+    const uint32_t c = (a + b) / 2;
+    if (key[c] >> 16 > i) b = c;
+    else a = c + 1;
+  }
+  off[i] = a;
 }
 __global__ void item_base_kernel(uint32_t n_items, const unsigned long long *__restrict__ base, uint4 *items) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -819,12 +956,6 @@ __global__ void far_fill_kernel(uint32_t nn, const uint32_t *__restrict__ far_pt
   const uint32_t q1 = far_ptr[a + 1];
   uint32_t j = off[a];
   for (uint32_t q0 = far_ptr[a]; q0 < q1; q0 += kFarChunk) items[j++] = make_uint4(a, q0, min(q0 + kFarChunk, q1), 0u);
-}
-
-// m = 1 in both channels of the paired layout: hi parts (1, 1), lo parts (0, 0)
-__global__ void ones_kernel(size_t n_el, float2 *m) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n_el) m[2 * i] = make_float2(1.f, 1.f), m[2 * i + 1] = make_float2(0.f, 0.f);
 }
 
 }  // namespace rsg
@@ -858,7 +989,9 @@ struct HMat {
   DevBuf<float2> fpart;
   DevBuf<uint32_t> colidx;
   DevBuf<uint4> items;
-  DevBuf<unsigned char> wts;  // near weights (NearW per entry), see hm_weights_kernel
+  DevBuf<float2> wts;  // near weights, see hm_weights_kernel
+  DevBuf<uint32_t> sched;  // the work items in the order of the near field, and its groups
+  uint32_t sched_off[9] = {};
   size_t n_wts = 0;
   DevBuf<float4> far_coef;
   DevBuf<double2> leaf_farA;
@@ -866,14 +999,14 @@ struct HMat {
   DevBuf<float4> xh, xl, nrm;
   DevBuf<double> up, farx;
   DevBuf<float2> up2;
-  DevBuf<float2> part, m, z;
+  DevBuf<float2> part, m, z;  // m: channel values (2 C floats per element)
   DevBuf<unsigned long long> qmax;  // per channel: largest |m| (see split_q)
   int pw_mode = 0, pw_k = 0;
   bool plain_rows = false;  // the near field of the next product in plain FP32 sums (inner operator)
   Profiler prof;
   double setup_times[3] = {0, 0, 0};  // seconds: work items, far coefficients, device part
 
-  HDev dev(int C_) const {
+  HDev dev() const {
     HDev d;
     d.start = start.p, d.end = end.p, d.right = right.p, d.parent = parent.p, d.leaves = leaves.p;
     d.chain_off = chain_off.p, d.chain = chain.p;
@@ -882,11 +1015,12 @@ struct HMat {
     d.n_far_items = (int)n_far_items;
     d.xh = xh.p, d.xl = xl.p, d.nrm = nrm.p, d.leaf_farA = leaf_farA.p;
     d.colidx = colidx.p, d.items = items.p, d.item_off = item_off.p, d.wts = wts.p;
+    d.sched = sched.p;
+    std::copy(sched_off, sched_off + 9, d.sched_off);
     d.up = up.p, d.up2 = up2.p, d.farx = farx.p, d.part = part.p, d.count = count.p, d.leafsum = leafsum.p;
-    d.m = m.p, d.z = z.p;
+    d.m = reinterpret_cast<const float *>(m.p), d.z = z.p;
     d.n_nodes = (int)tree.n_nodes(), d.n_leaves = (int)tree.leaves.size(), d.n_el = (int)n_el;
     d.n_items = (int)n_items;
-    d.C = C_;
     d.neg_s = (float)neg_s;
     d.pw_mode = pw_mode, d.pw_k = pw_k;
     return d;
@@ -917,23 +1051,25 @@ struct HMat {
     }
   }
 
-  template <int SEL, int CC>
-  void upward_far(const HDev &d) {
+  template <int SEL>
+  void upward_far(const HDev &d, int nb) {
+    constexpr int CC = kChannels<SEL>;
+    const unsigned gy = (unsigned)nb;
     size_t nn = tree.n_nodes(), nl = tree.leaves.size();
     cudaStream_t s = st();
     prof.begin(s, kind == FACE ? "metric_upward" : "vfrac_upward");
-    hm_upward_kernel<CC><<<nblk(nl * 32, 128), 128, 0, s>>>(d);
+    hm_upward_kernel<SEL><<<dim3(nblk(nl * 32, 128), gy), 128, 0, s>>>(d);
     RSG_LAUNCHED(ctx, "hm_upward");
     prof.end(s);
     prof.begin(s, kind == FACE ? "metric_far" : "vfrac_far");
     if (n_far_items > 0) {  // chi = 0 (all near) has none
-      hm_far_kernel<SEL, CC><<<nblk(n_far_items * (CC < 12 ? 1 : CC / 12) * 32, 256), 256, 0, s>>>(d);
+      hm_far_kernel<SEL><<<dim3(nblk(n_far_items * 32, 256), gy), 256, 0, s>>>(d);
       RSG_LAUNCHED(ctx, "hm_far");
     }
-    hm_far_final_kernel<CC><<<nblk(nn * CC, 256), 256, 0, s>>>(d);
+    hm_far_final_kernel<CC><<<dim3(nblk(nn * CC, 256), gy), 256, 0, s>>>(d);
     RSG_LAUNCHED(ctx, "hm_far_final");
     if (SEL != ONES) {
-      hm_chain_sum_kernel<CC><<<nblk(nl * CC, 256), 256, 0, s>>>(d, d.farx, d.leafsum);
+      hm_chain_sum_kernel<CC><<<dim3(nblk(nl * CC, 256), gy), 256, 0, s>>>(d, d.farx, d.leafsum);
       RSG_LAUNCHED(ctx, "hm_chain_sum");
     }
     prof.end(s);
@@ -999,19 +1135,40 @@ struct HMat {
       n_items = n_it;
     }
     lap(setup_times[0]);
-    // weight base of every item: its rows times its columns padded to 32
+    // weight base of every item
     {
-      DevBuf<unsigned long long> w(n_items + 1), base(n_items + 1);
+      DevBuf<unsigned long long> w(n_items + 1), base(n_items + 1), entries(1);
       RSG_CUDA("upload", cudaMemsetAsync(w.p + n_items, 0, sizeof(unsigned long long), s));
-      item_weights_kernel<<<nblk(n_items, 256), 256, 0, s>>>((uint32_t)n_items, items.p, leaves.p, start.p, end.p,
-                                                              w.p);
+      RSG_CUDA("upload", cudaMemsetAsync(entries.p, 0, sizeof(unsigned long long), s));
+      if (kind == FACE)
+        item_weights_kernel<FACE><<<nblk(n_items, 256), 256, 0, s>>>((uint32_t)n_items, items.p, leaves.p, start.p,
+                                                                     end.p, w.p, entries.p);
+      else
+        item_weights_kernel<VERTEX><<<nblk(n_items, 256), 256, 0, s>>>((uint32_t)n_items, items.p, leaves.p, start.p,
+                                                                       end.p, w.p, entries.p);
       RSG_LAUNCHED(ctx, "hm_item_weights");
       scan(w.p, base.p, n_items + 1);
-      unsigned long long tot = 0;
+      DevBuf<uint32_t> key(2 * n_items), idx(n_items), off(9);
+      item_key_kernel<<<nblk(n_items, 256), 256, 0, s>>>((uint32_t)n_items, items.p, leaves.p, start.p, end.p, key.p,
+                                                          idx.p);
+      RSG_LAUNCHED(ctx, "hm_item_key");
+      sched.alloc(n_items);
+      size_t bytes = 0;
+      RSG_CUDA("upload", cub::DeviceRadixSort::SortPairs(nullptr, bytes, key.p, key.p + n_items, idx.p, sched.p,
+                                                         (int)n_items, 0, 20, s));
+      if (bytes > tmp.n) tmp.alloc(bytes);
+      RSG_CUDA("upload", cub::DeviceRadixSort::SortPairs(tmp.p, bytes, key.p, key.p + n_items, idx.p, sched.p,
+                                                         (int)n_items, 0, 20, s));
+      sched_off_kernel<<<1, 32, 0, s>>>((uint32_t)n_items, key.p + n_items, off.p);
+      RSG_LAUNCHED(ctx, "hm_sched_off");
+      off.download(sched_off, 9, s);
+      unsigned long long tot = 0, n_entries = 0;
       RSG_CUDA("upload", copy_async(&tot, base.p + n_items, sizeof(tot), cudaMemcpyDeviceToHost, s));
+      RSG_CUDA("upload", copy_async(&n_entries, entries.p, sizeof(n_entries), cudaMemcpyDeviceToHost, s));
       RSG_CUDA("upload", cudaStreamSynchronize(s));
-      if (tot > UINT32_MAX) fail(RS_INVALID_OPTION, "InvalidOption", "upload", "near field too large");
-      n_wts = tot;
+      if (n_entries > UINT32_MAX || tot > UINT32_MAX)
+        fail(RS_INVALID_OPTION, "InvalidOption", "upload", "near field too large");
+      n_wts = 8 * (size_t)tot;
       item_base_kernel<<<nblk(n_items, 256), 256, 0, s>>>((uint32_t)n_items, base.p, items.p);
       RSG_LAUNCHED(ctx, "hm_item_weights");
     }
@@ -1031,8 +1188,8 @@ struct HMat {
       far_fill_kernel<<<nblk(nn, 256), 256, 0, s>>>((uint32_t)nn, blocks.far_ptr.p, far_item_off.p, far_items.p);
       RSG_LAUNCHED(ctx, "hm_far_items");
     }
-    count.alloc(nn);
-    RSG_CUDA("upload", cudaMemsetAsync(count.p, 0, nn * sizeof(uint32_t), s));
+    count.alloc(3 * nn);  // one set per vector of a pass
+    RSG_CUDA("upload", cudaMemsetAsync(count.p, 0, 3 * nn * sizeof(uint32_t), s));
     // far coefficients (kernel.far, hierarchical.rs:210-220 / 980-984) in FP64 on the device
     // from the node centroids (and, for faces, the node projectors)
     {
@@ -1061,23 +1218,18 @@ struct HMat {
                                                    xh.p, xl.p, kind == FACE ? nrm.p : nullptr);
     RSG_LAUNCHED(ctx, "hm_pack");
     // near weights of every work item, evaluated once; the product passes read them
-    wts.alloc(std::max<size_t>(n_wts * (kind == FACE ? sizeof(float2) : sizeof(float)), 16));
+    wts.alloc(std::max<size_t>(n_wts, 2));
     {
-      const HDev dw0 = dev(0);
+      const HDev dw0 = dev();
       const unsigned g = nblk(n_items * 8 * 32, 256);
-      if (kind == FACE) hm_weights_kernel<FACE><<<g, 256, 0, s>>>(dw0, n_wts);
-      else hm_weights_kernel<VERTEX><<<g, 256, 0, s>>>(dw0, n_wts);
+      if (kind == FACE) hm_weights_kernel<FACE><<<g, 256, 0, s>>>(dw0);
+      else hm_weights_kernel<VERTEX><<<g, 256, 0, s>>>(dw0);
       RSG_LAUNCHED(ctx, "hm_weights");
     }
     // far part of H~a: upward over psi = a (m = 1, 2 channels) and far sums per node
     reserve(4);
-    // m = 1 in both channels: hi parts (1, 1), lo parts (0, 0) in the paired layout
-    DevBuf<float2> mm(2 * n_el);
-    ones_kernel<<<nblk(n_el, 256), 256, 0, s>>>(n_el, mm.p);
-    RSG_LAUNCHED(ctx, "hm_ones");
-    HDev d = dev(2);
-    d.m = mm.p;
-    upward_far<ONES, 2>(d);
+    HDev d = dev();
+    upward_far<ONES>(d, 1);
     leaf_farA.alloc(std::max<size_t>(nl, 1));
     hm_chain_sum_kernel<2><<<nblk(nl * 2, 256), 256, 0, s>>>(d, farx.p, reinterpret_cast<double *>(leaf_farA.p));
     RSG_LAUNCHED(ctx, "hm_chain_sum");
@@ -1085,50 +1237,49 @@ struct HMat {
     lap(setup_times[2]);
   }
 
-  // z for the C-channel m already in `m` (faces: C = 12 nb, vertices: C = 4 nb).
-  template <int K, int CC>
-  void product_cc(int nb) {
+  // the near field of nb <= 3 vectors; the warps of the leaves of 8 rows first
+  template <int K, bool PLAIN, int NV>
+  void rows(const HDev &d, int nb) {
+    const int ipw[9] = {1,
+                        NearLanes<K, 1, PLAIN, NV>::IPW,
+                        NearLanes<K, 2, PLAIN, NV>::IPW,
+                        NearLanes<K, 3, PLAIN, NV>::IPW,
+                        NearLanes<K, 4, PLAIN, NV>::IPW,
+                        NearLanes<K, 5, PLAIN, NV>::IPW,
+                        NearLanes<K, 6, PLAIN, NV>::IPW,
+                        NearLanes<K, 7, PLAIN, NV>::IPW,
+                        NearLanes<K, 8, PLAIN, NV>::IPW};
+    const uint32_t passes = (uint32_t)(nb / NV);
+    RowsGrid gr;
+    gr.warps[9] = gr.warps[0] = 0;
+    for (int i = 8; i >= 1; --i)
+      gr.warps[i] = gr.warps[i + 1] + (sched_off[i] - sched_off[i - 1] + ipw[i] - 1) / ipw[i] * passes;
+    hm_rows_kernel<K, PLAIN, NV><<<nblk((size_t)gr.warps[1] * 32, 128), 128, 0, st()>>>(d, gr, passes);
+    RSG_LAUNCHED(ctx, "hm_rows");
+  }
+  template <bool PLAIN>
+  void rows_any(const HDev &d, int nb) {
+    if (kind == FACE) rows<FACE, PLAIN, 1>(d, nb);
+    else if (nb == 1) rows<VERTEX, PLAIN, 1>(d, nb);
+    else if (nb == 2) rows<VERTEX, PLAIN, 2>(d, nb);
+    else rows<VERTEX, PLAIN, 3>(d, nb);
+  }
+
+  // z of the nb vectors whose channel values are already in `m`.
+  template <int K>
+  void product_on(const HDev &d, int nb) {
     cudaStream_t s = st();
-    HDev d = dev(CC);
     constexpr int SEL = K == FACE ? FACE_CH : VERTEX_CH;
-    upward_far<SEL, CC>(d);
+    upward_far<SEL>(d, nb);
     prof.begin(s, K == FACE ? "metric_rows" : "vfrac_rows");
-    if constexpr (K == FACE) {
-      for (int q = 0; q < nb; ++q) {  // one vector (12 channels) per pass
-        if (plain_rows) hm_rows_kernel<K, 12, true><<<nblk(n_items * 32, 128), 128, 0, s>>>(d, 12 * q);
-        else hm_rows_kernel<K, 12, false><<<nblk(n_items * 32, 128), 128, 0, s>>>(d, 12 * q);
-        RSG_LAUNCHED(ctx, "hm_rows");
-      }
-    } else {
-      if (plain_rows) hm_rows_kernel<K, CC, true><<<nblk(n_items * 32, 128), 128, 0, s>>>(d, 0);
-      else hm_rows_kernel<K, CC, false><<<nblk(n_items * 32, 128), 128, 0, s>>>(d, 0);
-      RSG_LAUNCHED(ctx, "hm_rows");
-    }
+    if (plain_rows) rows_any<true>(d, nb);
+    else rows_any<false>(d, nb);
     prof.end(s);
     prof.begin(s, K == FACE ? "metric_epilogue" : "vfrac_epilogue");
-    epilogue<SEL, CC>(d);
-    prof.end(s);
-  }
-
-  // z from the near partial sums and the far chain sums (one thread per row and channel)
-  template <int SEL, int CC>
-  void epilogue(const HDev &d) {
-    hm_epilogue_kernel<SEL, CC><<<nblk(tree.leaves.size() * 8 * CC, 256), 256, 0, st()>>>(d);
+    // z from the near partial sums and the far chain sums (one thread per row and channel)
+    hm_epilogue_kernel<SEL><<<dim3(nblk(tree.leaves.size() * 8 * kChannels<SEL>, 256), (unsigned)nb), 256, 0, s>>>(d);
     RSG_LAUNCHED(ctx, "hm_epilogue");
-  }
-
-  void product(int nb) {
-    if (kind == FACE) {
-      if (nb == 1) product_cc<FACE, 12>(1);
-      else if (nb == 2) product_cc<FACE, 24>(2);
-      else if (nb == 3) product_cc<FACE, 36>(3);
-      else fail(RS_INTERNAL, "Internal", "product", "unsupported channel count");
-    } else {
-      if (nb == 1) product_cc<VERTEX, 4>(1);
-      else if (nb == 2) product_cc<VERTEX, 8>(2);
-      else if (nb == 3) product_cc<VERTEX, 12>(3);
-      else fail(RS_INTERNAL, "Internal", "product", "unsupported channel count");
-    }
+    prof.end(s);
   }
 
   void build_common(rs_ctx *c, Tree &&t, double chi, int leaf_pairs) {
@@ -1264,6 +1415,26 @@ void metric_setup(rs_metric *M, rs_ctx *ctx, int nv, int nf, const uint32_t *fac
 
 }  // namespace
 
+// The product of k <= 3 vectors in one tree pass on the scratch of d and qmax.
+static void face_product(rs_metric *M, const HDev &d, unsigned long long *qmax, int k, const double *xs, size_t ldx,
+                         double w_hi, double w_lo, double *ys, size_t ldy) {
+  HMat &h = M->h;
+  cudaStream_t s = h.st();
+  const unsigned gy = (unsigned)k;
+  h.prof.begin(s, "metric_m");
+  RSG_CUDA("product", cudaMemsetAsync(qmax, 0, 12 * k * sizeof(unsigned long long), s));
+  for (int pass = 0; pass < 2; ++pass) {
+    face_m_kernel<<<dim3(nblk(M->nf, 256), gy), 256, 0, s>>>(M->ops(), xs, ldx, const_cast<float *>(d.m), qmax, pass);
+    RSG_LAUNCHED(h.ctx, "face_m");
+  }
+  h.prof.end(s);
+  h.product_on<FACE>(d, k);
+  h.prof.begin(s, "metric_gather");
+  face_gather_kernel<<<dim3(nblk(M->nv, 128), gy), 128, 0, s>>>(M->ops(), d.z, w_hi, w_lo, ys, ldy);
+  RSG_LAUNCHED(h.ctx, "face_gather");
+  h.prof.end(s);
+}
+
 // FaceMetricTree::apply_batch (hierarchical.rs:540-622) on device vectors with leading
 // dimensions ldx, ldy (>= 3V): groups of <= 3 vectors per tree pass.
 void rsg::metric_apply_strided(rs_metric *M, double w_hi, double w_lo, int nb, const double *xs,
@@ -1274,22 +1445,9 @@ void rsg::metric_apply_strided(rs_metric *M, double w_hi, double w_lo, int nb, c
   M->h.plain_rows = plain;
   for (int q0 = 0; q0 < nb; q0 += 3) {
     int k = std::min(3, nb - q0);
-    int CC = 12 * k;
-    M->h.reserve(CC);
-    M->h.prof.begin(s, "metric_m");
+    M->h.reserve(12 * k);
     if (M->h.qmax.n < 64) M->h.qmax.alloc(64);
-    RSG_CUDA("product", cudaMemsetAsync(M->h.qmax.p, 0, CC * sizeof(unsigned long long), s));
-    for (int pass = 0; pass < 2; ++pass) {
-      face_m_kernel<<<nblk(M->nf, 256), 256, 0, s>>>(M->ops(), xs + q0 * ldx, ldx, k, CC, M->h.m.p, M->h.qmax.p, pass);
-      RSG_LAUNCHED(M->h.ctx, "face_m");
-    }
-    M->h.prof.end(s);
-    M->h.product(k);
-    M->h.prof.begin(s, "metric_gather");
-    face_gather_kernel<<<nblk(M->nv, 128), 128, 0, s>>>(M->ops(), M->h.z.p, k, CC, w_hi, w_lo,
-                                                        ys + q0 * ldy, ldy);
-    RSG_LAUNCHED(M->h.ctx, "face_gather");
-    M->h.prof.end(s);
+    face_product(M, M->h.dev(), M->h.qmax.p, k, xs + q0 * ldx, ldx, w_hi, w_lo, ys + q0 * ldy, ldy);
   }
 }
 
@@ -1300,18 +1458,19 @@ void rsg::vfrac_apply_strided(rs_vfrac *V, double scale, int nb, const double *x
   V->h.plain_rows = plain;
   for (int q0 = 0; q0 < nb; q0 += 3) {
     int k = std::min(3, nb - q0);
-    int CC = 4 * k;  // 3 k channels padded to a multiple of 4
-    V->h.reserve(CC);
+    const unsigned gy = (unsigned)k;
+    V->h.reserve(4 * k);
     if (V->h.qmax.n < 64) V->h.qmax.alloc(64);
-    RSG_CUDA("product", cudaMemsetAsync(V->h.qmax.p, 0, CC * sizeof(unsigned long long), s));
+    const HDev d = V->h.dev();
+    RSG_CUDA("product", cudaMemsetAsync(V->h.qmax.p, 0, 3 * k * sizeof(unsigned long long), s));
     for (int pass = 0; pass < 2; ++pass) {
-      vertex_m_kernel<<<nblk(V->nv, 256), 256, 0, s>>>(V->order.p, xs + q0 * ldx, ldx, V->nv, k, CC, V->h.m.p,
-                                                       V->h.qmax.p, pass);
+      vertex_m_kernel<<<dim3(nblk(V->nv, 256), gy), 256, 0, s>>>(V->order.p, xs + q0 * ldx, ldx, V->nv,
+                                                                 const_cast<float *>(d.m), V->h.qmax.p, pass);
       RSG_LAUNCHED(V->h.ctx, "vertex_m");
     }
-    V->h.product(k);
-    vertex_out_kernel<<<nblk(V->nv, 256), 256, 0, s>>>(V->order.p, V->h.xh.p, V->h.z.p, V->nv, k, CC,
-                                                       scale, ys + q0 * ldy, ldy);
+    V->h.product_on<VERTEX>(d, k);
+    vertex_out_kernel<<<dim3(nblk(V->nv, 256), gy), 256, 0, s>>>(V->order.p, V->h.xh.p, V->h.z.p, V->nv, scale,
+                                                                 ys + q0 * ldy, ldy);
     RSG_LAUNCHED(V->h.ctx, "vertex_out");
   }
 }
@@ -1533,7 +1692,7 @@ size_t noalloc_bytes(const HMat &h, int C) {
 }
 
 HDev noalloc_dev(const HMat &h, int C, unsigned char *base) {
-  HDev d = h.dev(C);
+  HDev d = h.dev();
   size_t nn = h.tree.n_nodes(), off = 0;
   auto take = [&](size_t bytes) {
     unsigned char *p = base + off;
@@ -1543,7 +1702,7 @@ HDev noalloc_dev(const HMat &h, int C, unsigned char *base) {
   d.up = reinterpret_cast<double *>(take(nn * C * sizeof(double)));
   d.up2 = reinterpret_cast<float2 *>(take(nn * C * sizeof(float2)));
   d.farx = reinterpret_cast<double *>(take(nn * C * sizeof(double)));
-  d.m = reinterpret_cast<const float2 *>(take(h.n_el * C * sizeof(float2)));
+  d.m = reinterpret_cast<const float *>(take(h.n_el * C * sizeof(float2)));
   d.z = reinterpret_cast<float2 *>(take(h.n_el * C * sizeof(float2)));
   d.part = reinterpret_cast<float2 *>(take(std::max<size_t>(h.n_items, 1) * 8 * C * sizeof(float2)));
   d.leafsum = reinterpret_cast<double *>(take(h.tree.leaves.size() * C * sizeof(double)));
@@ -1554,29 +1713,6 @@ HDev noalloc_dev(const HMat &h, int C, unsigned char *base) {
 // the per-channel magnitudes of the no-alloc product, after the buffers of noalloc_dev
 unsigned long long *noalloc_qmax(const HMat &h, int C, unsigned char *base) {
   return reinterpret_cast<unsigned long long *>(base + noalloc_bytes(h, C) - align256(64 * sizeof(unsigned long long)));
-}
-
-// The face product of one group of k <= 3 vectors on the given scratch (the kernels and order
-// of HMat::product_cc and metric_apply_strided).
-template <int CC>
-void noalloc_face_group(rs_metric *M, const HDev &d, unsigned long long *qmax, int k, const double *xs, size_t ldx,
-                        double w_hi, double w_lo, double *ys, size_t ldy) {
-  HMat &h = M->h;
-  cudaStream_t s = h.st();
-  float2 *m = const_cast<float2 *>(d.m);
-  RSG_CUDA("product", cudaMemsetAsync(qmax, 0, CC * sizeof(unsigned long long), s));
-  for (int pass = 0; pass < 2; ++pass) {
-    face_m_kernel<<<nblk(M->nf, 256), 256, 0, s>>>(M->ops(), xs, ldx, k, CC, m, qmax, pass);
-    RSG_LAUNCHED(h.ctx, "face_m");
-  }
-  h.upward_far<FACE_CH, CC>(d);
-  for (int q = 0; q < k; ++q) {
-    hm_rows_kernel<FACE, 12, false><<<nblk(h.n_items * 32, 128), 128, 0, s>>>(d, 12 * q);
-    RSG_LAUNCHED(h.ctx, "hm_rows");
-  }
-  h.epilogue<FACE_CH, CC>(d);
-  face_gather_kernel<<<nblk(M->nv, 128), 128, 0, s>>>(M->ops(), d.z, k, CC, w_hi, w_lo, ys, ldy);
-  RSG_LAUNCHED(h.ctx, "face_gather");
 }
 
 }  // namespace
@@ -1600,9 +1736,8 @@ extern "C" int rs_metric_apply_device_noalloc(rs_metric *M, double w_hi, double 
       const int k = std::min(3, nb - q0);
       HDev d = noalloc_dev(M->h, 12 * k, base);
       unsigned long long *qm = noalloc_qmax(M->h, 12 * k, base);
-      if (k == 1) noalloc_face_group<12>(M, d, qm, 1, xs_dev + q0 * ld, ld, w_hi, w_lo, ys_dev + q0 * ld, ld);
-      else if (k == 2) noalloc_face_group<24>(M, d, qm, 2, xs_dev + q0 * ld, ld, w_hi, w_lo, ys_dev + q0 * ld, ld);
-      else noalloc_face_group<36>(M, d, qm, 3, xs_dev + q0 * ld, ld, w_hi, w_lo, ys_dev + q0 * ld, ld);
+      M->h.plain_rows = false;
+      face_product(M, d, qm, k, xs_dev + q0 * ld, ld, w_hi, w_lo, ys_dev + q0 * ld, ld);
     }
   });
 }
