@@ -113,6 +113,9 @@ struct rs_ctx {
   std::atomic<int> refs{1};
   int device = 0;
   cudaStream_t stream = nullptr;
+  // A second stream, for work that runs beside the first within one entry point: it is forked from
+  // the context's stream by an event and joined to it again before the entry point returns.
+  cudaStream_t stream2 = nullptr;
   int sm_count = 0;
   int cc_major = 0, cc_minor = 0;
   std::string name;

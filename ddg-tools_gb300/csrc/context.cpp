@@ -52,6 +52,10 @@ void rsg::ctx_release(rs_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     cudaStreamDestroy(ctx->stream);
   }
+  if (ctx->stream2) {
+    cudaStreamSynchronize(ctx->stream2);
+    cudaStreamDestroy(ctx->stream2);
+  }
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   delete ctx;
 }
@@ -122,6 +126,11 @@ int rs_ctx_create(int ordinal, rs_ctx **out) {
                   "librsgpu is built for sm_103a (GB300); device is sm_" +
                       std::to_string(prop.major) + std::to_string(prop.minor));
       RSG_CUDA("context", cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+      // the second stream's kernels are short and wait behind the first one's large grids
+      // otherwise
+      int least = 0, greatest = 0;
+      RSG_CUDA("context", cudaDeviceGetStreamPriorityRange(&least, &greatest));
+      RSG_CUDA("context", cudaStreamCreateWithPriority(&c->stream2, cudaStreamNonBlocking, greatest));
     } catch (...) {
       delete c;
       throw;

@@ -11,12 +11,13 @@
 //
 // Per product (C channels per element: 9 gradient + 3 average per input vector for faces, 3
 // per vector for vertices):
-//   prologue    m = M x per element (float pairs), element-major [n][C], a plane per vector
-//   upward      up[node] = sum_{q in node} a_q m_q, bottom-up (the second child to arrive adds)
-//   far         farx[node] = sum_{b in far(node)} h(node, b) up[b]            (warp per node)
-//   rows        per leaf (warp): near sums over the chain's near blocks with H~a accumulated
-//               in the same loop, far sums along the chain, z = H~a m - H~(a m)
-//   epilogue    y = 2 M^T diag(a) W z (faces: per-vertex gather; vertices: y = 2 a z)
+//   prologue    m = M x per element (float pairs and FP64), element-major [n][C], a plane per vector
+//   upward      up[node] = sum_{q in node} a_q m_q, bottom-up over groups of nodes
+//   far         fpart[item] = sum_b h(node, b) up[b] over slices of a node's far blocks
+//   chain       per leaf the far sums of its root-to-leaf chain
+//   rows        near sums of every work item (beside the three far passes, on another stream)
+//   epilogue    z = near + (m_p H~a_far - H~(a m)_far) per element; y = 2 M^T diag(a) W z (faces:
+//               per-vertex gather; vertices: y = 2 a z)
 // H~a is formed with the same operations as H~(a m) for m = 1, so L 1 = 0 exactly (the
 // reference's null-space property, hierarchical.rs:13-16).
 #include <algorithm>
@@ -63,6 +64,9 @@ struct HDev {
   const float4 *xh;          // per BVH position: position hi (xyz), weight a (w)
   const float4 *xl;          // per BVH position: position lo (xyz): X = hi + lo to ~48 bits
   const float4 *nrm;         // per BVH position: normal (faces only)
+  const uint32_t *leaf_of;   // per BVH position: its leaf ordinal
+  const uint4 *grp;          // bottom groups of nodes: root, number of nodes, first leaf ordinal, leaves
+  const uint32_t *grp_depth; // and the number of the root's ancestors
   const double2 *leaf_farA;  // per leaf: far sums of psi = a (k_0, k_1) along its chain, the far part of H~a
   double *leafsum;           // per leaf: C channel far sums along its chain
   const uint32_t *colidx;    // near columns of every leaf's chain, flattened, leaf by leaf
@@ -71,15 +75,13 @@ struct HDev {
   const uint32_t *item_off;  // per leaf: its work items [item_off[k], item_off[k + 1])
   const uint32_t *sched;     // work items by the leaf's rows, then most columns first
   uint32_t sched_off[9];     // those of leaves of i rows: [sched_off[i - 1], sched_off[i])
-  double *up;                // per node: C channel sums of a m (FP64)
-  float2 *up2;               // the same sums as float pairs (hi, lo), read by the far sums
-  double *farx;              // per node: C channel far sums (FP64)
+  double *up;                // per node: C channel sums of a m (FP64; of group roots only)
+  float2 *up2;               // per node: the same sums as float pairs (hi, lo), read by the far sums
   float2 *part;              // per work item: 8 rows x C near sums as float pairs
-  uint32_t *count;           // per node: arrival counter of the upward pass
-  const float *m;            // channel values as float pairs: [n] records of 2 C floats, see m_get
-  float2 *z;                 // [n][C] results as float pairs
+  const float *m;            // channel values as float pairs: [n] records of C hi, then C lo parts
+  double *z;                 // [n][C]: the channel values in FP64 (hi + lo), then the results in place
   // (the buffers with C channels hold one such plane per vector, vector by vector)
-  int n_nodes, n_leaves, n_el, n_items, n_far_items;
+  int n_nodes, n_leaves, n_el, n_items, n_far_items, n_grp;
   float neg_s;               // kernel exponent e applied to r^2: r2^e
   int pw_mode, pw_k;         // e = pw_k / pw_mode for pw_mode 2 or 3 (exact roots), else powf
 };
@@ -89,24 +91,6 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &t) {
   s = a + b;
   const float bv = s - a;
   t = (a - (s - bv)) + (b - bv);
-}
-
-// Layout of the channel values of one element: the hi parts, then the lo parts (12 and 12 floats
-// for faces; 4 and 4, the last of them zero, for vertices).
-template <int SEL>
-__device__ __forceinline__ float2 m_get(const float *f, int c) {
-  if (SEL == ONES) return make_float2(1.f, 0.f);
-  return make_float2(f[c], f[kChannels<SEL> + c]);
-}
-// the values v[0 .. C) of one element
-template <int C>
-__device__ __forceinline__ void m_store(float *f, const float2 (&v)[C]) {
-  float4 *o = reinterpret_cast<float4 *>(f);
-#pragma unroll
-  for (int i = 0; i < C; i += 4) {
-    o[i / 4] = make_float4(v[i].x, v[i + 1].x, v[i + 2].x, v[i + 3].x);
-    o[(C + i) / 4] = make_float4(v[i].y, v[i + 1].y, v[i + 2].y, v[i + 3].y);
-  }
 }
 
 // Two FP32 values in one 64-bit register (first in the low half) and the packed FP32 pair
@@ -144,10 +128,24 @@ __device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
 }
 constexpr f32x2 kF2Sign = 0x8000000080000000ull;  // both halves' sign bits
 
+// Conversions between FP32 and FP64 from the bits. GB300 converts at its FP64 rate, two lanes per
+// clock and SM, which bounded every pass around the near field; integer instructions run at 64.
+__device__ __forceinline__ double f2d(float x) {  // (double)x
+  const unsigned b = __float_as_uint(x), e = (b >> 23) & 0xffu;
+  if (e - 1u >= 254u) return (double)x;  // zero, subnormal, infinity, NaN
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ double rn24(double x) {  // (double)(float)x
+  const unsigned hi = (unsigned)__double2hiint(x), e = (hi >> 20) & 0x7ffu;
+  if (e - 897u >= 253u) return (double)(float)x;  // not a normal float
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  return __longlong_as_double((long long)((b + 0x0fffffffull + ((b >> 29) & 1ull)) & ~0x1fffffffull));
+}
+
 // v as a float pair: hi = v rounded to FP32, lo = the rest rounded
 __device__ __forceinline__ float2 to_pair(double v) {
   const float h = (float)v;
-  return make_float2(h, (float)(v - (double)h));
+  return make_float2(h, (float)(v - f2d(h)));
 }
 
 // (h, l) += (oh, ol) for float pairs.
@@ -200,54 +198,88 @@ __device__ __forceinline__ void near_kernel(const HDev &d, float d0, float d1, f
   }
 }
 
-// Bottom-up channel sums in FP64: one warp per leaf (lanes over the channels) sums its
-// elements in registers, then climbs; at every parent the second child to arrive adds
-// left + right (fixed order, no waiting). The far field is FP64 end to end (upward, far sums, chain push-down): its sums
-// cancel against m_p H~a for a smooth input just as the near sums do, and at O(nodes) and
-// O(far blocks) work the FP64 rate costs little.
+// Bottom-up channel sums in FP64: up[node] = left + right, and for a leaf its elements added in
+// order. (The far field's sums cancel against m_p H~a for a smooth input just as the near sums do.)
+// The nodes are cut into bottom groups (a subtree of at most 16 leaves, a block each) and above
+// them, level by level, groups of at most 128 roots of the level below, each again a block: the
+// leaves of a group are summed side by side and its inner nodes in decreasing index (children
+// before parents, the tree's indices being in preorder) from shared memory. Climbing from every leaf with an
+// arrival counter per node took 0.125 ms at 204,800 faces: 26 levels of fence, atomic and load, and
+// twelve of 32 lanes at FP64 work.
+constexpr int kGrpLeaves = 16, kGrpNodes = 2 * kGrpLeaves - 1, kGrpExt = 128;
+
 template <int SEL>
-__global__ void hm_upward_kernel(HDev d) {
-  // one warp per leaf and vector, lane l holding channel l
+__global__ void __launch_bounds__(192) hm_upward_kernel(HDev d) {
   constexpr int CC = kChannels<SEL>;
-  const int k = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31, c = lane;
+  __shared__ double sh[kGrpNodes * CC];
+  __shared__ uint32_t rt[kGrpNodes];
+  const uint4 gr = d.grp[blockIdx.x];
   const size_t pn = blockIdx.y * (size_t)d.n_nodes;
-  if (k >= d.n_leaves) return;
-  const uint32_t leaf = d.leaves[k];
-  double u = 0.0;
-  if (c < CC)
-    for (uint32_t p = d.start[leaf]; p < d.end[leaf]; ++p) {
-      const double a = d.xh[p].w;
-      const float2 v = m_get<SEL>(d.m + (blockIdx.y * (size_t)d.n_el + p) * (2 * CC), c);
-      u = fma(a, (double)v.x + (double)v.y, u);
+  if (threadIdx.x < gr.y) rt[threadIdx.x] = d.right[gr.x + threadIdx.x];
+  for (uint32_t t = threadIdx.x; t < gr.w * CC; t += blockDim.x) {
+    const uint32_t l = t / CC, c = t - l * CC, leaf = d.leaves[gr.z + l], p0 = d.start[leaf], n = d.end[leaf] - p0;
+    const double *z = d.z + (blockIdx.y * (size_t)d.n_el + p0) * CC + c;
+    double v[8], a[8], u = 0.0;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+      v[i] = i < n ? (SEL == ONES ? 1.0 : z[i * CC]) : 0.0;
+      a[i] = i < n ? f2d(d.xh[p0 + i].w) : 0.0;
     }
-  if (c < CC) d.up[(pn + leaf) * CC + c] = u, d.up2[(pn + leaf) * CC + c] = to_pair(u);
-  uint32_t n = leaf;
-  while (n != 0) {
-    const uint32_t par = d.parent[n];
-    __threadfence();  // this warp's sums of n, before the arrival is counted
-    __syncwarp();
-    unsigned old = 0u;
-    if (lane == 0) old = atomicAdd(&d.count[pn + par], 1u);
-    old = __shfl_sync(0xffffffffu, old, 0);
-    if ((old & 1u) == 0u) return;  // first child to arrive: the sibling's warp adds
-    __threadfence();
-    if (c < CC) {
-      const double v = __ldcg(d.up + (pn + par + 1) * CC + c) + __ldcg(d.up + (pn + d.right[par]) * CC + c);
-      d.up[(pn + par) * CC + c] = v, d.up2[(pn + par) * CC + c] = to_pair(v);
-    }
-    n = par;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i)
+      if (i < n) u = fma(a[i], v[i], u);
+    sh[(leaf - gr.x) * CC + c] = u;
+  }
+  __syncthreads();
+  if (threadIdx.x < CC) {
+    const uint32_t c = threadIdx.x;
+    for (int i = (int)gr.y - 1; i >= 0; --i)
+      if (rt[i]) sh[i * CC + c] = sh[(i + 1) * CC + c] + sh[(rt[i] - gr.x) * CC + c];
+  }
+  __syncthreads();
+  for (uint32_t t = threadIdx.x; t < gr.y * CC; t += blockDim.x) d.up2[(pn + gr.x) * CC + t] = to_pair(sh[t]);
+  if (threadIdx.x < CC) d.up[(pn + gr.x) * CC + threadIdx.x] = sh[threadIdx.x];
+}
+
+// One level above: group = (first of its roots of the level below in ext, their number, first of
+// its inner nodes in inner, their number); inner nodes in decreasing index with the slots of
+// their children (roots first, then the inner nodes in order).
+template <int CC>
+__global__ void __launch_bounds__(128) hm_upward_level_kernel(HDev d, const uint4 *__restrict__ groups,
+                                                              const uint32_t *__restrict__ ext,
+                                                              const uint32_t *__restrict__ inner,
+                                                              const uint2 *__restrict__ child) {
+  __shared__ double sh[(2 * kGrpExt - 1) * CC];
+  __shared__ uint2 ch[kGrpExt];
+  const uint4 gr = groups[blockIdx.x];
+  const size_t pn = blockIdx.y * (size_t)d.n_nodes;
+  for (uint32_t i = threadIdx.x; i < gr.w; i += blockDim.x) ch[i] = child[gr.z + i];
+  for (uint32_t t = threadIdx.x; t < gr.y * CC; t += blockDim.x)
+    sh[t] = d.up[(pn + ext[gr.x + t / CC]) * CC + t % CC];
+  __syncthreads();
+  if (threadIdx.x < CC)
+    for (uint32_t i = 0; i < gr.w; ++i)
+      sh[(gr.y + i) * CC + threadIdx.x] = sh[ch[i].x * CC + threadIdx.x] + sh[ch[i].y * CC + threadIdx.x];
+  __syncthreads();
+  for (uint32_t t = threadIdx.x; t < gr.w * CC; t += blockDim.x) {
+    const size_t o = (pn + inner[gr.z + t / CC]) * CC + t % CC;
+    const double v = sh[gr.y * CC + t];
+    d.up2[o] = to_pair(v);
+    if (t / CC + 1 == gr.w) d.up[o] = v;  // the group's root
   }
 }
 
-// farx[a][c] = sum over the far blocks (a, b) of h(a, b)[kernel(c)] up[b][c] (block_tree.rs:
-// 564-578) in double-float arithmetic: the coefficients and the node sums are float pairs
-// (about 48 bits), each product is formed exactly to that width (FMA) and added by error-free
-// transformations; the result is handed on in FP64. GB300 issues FP32 at many times its FP64
-// rate. One warp per (item, vector): lane = sub C + c holds channel c and takes the item's far
-// blocks sub, sub + 2, ... (sub = 0, 1); the two partial sums are then added. The operations
-// do not depend on the channel count, so the pass over psi = a (two channels) and a product
-// pass add the same terms in the same order.
+constexpr uint32_t kFarChunk = 64;  // far blocks per far work item
+
+// fpart[item][c] = sum over the item's far blocks (a, b) of h(a, b)[kernel(c)] up[b][c]
+// (block_tree.rs:564-578) in double-float arithmetic: the coefficients and the node sums are float
+// pairs (about 48 bits), each product is formed exactly to that width (FMA) and added by error-free
+// transformations. GB300 issues FP32 at many times its FP64 rate. One warp per item, all vectors:
+// lane = sub C + c holds channel c and takes the item's far blocks sub, sub + 2, ... (sub = 0, 1);
+// the two partial sums are then added. The item's columns and coefficients come in first, coalesced,
+// so that the gathers of the node sums are independent of one another. The operations do not
+// depend on the channel count, so the pass over psi = a (two channels) and a product pass add the
+// same terms in the same order.
 __device__ __forceinline__ void df_fma(float &ah, float &al, float kh, float kl, float uh, float ul) {
   const float ph = kh * uh;
   float pe = fmaf(kh, uh, -ph);
@@ -261,57 +293,98 @@ __device__ __forceinline__ void df_fma(float &ah, float &al, float kh, float kl,
 }
 
 template <int SEL>
-__global__ void hm_far_kernel(HDev d) {
+__global__ void __launch_bounds__(256) hm_far_kernel(HDev d, int nb) {
   constexpr int CC = kChannels<SEL>;
   static_assert(2 * CC <= 32, "two blocks at a time");
-  const int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+  __shared__ float4 coef[8][kFarChunk];
+  __shared__ uint32_t col[8][kFarChunk];
+  const int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5), wib = threadIdx.x >> 5;
   if (w >= d.n_far_items) return;
   const uint4 it = d.far_items[w];
   const int lane = threadIdx.x & 31, sub = lane / CC, ch = lane - sub * CC;
-  const float2 *up2 = d.up2 + blockIdx.y * (size_t)d.n_nodes * CC;
-  float ah = 0.f, al = 0.f;
-  if (sub < 2) {
-    const bool k1 = uses_k1<SEL>(ch);
-    uint32_t q = it.y + sub;
-    // four of the lane's blocks at a time: loads first, then the additions in order
-    for (; q + 6 < it.z; q += 8) {
-      float4 kk[4];
-      float2 u[4];
+  const uint32_t n = it.z - it.y;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        kk[i] = d.far_coef[q + 2 * i];
-        u[i] = up2[(size_t)d.far_col[q + 2 * i] * CC + ch];
+  for (uint32_t i = lane; i < kFarChunk; i += 32)
+    if (i < n) coef[wib][i] = __ldg(d.far_coef + it.y + i), col[wib][i] = __ldg(d.far_col + it.y + i) * CC;
+  __syncwarp();
+  const float2 *kp = reinterpret_cast<const float2 *>(&coef[wib][0]) + (uses_k1<SEL>(ch) ? 1 : 0);
+  for (int q = 0; q < nb; ++q) {
+    const float2 *__restrict__ up2 = d.up2 + q * (size_t)d.n_nodes * CC + ch;
+    float ah = 0.f, al = 0.f;
+    if (sub < 2) {
+      uint32_t b = sub;
+      for (; b + 14 < n; b += 16) {
+        float2 u[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) u[i] = __ldg(up2 + col[wib][b + 2 * i]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float2 k = kp[2 * (b + 2 * i)];
+          df_fma(ah, al, k.x, k.y, u[i].x, u[i].y);
+        }
       }
+      float2 u[8];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        df_fma(ah, al, k1 ? kk[i].z : kk[i].x, k1 ? kk[i].w : kk[i].y, u[i].x, u[i].y);
+      for (int i = 0; i < 8; ++i) u[i] = b + 2 * i < n ? __ldg(up2 + col[wib][b + 2 * i]) : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (b + 2 * i < n) {
+          const float2 k = kp[2 * (b + 2 * i)];
+          df_fma(ah, al, k.x, k.y, u[i].x, u[i].y);
+        }
     }
-    for (; q < it.z; q += 2) {
-      const float4 k = d.far_coef[q];
-      const float2 u = up2[(size_t)d.far_col[q] * CC + ch];
-      df_fma(ah, al, k1 ? k.z : k.x, k1 ? k.w : k.y, u.x, u.y);
-    }
+    const float oh = __shfl_down_sync(0xffffffffu, ah, CC), ol = __shfl_down_sync(0xffffffffu, al, CC);
+    pair_add(ah, al, oh, ol);
+    if (sub == 0) d.fpart[(q * (size_t)d.n_far_items + w) * CC + ch] = make_float2(ah, al);
   }
-  const float oh = __shfl_down_sync(0xffffffffu, ah, CC), ol = __shfl_down_sync(0xffffffffu, al, CC);
-  pair_add(ah, al, oh, ol);
-  if (sub == 0) d.fpart[(blockIdx.y * (size_t)d.n_far_items + w) * CC + ch] = make_float2(ah, al);
 }
 
-// farx[a][c]: the node's item partials added in item order as float pairs, handed on in FP64
-// (zero for a node without far blocks); one thread per (node, channel)
+// The far sums of a node: its item partials added in item order as float pairs, in FP64 (zero for
+// a node without far blocks).
 template <int CC>
-__global__ void hm_far_final_kernel(HDev d) {
-  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (t >= (size_t)d.n_nodes * CC) return;
-  const size_t a = t / CC;
-  const int c = (int)(t - a * CC);
+__device__ __forceinline__ double far_of_node(const HDev &d, const float2 *__restrict__ fp, uint32_t a, int c) {
   float h = 0.f, l = 0.f;
-  const float2 *fp = d.fpart + blockIdx.y * (size_t)d.n_far_items * CC;
   for (uint32_t i = d.far_item_off[a]; i < d.far_item_off[a + 1]; ++i) {
     const float2 v = fp[(size_t)i * CC + c];
     pair_add(h, l, v.x, v.y);
   }
-  d.farx[blockIdx.y * (size_t)d.n_nodes * CC + t] = (double)h + (double)l;
+  return f2d(h) + f2d(l);
+}
+
+// Per (leaf, channel): the far sums along the leaf's chain, from the root down in FP64, shared by the
+// leaf's rows. A block per bottom group: the sums of the root's ancestors, then down the group's
+// nodes in preorder, a node's sum being its parent's plus its own: each node is added once and
+// not once per leaf below it. With psi = a (ONES) the same sums give the far part of H~a.
+template <int SEL>
+__global__ void __launch_bounds__(192) hm_chain_sum_kernel(HDev d, double *__restrict__ dst) {
+  constexpr int CC = kChannels<SEL>, kAnc = 32;
+  __shared__ double sh[kGrpNodes * CC], anc[kAnc * CC];
+  __shared__ uint32_t par[kGrpNodes];
+  const uint4 gr = d.grp[blockIdx.x];
+  const uint32_t depth = d.grp_depth[blockIdx.x];
+  const uint32_t *chain = d.chain + d.chain_off[gr.z];
+  const float2 *fp = d.fpart + blockIdx.y * (size_t)d.n_far_items * CC;
+  if (threadIdx.x < gr.y) par[threadIdx.x] = d.parent[gr.x + threadIdx.x] - gr.x;
+  for (uint32_t t = threadIdx.x; t < gr.y * CC; t += blockDim.x) sh[t] = far_of_node<CC>(d, fp, gr.x + t / CC, t % CC);
+  double s = 0.0;
+  for (uint32_t a0 = 0; a0 < depth; a0 += kAnc) {
+    const uint32_t na = min((uint32_t)kAnc, depth - a0);
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < na * CC; t += blockDim.x) anc[t] = far_of_node<CC>(d, fp, chain[a0 + t / CC], t % CC);
+    __syncthreads();
+    if (threadIdx.x < CC)
+      for (uint32_t i = 0; i < na; ++i) s += anc[i * CC + threadIdx.x];
+  }
+  __syncthreads();
+  if (threadIdx.x < CC) {
+    sh[threadIdx.x] = s + sh[threadIdx.x];
+    for (uint32_t i = 1; i < gr.y; ++i) sh[i * CC + threadIdx.x] = sh[par[i] * CC + threadIdx.x] + sh[i * CC + threadIdx.x];
+  }
+  __syncthreads();
+  for (uint32_t t = threadIdx.x; t < gr.w * CC; t += blockDim.x) {
+    const uint32_t k = gr.z + t / CC;
+    dst[(blockIdx.y * (size_t)d.n_leaves + k) * CC + t % CC] = sh[(d.leaves[k] - gr.x) * CC + t % CC];
+  }
 }
 
 // Far coefficients (k_0, k_1) of every far block, FP64, as float pairs (hi, lo): d the centroid
@@ -375,7 +448,6 @@ struct NearLanes {
 constexpr int kNearStages = 3;  // tiles of a warp in shared memory: one in use, two in flight
 template <int KIND, int NV>
 constexpr int kStageFloats = KIND == FACE ? 960 : 256 * NV + 96;  // of all the items of a warp
-constexpr uint32_t kFarChunk = 64;  // far blocks per far work item
 
 // float2 weights of an item of ns rows and ncol columns, a multiple of 8
 template <int KIND>
@@ -655,36 +727,20 @@ __global__ void __launch_bounds__(128, 4) hm_rows_kernel(HDev d, RowsGrid gr, ui
   else if (w < gr.warps[1]) rows_items<KIND, 1, PLAIN, NV>(d, st, w - gr.warps[2], nb);
 }
 
-// Per (leaf, channel): the far sums along the leaf's chain (root to leaf), FP64, shared by the
-// leaf's rows. With psi = a (CC = 2, ONES) the same sums give the far part of H~a per leaf.
-template <int CC>
-__global__ void hm_chain_sum_kernel(HDev d, const double *__restrict__ src, double *__restrict__ dst) {
-  size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (t >= (size_t)d.n_leaves * CC) return;
-  const int k = (int)(t / CC), c = (int)(t % CC);
-  double s = 0.0;
-  src += blockIdx.y * (size_t)d.n_nodes * CC;
-  for (uint32_t ci = d.chain_off[k]; ci < d.chain_off[k + 1]; ++ci) s += src[(size_t)d.chain[ci] * CC + c];
-  dst[blockIdx.y * (size_t)d.n_leaves * CC + t] = s;
-}
-
-// Per (row, channel): z = near + (m_p H~a_far - H~(a m)_far), the near sums of the leaf's
+// Per (element, channel): z = near + (m_p H~a_far - H~(a m)_far), the near sums of the leaf's
 // items (in item order, as float pairs) plus the leaf's chain sums of the far field (FP64,
-// hm_chain_sum_kernel). The far part of H~a was summed with the same operations from psi = a,
-// so m = 1 gives z = 0 exactly.
+// hm_chain_sum_kernel), rounded to a float pair's 48 bits. The far part of H~a was summed with the
+// same operations from psi = a, so m = 1 gives z = 0 exactly.
 template <int SEL>
 __global__ void hm_epilogue_kernel(HDev d) {
   constexpr int CC = kChannels<SEL>;
   const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  const size_t row = t / CC;
-  const int c = (int)(t - row * CC);
-  const uint32_t k = (uint32_t)(row >> 3), r = (uint32_t)(row & 7);
-  if (k >= (uint32_t)d.n_leaves) return;
+  const uint32_t p = (uint32_t)(t / CC);
+  const int c = (int)(t - (size_t)p * CC);
+  if (p >= (uint32_t)d.n_el) return;
   if (SEL == VERTEX_CH && c == 3) return;  // padding
-  const uint32_t leaf = d.leaves[k];
-  const uint32_t s0 = d.start[leaf];
-  if (r >= d.end[leaf] - s0) return;
-  const size_t p = blockIdx.y * (size_t)d.n_el + s0 + r;
+  const uint32_t k = d.leaf_of[p], r = p - d.start[d.leaves[k]];
+  double *z = d.z + (blockIdx.y * (size_t)d.n_el + p) * CC + c;
   const float2 *part = d.part + blockIdx.y * (size_t)d.n_items * 8 * CC;
   float nh = 0.f, nl = 0.f;
   for (uint32_t i = d.item_off[k]; i < d.item_off[k + 1]; ++i) {
@@ -692,25 +748,29 @@ __global__ void hm_epilogue_kernel(HDev d) {
     pair_add(nh, nl, v.x, v.y);
   }
   const double2 fa = d.leaf_farA[k];
-  const float2 mv = m_get<SEL>(d.m + p * (2 * CC), c);
-  const double far = ((double)mv.x + (double)mv.y) * (uses_k1<SEL>(c) ? fa.y : fa.x) -
-                     d.leafsum[(blockIdx.y * (size_t)d.n_leaves + k) * CC + c];
-  const double zz = ((double)nh + (double)nl) + far;
-  const float zh = (float)zz;
-  d.z[p * CC + c] = make_float2(zh, (float)(zz - (double)zh));
+  const double far = *z * (uses_k1<SEL>(c) ? fa.y : fa.x) - d.leafsum[(blockIdx.y * (size_t)d.n_leaves + k) * CC + c];
+  const double zz = (f2d(nh) + f2d(nl)) + far;
+  const double zh = rn24(zz);
+  *z = zh + rn24(zz - zh);
+}
+
+// leaf_of[p] = k for the elements p of leaf k
+__global__ void leaf_of_kernel(uint32_t nl, const uint32_t *__restrict__ leaves, const uint32_t *__restrict__ start,
+                               const uint32_t *__restrict__ end, uint32_t *leaf_of) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nl) return;
+  for (uint32_t p = start[leaves[k]]; p < end[leaves[k]]; ++p) leaf_of[p] = k;
 }
 
 // ------------------------------------------------------------------ face prologue / epilogue
 
-struct FaceOps {
-  const uint32_t *faces;   // 3F original order
-  const uint32_t *order;   // BVH position -> face
-  const uint32_t *position;  // face -> BVH position
+struct FaceOps {  // the faces in BVH order
+  const uint32_t *faces;   // 3 per face
   // FP64 both: the gradient rows of a face sum to zero and the area-weighted rows around a
   // vertex sum to zero, and a smooth input leaves only what survives those cancellations
-  const double *g;         // 9 per face (original order): g_c (df_coefficients, mod.rs:120-131)
+  const double *g;         // 9 per face: g_c (df_coefficients, mod.rs:120-131)
   const double *area;      // per face
-  const uint32_t *inc_off, *inc;  // vertex -> (face << 2 | corner), faces ascending
+  const uint32_t *inc_off, *inc;  // vertex -> (BVH position << 2 | corner), faces by ascending index
   int nv, nf;
 };
 
@@ -725,109 +785,149 @@ struct FaceOps {
 __device__ __forceinline__ double pow2(int k) {  // 2^k, from the bits when it is a normal number
   return (k >= -1022 && k <= 1023) ? __longlong_as_double((long long)(k + 1023) << 52) : ldexp(1.0, k);
 }
+// The rounding to the grid is the addition of 1.5 2^52 Q and its subtraction (|v| < 2^51 Q), and
+// the integer k stands in the low word of the sum.
 __device__ __forceinline__ float2 split_q(double v, unsigned long long qbits) {
   const unsigned hw = (unsigned)(qbits >> 32);
   if (hw == 0u) return make_float2(0.f, 0.f);
   const int ef = (int)((hw >> 20) & 0x7ffu);
+  if (ef - 923u < 200u) {  // 2^-100 <= max < 2^100: Q and k Q are normal FP32 numbers
+    const int e = ef - 1023;
+    const double c = __hiloint2double((int)(((unsigned)(e + 30 + 1023) << 20) | 0x80000u), 0);  // 1.5 2^52 Q
+    const double t = v + c, hi = t - c;
+    const float kq = (float)__double2loint(t) * __uint_as_float((unsigned)(e - 22 + 127) << 23);
+    return make_float2(kq, (float)(v - hi));
+  }
   const int e = ef ? ef - 1023 : ilogb(__longlong_as_double((long long)qbits));
   const double hi = rint(v * pow2(22 - e)) * pow2(e - 22);
   return make_float2((float)hi, (float)(v - hi));
 }
 
-// pass 0: the channels' largest magnitudes (a warp maximum of the high words, then one atomic
-// per warp and channel; every lane of the warp takes part, `act` false contributing 0);
-// pass 1: the split value
-__device__ __forceinline__ void emit(float2 &o, int c, double v, unsigned long long *qmax, int pass, bool act) {
-  if (pass == 0) {
-    unsigned a = act ? (unsigned)((unsigned long long)__double_as_longlong(fabs(v)) >> 32) : 0u;
-    a = __reduce_max_sync(0xffffffffu, a);
-    if ((threadIdx.x & 31) == 0 && a != 0u) atomicMax(qmax + c, (unsigned long long)a << 32);
-  } else if (act) {
-    o = split_q(v, qmax[c]);
+// qmax[c] = the largest high word of |v[c]| over the threads of the block with `act`
+// (every thread of the block takes part)
+template <int C>
+__device__ __forceinline__ void block_max(const double (&v)[C], bool act, unsigned long long *qmax) {
+  __shared__ unsigned sh[C][8];
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const unsigned a = __reduce_max_sync(0xffffffffu, act ? (unsigned)__double2hiint(v[c]) & 0x7fffffffu : 0u);
+    if ((threadIdx.x & 31) == 0) sh[c][threadIdx.x >> 5] = a;
+  }
+  __syncthreads();
+  if (threadIdx.x < C) {
+    unsigned a = 0u;
+    for (unsigned w = 0; w < blockDim.x / 32; ++w) a = max(a, sh[threadIdx.x][w]);
+    if (a != 0u) atomicMax(qmax + threadIdx.x, (unsigned long long)a << 32);
   }
 }
 
-// m per face in BVH order (FaceMetricTree::product, hierarchical.rs:711-746), in FP64 and
-// stored as float pairs; channels 3k + r = sum_c x[3 t_c + k] g_c[r] (gradient) and 9 + k =
-// (x_0 + x_1 + x_2)/3 for axis k (average; the division by 3 is a product with the rounded 1/3,
-// within an FP64 unit of the quotient, far below the float pairs' resolution). blockIdx.y is
-// the vector.
-__global__ void face_m_kernel(FaceOps o, const double *__restrict__ xs, size_t ldx, float *m, unsigned long long *qmax,
-                              int pass) {
+// The channel values per face in BVH order (FaceMetricTree::product, hierarchical.rs:711-746), in
+// FP64, and the channels' largest magnitudes; channels 3k + r = sum_c x[3 t_c + k] g_c[r]
+// (gradient) and 9 + k = (x_0 + x_1 + x_2)/3 for axis k (average; the division by 3 is a product
+// with the rounded 1/3, within an FP64 unit of the quotient, far below the float pairs'
+// resolution). blockIdx.y is the vector.
+__global__ void __launch_bounds__(256) face_m_kernel(FaceOps o, const double *__restrict__ xs, size_t ldx,
+                                                     double *__restrict__ z, unsigned long long *qmax) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
-  const bool act = p < o.nf;  // the whole warp runs the loops (warp maxima in pass 0)
-  const uint32_t f = act ? o.order[p] : 0;
-  const uint32_t *t = o.faces + 3 * (size_t)f;
-  const double *g = o.g + 9 * (size_t)f;
+  const bool act = p < o.nf;
+  const uint32_t *t = o.faces + 3 * (size_t)(act ? p : 0);
+  const double *g = o.g + 9 * (size_t)(act ? p : 0);
   const double *x = xs + q * ldx;
-  float2 v[12];
+  double v[12];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const double x0 = x[3 * (size_t)t[0] + k], x1 = x[3 * (size_t)t[1] + k], x2 = x[3 * (size_t)t[2] + k];
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
-      emit(v[3 * k + r], 12 * q + 3 * k + r, x0 * g[r] + x1 * g[3 + r] + x2 * g[6 + r], qmax, pass, act);
-    emit(v[9 + k], 12 * q + 9 + k, ((x0 + x1) + x2) * (1.0 / 3.0), qmax, pass, act);
+    for (int r = 0; r < 3; ++r) v[3 * k + r] = x0 * g[r] + x1 * g[3 + r] + x2 * g[6 + r];
+    v[9 + k] = ((x0 + x1) + x2) * (1.0 / 3.0);
   }
-  if (pass == 1 && act) m_store<12>(m + ((size_t)q * o.nf + p) * 24, v);
+  block_max<12>(v, act, qmax + 12 * q);
+  if (act) {
+    double2 *zp = reinterpret_cast<double2 *>(z + ((size_t)q * o.nf + p) * 12);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) zp[i] = make_double2(v[2 * i], v[2 * i + 1]);
+  }
 }
 
-// y_v = 2 sum_{S ni v} a_S (w_hi g_c . z_hi + w_lo z_lo / 3) in FP64 (hierarchical.rs:779-811).
-__global__ void face_gather_kernel(FaceOps o, const float2 *__restrict__ z, double w_hi, double w_lo,
+// The channel values split into float pairs: m, and in z their sum hi + lo in FP64 in
+// place of the values; one thread per four channels of an element, blockIdx.y the vector.
+template <int CC>
+__global__ void split_m_kernel(size_t n_el, double *__restrict__ z, float *__restrict__ m,
+                               const unsigned long long *__restrict__ qmax) {
+  constexpr int NC = CC == 4 ? 3 : CC;  // channels that have a magnitude (the fourth of vertices is zero)
+  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const size_t p = t / (CC / 4);
+  const int c0 = 4 * (int)(t - p * (CC / 4));
+  if (p >= n_el) return;
+  double2 *zp = reinterpret_cast<double2 *>(z + (blockIdx.y * n_el + p) * CC + c0);
+  const double2 a = zp[0], b = zp[1];
+  const double v[4] = {a.x, a.y, b.x, b.y};
+  float2 w[4];
+  double s[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    w[i] = c0 + i < NC ? split_q(v[i], qmax[blockIdx.y * NC + c0 + i]) : make_float2(0.f, 0.f);
+    s[i] = f2d(w[i].x) + f2d(w[i].y);
+  }
+  zp[0] = make_double2(s[0], s[1]), zp[1] = make_double2(s[2], s[3]);
+  float *f = m + (blockIdx.y * n_el + p) * (2 * CC) + c0;
+  *reinterpret_cast<float4 *>(f) = make_float4(w[0].x, w[1].x, w[2].x, w[3].x);
+  *reinterpret_cast<float4 *>(f + CC) = make_float4(w[0].y, w[1].y, w[2].y, w[3].y);
+}
+
+// y_v = 2 sum_{S ni v} a_S (w_hi g_c . z_hi + w_lo z_lo / 3) in FP64 (hierarchical.rs:779-811), the
+// multiply-adds written out so that every build rounds alike (a flow's solves magnify a last bit).
+__global__ void face_gather_kernel(FaceOps o, const double *__restrict__ z, double w_hi, double w_lo,
                                    double *__restrict__ ys, size_t ldy) {
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= o.nv) return;
-  {
-    const int q = blockIdx.y;
-    double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
-    for (uint32_t e = o.inc_off[v]; e < o.inc_off[v + 1]; ++e) {
-      uint32_t fc = o.inc[e], f = fc >> 2, c = fc & 3;
-      double a = o.area[f];
-      const double *g = o.g + 9 * (size_t)f + 3 * c;
-      const float2 *zs = z + ((size_t)q * o.nf + o.position[f]) * 12;
-      double acc[3];
-      for (int k = 0; k < 3; ++k) {
-        const float2 *zh = zs + 3 * k;
-        double hi = g[0] * ((double)zh[0].x + zh[0].y) + g[1] * ((double)zh[1].x + zh[1].y) +
-                    g[2] * ((double)zh[2].x + zh[2].y);
-        double lo = (double)zs[9 + k].x + zs[9 + k].y;
-        acc[k] = a * (w_hi * hi + w_lo * (1.0 / 3.0) * lo);
-      }
-      acc0 += acc[0], acc1 += acc[1], acc2 += acc[2];
+  const int q = blockIdx.y;
+  double acc[3] = {0.0, 0.0, 0.0};
+  const double wl = __dmul_rn(w_lo, 1.0 / 3.0);
+  for (uint32_t e = o.inc_off[v]; e < o.inc_off[v + 1]; ++e) {
+    uint32_t pc = o.inc[e], p = pc >> 2, c = pc & 3;
+    double a = o.area[p];
+    const double *g = o.g + 9 * (size_t)p + 3 * c;
+    const double *zs = z + ((size_t)q * o.nf + p) * 12;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double *zh = zs + 3 * k;
+      const double hi = __fma_rn(g[2], zh[2], __fma_rn(g[0], zh[0], __dmul_rn(g[1], zh[1])));
+      acc[k] = __fma_rn(a, __fma_rn(w_hi, hi, __dmul_rn(wl, zs[9 + k])), acc[k]);
     }
-    double *y = ys + q * ldy + 3 * (size_t)v;
-    y[0] = 2.0 * acc0, y[1] = 2.0 * acc1, y[2] = 2.0 * acc2;
   }
+  double *y = ys + q * ldy + 3 * (size_t)v;
+  y[0] = 2.0 * acc[0], y[1] = 2.0 * acc[1], y[2] = 2.0 * acc[2];
 }
 
 // ------------------------------------------------------------------ vertex prologue / epilogue
 
 // Channels of the vertex operator: m = x per axis (psi = a x in the upward sums); blockIdx.y is
 // the vector.
-__global__ void vertex_m_kernel(const uint32_t *order, const double *__restrict__ xs, size_t ldx, int nv, float *m,
-                                unsigned long long *qmax, int pass) {
+__global__ void __launch_bounds__(256) vertex_m_kernel(const uint32_t *order, const double *__restrict__ xs, size_t ldx,
+                                                       int nv, double *__restrict__ z, unsigned long long *qmax) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
-  const bool act = p < nv;  // the whole warp runs the loops (warp maxima in pass 0)
+  const bool act = p < nv;
   const uint32_t v = act ? order[p] : 0;
-  float2 mv[4];
-  mv[3] = make_float2(0.f, 0.f);
+  double x[3];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) emit(mv[k], 3 * q + k, xs[q * ldx + 3 * (size_t)v + k], qmax, pass, act);
-  if (pass == 1 && act) m_store<4>(m + ((size_t)q * nv + p) * 8, mv);
+  for (int k = 0; k < 3; ++k) x[k] = xs[q * ldx + 3 * (size_t)v + k];
+  block_max<3>(x, act, qmax + 3 * q);
+  if (act) {
+    double2 *zp = reinterpret_cast<double2 *>(z + ((size_t)q * nv + p) * 4);
+    zp[0] = make_double2(x[0], x[1]), zp[1] = make_double2(x[2], 0.0);
+  }
 }
 
 // y = 2 a (H~a x - H~(a x)) = 2 a z (hierarchical.rs:1330-1343).
-__global__ void vertex_out_kernel(const uint32_t *order, const float4 *el, const float2 *z, int nv, double scale,
+__global__ void vertex_out_kernel(const uint32_t *order, const float4 *el, const double *z, int nv, double scale,
                                   double *__restrict__ ys, size_t ldy) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= nv) return;
   const int q = blockIdx.y;
   uint32_t v = order[p];
   double a = el[p].w;
-  for (int k = 0; k < 3; ++k) {
-    const float2 zz = z[((size_t)q * nv + p) * 4 + k];
-    ys[q * ldy + 3 * (size_t)v + k] = scale * 2.0 * a * ((double)zz.x + zz.y);
-  }
+  for (int k = 0; k < 3; ++k) ys[q * ldy + 3 * (size_t)v + k] = scale * 2.0 * a * z[((size_t)q * nv + p) * 4 + k];
 }
 
 // Element records: positions as float pairs (hi + lo), weights, normals; FP64 in.
@@ -983,7 +1083,23 @@ struct HMat {
   size_t n_el = 0, n_items = 0;
   double neg_s = 0;
   DevBuf<uint32_t> start, end, right, parent, leaves, chain_off, chain, item_off;
-  DevBuf<uint32_t> count, far_item_off;
+  DevBuf<uint32_t> far_item_off, leaf_of;
+  // the groups of the upward sums: the bottom ones, and the levels above (see hm_upward_kernel)
+  DevBuf<uint4> grp;
+  DevBuf<uint32_t> grp_depth;
+  struct Level {
+    DevBuf<uint4> groups;
+    DevBuf<uint32_t> ext, inner;
+    DevBuf<uint2> child;
+  };
+  std::vector<Level> levels;
+  // the far passes run on the context's second stream beside the near field
+  struct Event {
+    cudaEvent_t e = nullptr;
+    ~Event() {
+      if (e) cudaEventDestroy(e);
+    }
+  } ev_fork, ev_join;
   DevBuf<uint4> far_items;
   size_t n_far_items = 0;
   DevBuf<float2> fpart;
@@ -997,9 +1113,9 @@ struct HMat {
   DevBuf<double2> leaf_farA;
   DevBuf<double> leafsum;
   DevBuf<float4> xh, xl, nrm;
-  DevBuf<double> up, farx;
+  DevBuf<double> up, z;
   DevBuf<float2> up2;
-  DevBuf<float2> part, m, z;  // m: channel values (2 C floats per element)
+  DevBuf<float2> part, m;  // m: channel values (2 C floats per element)
   DevBuf<unsigned long long> qmax;  // per channel: largest |m| (see split_q)
   int pw_mode = 0, pw_k = 0;
   bool plain_rows = false;  // the near field of the next product in plain FP32 sums (inner operator)
@@ -1017,7 +1133,8 @@ struct HMat {
     d.colidx = colidx.p, d.items = items.p, d.item_off = item_off.p, d.wts = wts.p;
     d.sched = sched.p;
     std::copy(sched_off, sched_off + 9, d.sched_off);
-    d.up = up.p, d.up2 = up2.p, d.farx = farx.p, d.part = part.p, d.count = count.p, d.leafsum = leafsum.p;
+    d.up = up.p, d.up2 = up2.p, d.part = part.p, d.leafsum = leafsum.p;
+    d.leaf_of = leaf_of.p, d.grp = grp.p, d.grp_depth = grp_depth.p, d.n_grp = (int)grp.n;
     d.m = reinterpret_cast<const float *>(m.p), d.z = z.p;
     d.n_nodes = (int)tree.n_nodes(), d.n_leaves = (int)tree.leaves.size(), d.n_el = (int)n_el;
     d.n_items = (int)n_items;
@@ -1030,7 +1147,7 @@ struct HMat {
   // Channel scratch for C channels.
   void reserve(int C_) {
     size_t nn = tree.n_nodes();
-    if ((size_t)C_ * nn > up.n) up.alloc((size_t)C_ * nn), up2.alloc((size_t)C_ * nn), farx.alloc((size_t)C_ * nn);
+    if ((size_t)C_ * nn > up.n) up.alloc((size_t)C_ * nn), up2.alloc((size_t)C_ * nn);
     if ((size_t)C_ * n_far_items > fpart.n) fpart.alloc(std::max<size_t>((size_t)C_ * n_far_items, 1));
     if ((size_t)C_ * tree.leaves.size() > leafsum.n) leafsum.alloc((size_t)C_ * tree.leaves.size());
     if ((size_t)C_ * n_el > m.n) m.alloc((size_t)C_ * n_el), z.alloc((size_t)C_ * n_el);
@@ -1051,28 +1168,94 @@ struct HMat {
     }
   }
 
+  // the upward sums, the far sums and the chain sums (into dst) on stream s
   template <int SEL>
-  void upward_far(const HDev &d, int nb) {
+  void upward_far(const HDev &d, int nb, double *dst, cudaStream_t s) {
     constexpr int CC = kChannels<SEL>;
     const unsigned gy = (unsigned)nb;
-    size_t nn = tree.n_nodes(), nl = tree.leaves.size();
-    cudaStream_t s = st();
     prof.begin(s, kind == FACE ? "metric_upward" : "vfrac_upward");
-    hm_upward_kernel<SEL><<<dim3(nblk(nl * 32, 128), gy), 128, 0, s>>>(d);
+    hm_upward_kernel<SEL><<<dim3((unsigned)d.n_grp, gy), 192, 0, s>>>(d);
     RSG_LAUNCHED(ctx, "hm_upward");
+    for (const Level &l : levels) {
+      hm_upward_level_kernel<CC><<<dim3((unsigned)l.groups.n, gy), 128, 0, s>>>(d, l.groups.p, l.ext.p, l.inner.p, l.child.p);
+      RSG_LAUNCHED(ctx, "hm_upward");
+    }
     prof.end(s);
     prof.begin(s, kind == FACE ? "metric_far" : "vfrac_far");
     if (n_far_items > 0) {  // chi = 0 (all near) has none
-      hm_far_kernel<SEL><<<dim3(nblk(n_far_items * 32, 256), gy), 256, 0, s>>>(d);
+      hm_far_kernel<SEL><<<nblk(n_far_items * 32, 256), 256, 0, s>>>(d, nb);
       RSG_LAUNCHED(ctx, "hm_far");
     }
-    hm_far_final_kernel<CC><<<dim3(nblk(nn * CC, 256), gy), 256, 0, s>>>(d);
-    RSG_LAUNCHED(ctx, "hm_far_final");
-    if (SEL != ONES) {
-      hm_chain_sum_kernel<CC><<<dim3(nblk(nl * CC, 256), gy), 256, 0, s>>>(d, d.farx, d.leafsum);
-      RSG_LAUNCHED(ctx, "hm_chain_sum");
-    }
+    hm_chain_sum_kernel<SEL><<<dim3((unsigned)d.n_grp, gy), 192, 0, s>>>(d, dst);
+    RSG_LAUNCHED(ctx, "hm_chain_sum");
     prof.end(s);
+  }
+
+  // The groups of the upward sums (see hm_upward_kernel), from the tree.
+  void build_groups() {
+    const Tree &T = tree;
+    const size_t nn = T.n_nodes();
+    cudaStream_t s = st();
+    std::vector<uint32_t> size(nn, 1);
+    for (size_t i = nn; i-- > 0;)
+      if (T.right[i]) size[i] = 1 + size[i + 1] + size[T.right[i]];
+    std::vector<uint4> g;
+    std::vector<uint32_t> depth;
+    // the nodes not yet inside a group in preorder, each with whether it is a root of one
+    std::vector<std::pair<uint32_t, bool>> cur, next;
+    std::vector<uint32_t> ends;  // ends of the subtrees of the current node's ancestors
+    for (uint32_t n = 0, k = 0; n < nn;) {
+      while (!ends.empty() && ends.back() <= n) ends.pop_back();
+      if ((size[n] + 1) / 2 <= (uint32_t)kGrpLeaves) {
+        const uint32_t nl = (size[n] + 1) / 2;
+        g.push_back(make_uint4(n, size[n], k, nl));
+        depth.push_back((uint32_t)ends.size());
+        cur.push_back({n, true});
+        k += nl, n += size[n];
+      } else {
+        cur.push_back({n, false});
+        ends.push_back(n + size[n]);
+        ++n;
+      }
+    }
+    up_vec(grp, g, s), up_vec(grp_depth, depth, s);
+    levels.clear();
+    while (cur.size() > 1) {
+      const size_t m = cur.size();
+      std::vector<uint32_t> roots(m + 1, 0);  // roots before each entry
+      for (size_t i = 0; i < m; ++i) roots[i + 1] = roots[i] + (cur[i].second ? 1u : 0u);
+      std::vector<uint4> groups;
+      std::vector<uint32_t> ext, inner, slot(nn);
+      std::vector<uint2> child;
+      next.clear();
+      for (size_t i = 0; i < m;) {
+        const uint32_t n = cur[i].first;
+        const size_t j = (size_t)(std::lower_bound(cur.begin() + i, cur.end(), std::make_pair(n + size[n], false)) - cur.begin());
+        if (cur[i].second || roots[j] - roots[i] > (uint32_t)kGrpExt) {
+          next.push_back(cur[i++]);
+          continue;
+        }
+        uint4 gr = make_uint4((uint32_t)ext.size(), 0, (uint32_t)inner.size(), 0);
+        for (size_t a = i; a < j; ++a)
+          if (cur[a].second) slot[cur[a].first] = gr.y++, ext.push_back(cur[a].first);
+        for (size_t a = j; a-- > i;)
+          if (!cur[a].second) {
+            const uint32_t v = cur[a].first;
+            inner.push_back(v);
+            child.push_back(make_uint2(slot[v + 1], slot[T.right[v]]));
+            slot[v] = gr.y + gr.w++;
+          }
+        groups.push_back(gr);
+        next.push_back({n, true});
+        i = j;
+      }
+      levels.emplace_back();
+      Level &l = levels.back();
+      up_vec(l.groups, groups, s), up_vec(l.ext, ext, s), up_vec(l.inner, inner, s), up_vec(l.child, child, s);
+      RSG_CUDA("upload", cudaStreamSynchronize(s));  // before the staging vectors go
+      cur.swap(next);
+    }
+    RSG_CUDA("upload", cudaStreamSynchronize(s));
   }
 
   // Uploads the tree, the near column ranges split into work items, the element records and
@@ -1188,8 +1371,12 @@ struct HMat {
       far_fill_kernel<<<nblk(nn, 256), 256, 0, s>>>((uint32_t)nn, blocks.far_ptr.p, far_item_off.p, far_items.p);
       RSG_LAUNCHED(ctx, "hm_far_items");
     }
-    count.alloc(3 * nn);  // one set per vector of a pass
-    RSG_CUDA("upload", cudaMemsetAsync(count.p, 0, 3 * nn * sizeof(uint32_t), s));
+    leaf_of.alloc(n_el);
+    leaf_of_kernel<<<nblk(nl, 128), 128, 0, s>>>((uint32_t)nl, leaves.p, start.p, end.p, leaf_of.p);
+    RSG_LAUNCHED(ctx, "hm_leaf_of");
+    build_groups();
+    RSG_CUDA("upload", cudaEventCreateWithFlags(&ev_fork.e, cudaEventDisableTiming));
+    RSG_CUDA("upload", cudaEventCreateWithFlags(&ev_join.e, cudaEventDisableTiming));
     // far coefficients (kernel.far, hierarchical.rs:210-220 / 980-984) in FP64 on the device
     // from the node centroids (and, for faces, the node projectors)
     {
@@ -1229,10 +1416,8 @@ struct HMat {
     // far part of H~a: upward over psi = a (m = 1, 2 channels) and far sums per node
     reserve(4);
     HDev d = dev();
-    upward_far<ONES>(d, 1);
     leaf_farA.alloc(std::max<size_t>(nl, 1));
-    hm_chain_sum_kernel<2><<<nblk(nl * 2, 256), 256, 0, s>>>(d, farx.p, reinterpret_cast<double *>(leaf_farA.p));
-    RSG_LAUNCHED(ctx, "hm_chain_sum");
+    upward_far<ONES>(d, 1, reinterpret_cast<double *>(leaf_farA.p), s);
     RSG_CUDA("upload", cudaStreamSynchronize(s));
     lap(setup_times[2]);
   }
@@ -1265,19 +1450,31 @@ struct HMat {
     else rows<VERTEX, PLAIN, 3>(d, nb);
   }
 
-  // z of the nb vectors whose channel values are already in `m`.
+  // z of the nb vectors whose channel values are already in `z`: the far passes (latency, FP64 and
+  // gathers) on the second stream beside the near field (FP32 and shared memory), unless the kernels
+  // are being timed one by one
   template <int K>
-  void product_on(const HDev &d, int nb) {
+  void product_on(const HDev &d, int nb, const unsigned long long *qmax_) {
     cudaStream_t s = st();
-    constexpr int SEL = K == FACE ? FACE_CH : VERTEX_CH;
-    upward_far<SEL>(d, nb);
+    constexpr int SEL = K == FACE ? FACE_CH : VERTEX_CH, CC = kChannels<SEL>;
+    prof.begin(s, K == FACE ? "metric_m" : "vfrac_m");
+    split_m_kernel<CC><<<dim3(nblk(n_el * (CC / 4), 256), (unsigned)nb), 256, 0, s>>>(n_el, d.z, const_cast<float *>(d.m), qmax_);
+    RSG_LAUNCHED(ctx, "split_m");
+    prof.end(s);
+    cudaStream_t far = prof.active ? s : ctx->stream2;
+    if (far != s) {
+      RSG_CUDA("product", cudaEventRecord(ev_fork.e, s));
+      RSG_CUDA("product", cudaStreamWaitEvent(far, ev_fork.e, 0));
+    }
+    upward_far<SEL>(d, nb, d.leafsum, far);
+    if (far != s) RSG_CUDA("product", cudaEventRecord(ev_join.e, far));
     prof.begin(s, K == FACE ? "metric_rows" : "vfrac_rows");
     if (plain_rows) rows_any<true>(d, nb);
     else rows_any<false>(d, nb);
     prof.end(s);
+    if (far != s) RSG_CUDA("product", cudaStreamWaitEvent(s, ev_join.e, 0));
     prof.begin(s, K == FACE ? "metric_epilogue" : "vfrac_epilogue");
-    // z from the near partial sums and the far chain sums (one thread per row and channel)
-    hm_epilogue_kernel<SEL><<<dim3(nblk(tree.leaves.size() * 8 * kChannels<SEL>, 256), (unsigned)nb), 256, 0, s>>>(d);
+    hm_epilogue_kernel<SEL><<<dim3(nblk(n_el * CC, 256), (unsigned)nb), 256, 0, s>>>(d);
     RSG_LAUNCHED(ctx, "hm_epilogue");
     prof.end(s);
   }
@@ -1308,12 +1505,12 @@ struct rs_metric {
   // far coefficients, device part (uploads, element records, weights, far part of H~a)
   double build_times[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   FaceGeom geom;
-  DevBuf<uint32_t> faces, order, position, inc_off, inc;
+  DevBuf<uint32_t> faces, inc_off, inc;
   DevBuf<double> g, area;
   DevBuf<double> xbuf, ybuf;
   FaceOps ops() const {
     FaceOps o;
-    o.faces = faces.p, o.order = order.p, o.position = position.p, o.g = g.p, o.area = area.p;
+    o.faces = faces.p, o.g = g.p, o.area = area.p;
     o.inc_off = inc_off.p, o.inc = inc.p, o.nv = nv, o.nf = nf;
     return o;
   }
@@ -1377,7 +1574,11 @@ void metric_setup(rs_metric *M, rs_ctx *ctx, int nv, int nf, const uint32_t *fac
   cudaStream_t s = M->h.st();
   // df coefficients (RS/src/metric/mod.rs:120-131) in FP64
   std::vector<double> gh(9 * (size_t)nf), ah(nf);
-  for (int f = 0; f < nf; ++f) {
+  std::vector<uint32_t> fh(3 * (size_t)nf), posn(nf);
+  for (int pp = 0; pp < nf; ++pp) {
+    const uint32_t f = M->h.tree.order[pp];
+    posn[f] = (uint32_t)pp;
+    std::copy(faces + 3 * (size_t)f, faces + 3 * (size_t)f + 3, fh.begin() + 3 * (size_t)pp);
     const double *p0 = pos + 3 * (size_t)faces[3 * f], *p1 = pos + 3 * (size_t)faces[3 * f + 1],
                  *p2 = pos + 3 * (size_t)faces[3 * f + 2];
     double u[3], w[3], n[3];
@@ -1389,14 +1590,12 @@ void metric_setup(rs_metric *M, rs_ctx *ctx, int nv, int nf, const uint32_t *fac
     const double *pa[3] = {p1, p2, p0}, *pb[3] = {p2, p0, p1};
     for (int c = 0; c < 3; ++c) {
       double e[3] = {pb[c][0] - pa[c][0], pb[c][1] - pa[c][1], pb[c][2] - pa[c][2]};
-      gh[9 * f + 3 * c + 0] = ww[1] * e[2] - ww[2] * e[1];
-      gh[9 * f + 3 * c + 1] = ww[2] * e[0] - ww[0] * e[2];
-      gh[9 * f + 3 * c + 2] = ww[0] * e[1] - ww[1] * e[0];
+      gh[9 * (size_t)pp + 3 * c + 0] = ww[1] * e[2] - ww[2] * e[1];
+      gh[9 * (size_t)pp + 3 * c + 1] = ww[2] * e[0] - ww[0] * e[2];
+      gh[9 * (size_t)pp + 3 * c + 2] = ww[0] * e[1] - ww[1] * e[0];
     }
-    ah[f] = M->geom.area[f];
+    ah[pp] = M->geom.area[f];
   }
-  std::vector<uint32_t> fh(faces, faces + 3 * (size_t)nf), posn(nf);
-  for (int p = 0; p < nf; ++p) posn[M->h.tree.order[p]] = (uint32_t)p;
   std::vector<uint32_t> ioff((size_t)nv + 1, 0), inc(3 * (size_t)nf);
   for (int f = 0; f < nf; ++f)
     for (int c = 0; c < 3; ++c) ioff[faces[3 * f + c] + 1]++;
@@ -1404,9 +1603,9 @@ void metric_setup(rs_metric *M, rs_ctx *ctx, int nv, int nf, const uint32_t *fac
   {
     std::vector<uint32_t> fill(ioff.begin(), ioff.end() - 1);
     for (int f = 0; f < nf; ++f)
-      for (int c = 0; c < 3; ++c) inc[fill[faces[3 * f + c]]++] = ((uint32_t)f << 2) | c;
+      for (int c = 0; c < 3; ++c) inc[fill[faces[3 * f + c]]++] = (posn[f] << 2) | c;
   }
-  up_vec(M->faces, fh, s), up_vec(M->order, M->h.tree.order, s), up_vec(M->position, posn, s);
+  up_vec(M->faces, fh, s);
   up_vec(M->g, gh, s), up_vec(M->area, ah, s), up_vec(M->inc_off, ioff, s), up_vec(M->inc, inc, s);
   lap(4);
   M->h.setup(M->geom.bary.data(), M->geom.area.data(), M->geom.normal.data(), proj.data());
@@ -1423,12 +1622,10 @@ static void face_product(rs_metric *M, const HDev &d, unsigned long long *qmax, 
   const unsigned gy = (unsigned)k;
   h.prof.begin(s, "metric_m");
   RSG_CUDA("product", cudaMemsetAsync(qmax, 0, 12 * k * sizeof(unsigned long long), s));
-  for (int pass = 0; pass < 2; ++pass) {
-    face_m_kernel<<<dim3(nblk(M->nf, 256), gy), 256, 0, s>>>(M->ops(), xs, ldx, const_cast<float *>(d.m), qmax, pass);
-    RSG_LAUNCHED(h.ctx, "face_m");
-  }
+  face_m_kernel<<<dim3(nblk(M->nf, 256), gy), 256, 0, s>>>(M->ops(), xs, ldx, d.z, qmax);
+  RSG_LAUNCHED(h.ctx, "face_m");
   h.prof.end(s);
-  h.product_on<FACE>(d, k);
+  h.product_on<FACE>(d, k, qmax);
   h.prof.begin(s, "metric_gather");
   face_gather_kernel<<<dim3(nblk(M->nv, 128), gy), 128, 0, s>>>(M->ops(), d.z, w_hi, w_lo, ys, ldy);
   RSG_LAUNCHED(h.ctx, "face_gather");
@@ -1463,13 +1660,11 @@ void rsg::vfrac_apply_strided(rs_vfrac *V, double scale, int nb, const double *x
     if (V->h.qmax.n < 64) V->h.qmax.alloc(64);
     const HDev d = V->h.dev();
     RSG_CUDA("product", cudaMemsetAsync(V->h.qmax.p, 0, 3 * k * sizeof(unsigned long long), s));
-    for (int pass = 0; pass < 2; ++pass) {
-      vertex_m_kernel<<<dim3(nblk(V->nv, 256), gy), 256, 0, s>>>(V->order.p, xs + q0 * ldx, ldx, V->nv,
-                                                                 const_cast<float *>(d.m), V->h.qmax.p, pass);
-      RSG_LAUNCHED(V->h.ctx, "vertex_m");
-    }
-    V->h.product_on<VERTEX>(d, k);
-    vertex_out_kernel<<<dim3(nblk(V->nv, 256), gy), 256, 0, s>>>(V->order.p, V->h.xh.p, V->h.z.p, V->nv, scale,
+    vertex_m_kernel<<<dim3(nblk(V->nv, 256), gy), 256, 0, s>>>(V->order.p, xs + q0 * ldx, ldx, V->nv, d.z,
+                                                               V->h.qmax.p);
+    RSG_LAUNCHED(V->h.ctx, "vertex_m");
+    V->h.product_on<VERTEX>(d, k, V->h.qmax.p);
+    vertex_out_kernel<<<dim3(nblk(V->nv, 256), gy), 256, 0, s>>>(V->order.p, V->h.xh.p, d.z, V->nv, scale,
                                                                  ys + q0 * ldy, ldy);
     RSG_LAUNCHED(V->h.ctx, "vertex_out");
   }
@@ -1651,8 +1846,8 @@ int rs_vfrac_stats(rs_vfrac *V, int64_t *o) {
 //
 // Limits: the scratch is kNoAllocScratchBytes per device, shared by every call in the process,
 // so calls that overlap in time (two host threads, or two streams in flight) race on it and
-// must be serialized by the caller; a call also uses the metric's own arrival counters (the
-// upward pass), so it must not overlap any other product on the same rs_metric either. The
+// must be serialized by the caller; a call also uses the metric's own events and the
+// context's second stream, so it must not overlap any other product on the same rs_metric either. The
 // array is resident on every device where this file's kernels are loaded (from the first
 // metric build or product there, with lazy module loading), whether or not this entry point
 // is ever called. The first call on a device looks up the array's address
@@ -1681,7 +1876,8 @@ unsigned char *noalloc_scratch(int device) {
 
 inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
-// Scratch bytes of one tree pass with C channels (the layout carved below).
+// Scratch bytes a call with C channels is admitted by: the layout carved below and an FP64 value
+// per node and channel beside it (not used).
 size_t noalloc_bytes(const HMat &h, int C) {
   size_t nn = h.tree.n_nodes();
   return 2 * align256(nn * C * sizeof(double)) + align256(nn * C * sizeof(float2)) +
@@ -1701,9 +1897,8 @@ HDev noalloc_dev(const HMat &h, int C, unsigned char *base) {
   };
   d.up = reinterpret_cast<double *>(take(nn * C * sizeof(double)));
   d.up2 = reinterpret_cast<float2 *>(take(nn * C * sizeof(float2)));
-  d.farx = reinterpret_cast<double *>(take(nn * C * sizeof(double)));
   d.m = reinterpret_cast<const float *>(take(h.n_el * C * sizeof(float2)));
-  d.z = reinterpret_cast<float2 *>(take(h.n_el * C * sizeof(float2)));
+  d.z = reinterpret_cast<double *>(take(h.n_el * C * sizeof(float2)));
   d.part = reinterpret_cast<float2 *>(take(std::max<size_t>(h.n_items, 1) * 8 * C * sizeof(float2)));
   d.leafsum = reinterpret_cast<double *>(take(h.tree.leaves.size() * C * sizeof(double)));
   d.fpart = reinterpret_cast<float2 *>(take(std::max<size_t>(h.n_far_items, 1) * C * sizeof(float2)));

@@ -196,7 +196,7 @@ int rs_metric_apply_device(rs_metric *m, double w_hi, double w_lo, int nb, const
  * where the library's metric kernels are loaded, whether or not this call is ever made (with
  * CUDA_MODULE_LOADING=LAZY, the CUDA default, from the first metric build or product on that
  * device). Calls that overlap in time race on the shared scratch, and a call also shares the
- * metric's arrival counters with the other products of the same rs_metric: serialize them
+ * metric's events and the context's second stream with the other products: serialize them
  * with each other and with every product on that metric. The first call on a device looks up
  * the scratch address; make that call outside any stream capture. */
 int rs_metric_apply_device_noalloc(rs_metric *m, double w_hi, double w_lo, int nb,
