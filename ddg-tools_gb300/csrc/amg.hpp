@@ -36,56 +36,52 @@ struct AmgHost {
 AmgHost amg_setup(const Csr &A, int coarse_max = 300, int max_levels = 12,
                   const std::vector<uint32_t> *groups = nullptr);
 
-// The hierarchy on the device and its V-cycle for C interleaved columns per row
-// (x[row * C + c]): pre- and post-smoothing by `sweeps` damped Jacobi steps, dense coarse solve.
-// Each sparse product gives a row to a group of 1-32 lanes sized to the matrix's mean row length
-// (the coarse operators of smoothed aggregation have 40-70 nonzeros per row on a few hundred
-// rows, where one thread per row would leave the GPU idle behind long serial loops).
+// The hierarchy on the device: conjugate gradients preconditioned by V-cycles of two damped Jacobi
+// sweeps before and after each coarser solve and a dense coarse solve, in one persistent kernel
+// (amg.cu). Each sparse product gives a row to a group of 1-32 lanes sized to the matrix's mean row
+// length (the coarse operators of smoothed aggregation have 40-70 nonzeros per row on a few
+// hundred rows, where one thread per row would leave the GPU idle behind long serial loops).
 struct AmgDevice {
+  struct Mat {  // CSR with the column and the value of a nonzero side by side
+    DevBuf<int> ptr;
+    DevBuf<int2> cv;
+    size_t nnz = 0;
+    int tpr = 1;  // lanes per row
+    void upload(const Csr &A, cudaStream_t s);
+  };
   struct Level {
     int n = 0;
-    int tpr_a = 1, tpr_r = 1, tpr_p = 1;  // lanes per row of A, R (rows of level l+1) and P
-    DevBuf<int> ap, ac, pp, pc, rp, rc;
-    DevBuf<mgreal> av, pv, rv, dinv;
-    DevBuf<mgreal> x, b, r, t;  // C columns each
+    Mat a, p, r;  // A_l, P_l (rows of level l), R_l (rows of level l + 1)
+    DevBuf<mgreal> dinv;
+    DevBuf<mgreal> x, b, res, t;  // up to 12 columns each
   };
   std::vector<Level> L;
   DevBuf<mgreal> cinv;
-  int C = 0, sweeps = 2;
   void upload(const AmgHost &h, cudaStream_t s);
-  void reserve(int C_);
-  // x = V-cycle(b) on level 0; b and x are n_0 x C device arrays (x overwritten).
-  // pre0: the first Jacobi sweep of level 0 (dinv b) is already in place.
-  void vcycle(rs_ctx *ctx, const mgreal *b, mgreal *x, int C_, bool pre0 = false);
-  // y = A_0 x for C columns.
-  void spmv0(rs_ctx *ctx, const mgreal *x, mgreal *y, int C_);
   // x ~ A_0^-1 b by `iters` steps of conjugate gradients per column, preconditioned by one
-  // V-cycle each (x_0 = 0; iters = 1 is the V-cycle with the optimal step length). The
+  // V-cycle each (x_0 = 0; iters = 1 is the V-cycle with the optimal step length), for n_0 x C
+  // device arrays, C = 3, 6, 9 or 12 interleaved columns per row (x[row * C + c]). The
   // scalars stay on the device (no host synchronization); a fixed number of steps makes it a
   // nonlinear map of b, which flexible GMRES (the stored preconditioned vectors) allows.
-  void pcg(rs_ctx *ctx, const mgreal *b, mgreal *x, int C_, int iters);
-  DevBuf<mgreal> cg_r, cg_z, cg_p, cg_q;  // n_0 x C each
-  DevBuf<double> cg_part, cg_s;           // per-block partial sums; scalars
-  DevBuf<unsigned> cg_ticket;  // blocks done in the current dot-product launch (0 between launches)
-  struct Graph {
-    const mgreal *b = nullptr;
-    mgreal *x = nullptr;
-    int C = 0, iters = 0;
-    int64_t launches = 0;
-    cudaGraphExec_t exec = nullptr;
-  };
-  std::vector<Graph> graphs;  // captured conjugate-gradient solves
+  void pcg(rs_ctx *ctx, const mgreal *b, mgreal *x, int C, int iters);
+  // fails when an earlier solve gave up at a barrier (to be called once the stream has been waited for)
+  void check() const;
   AmgDevice() = default;
   AmgDevice(const AmgDevice &) = delete;
   AmgDevice &operator=(const AmgDevice &) = delete;
   ~AmgDevice();
 
  private:
-  template <int CC>
-  void vcycle_t(rs_ctx *ctx, const mgreal *b, mgreal *x, bool pre0);
-  template <int CC>
-  void spmv0_t(rs_ctx *ctx, const mgreal *x, mgreal *y);
-  void pcg_body(rs_ctx *ctx, const mgreal *b, mgreal *x, int C_, int iters);
+  template <int C>
+  void launch(rs_ctx *ctx, const mgreal *b, mgreal *x, int iters);
+  DevBuf<mgreal> cg_p, cg_q;  // with level 0's b and x as the residual and its preconditioned form
+  DevBuf<double> cg_part;     // per-chunk partial sums of the dot products
+  DevBuf<unsigned long long> counter;  // arrivals at the grid barrier
+  int *error = nullptr, *error_dev = nullptr;  // mapped host memory: set by a solve that gave up
+  int grid = 1, threads = 256, smem_bytes = 0;
+  // one cluster of blocks where its shared memory holds three columns: the bytes (0: it does not)
+  int cluster_threads = 256, cluster_smem = 0;
+  cudaLaunchConfig_t cluster_config(cudaStream_t s, cudaLaunchAttribute &at) const;
 };
 
 }  // namespace rsg

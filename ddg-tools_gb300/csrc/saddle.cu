@@ -500,6 +500,7 @@ struct rs_solver {
     }
     gmres_batch(ctx, inner_plain ? op_inner : op, use_prec ? &prec : nullptr, nb, b, x, o, last,
                 inner_plain ? &op : nullptr);
+    amg.check();
   }
 };
 
@@ -912,7 +913,7 @@ int rs_solver_multigrid_levels(rs_solver *S, int64_t *out, int max_levels, int *
     int n = (int)S->amg.L.size();
     for (int l = 0; l < n && l < max_levels; ++l) {
       out[2 * l] = S->amg.L[l].n;
-      out[2 * l + 1] = (int64_t)S->amg.L[l].av.n;
+      out[2 * l + 1] = (int64_t)S->amg.L[l].a.nnz;
     }
     *n_levels = n;
   });
@@ -1054,6 +1055,7 @@ int rs_solver_precondition(rs_solver *S, int nb, const double *r, double *z) {
   return guard([&] {
     S->ctx->use();
     host_roundtrip(S, nb, r, z, [&](const double *a, double *b) { S->apply_prec(nb, a, b); });
+    S->amg.check();
   });
 }
 
