@@ -23,6 +23,7 @@
 // / 14.4 -> 6.6 / 8.3 / 8.6 ms; 4,356 rows 20.9 / 23.6 / 27.3 -> 14.2 / 16.8 / 18.0 ms; 25,600 rows 43.4
 // / 50.1 / 56.4 -> 33.4 / 37.4 / 43.5 ms; 102,400 rows 101 / 124 / 154 -> 89 / 105 / 141 ms.
 #include "amg.hpp"
+#include "fp64_bits.cuh"
 
 namespace rsg {
 
@@ -221,14 +222,8 @@ struct NoVals {};
 // 16 to 1), by one warp: past 32 apart the columns share the lanes, as FP64 instructions cost a warp
 // sixteen cycles whatever its idle lanes. Lanes 0, 16, 8 and 24 end with the sums of columns 0 to 3. sh: the columns, 128
 // values each, all zero from `count` on (whose additions are left out).
-template <class T>
-__device__ __forceinline__ double to_f64(T v) { return v; }
-template <>
-__device__ __forceinline__ double to_f64<float>(float v) {  // from the bits (conversions run at the FP64 rate)
-  const unsigned b = __float_as_uint(v), e = (b >> 23) & 0xffu;
-  if (e - 1u >= 254u) return (double)v;
-  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
-}
+__device__ __forceinline__ double to_f64(double v) { return v; }
+__device__ __forceinline__ double to_f64(float v) { return f2d(v); }
 __device__ __forceinline__ double tree32x4(const double (&v)[4], int lane) {
   // 16 apart: lanes 0-15 keep columns 0 and 2, lanes 16-31 columns 1 and 3; 8 apart likewise
   const bool u16 = lane & 16, u8 = lane & 8;

@@ -23,6 +23,7 @@
 
 #include "bh_kernels.cuh"
 #include "common.hpp"
+#include "fp64_bits.cuh"
 #include "host_tree.hpp"
 #include "profile.hpp"
 
@@ -32,14 +33,28 @@ constexpr int kMaxDepth = 96;  // DFS stack bound of the list traversal (checked
 
 // ------------------------------------------------------------------ refit
 
+// x as a float pair: hi = x rounded to FP32, lo = the rest rounded
+__device__ __forceinline__ void split(double x, float &hi, float &lo) {
+  hi = d2f(x);
+  lo = d2f(x - f2d(hi));
+}
+
 // The node centroid in FP64 and as a float pair (hi + lo) for the pair kernel.
 __device__ __forceinline__ void store_centroid(const BhDev &d, uint32_t n, double x, double y,
                                                double z, double A) {
   d.ncA[n] = make_double4(x, y, z, A);
-  float hx = (float)x, hy = (float)y, hz = (float)z;
-  d.nch[n] = make_float4(hx, hy, hz, (float)A);
-  d.ncl[n] = make_float4((float)(x - (double)hx), (float)(y - (double)hy), (float)(z - (double)hz), 0.f);
+  float hx, hy, hz, lx, ly, lz;
+  split(x, hx, lx), split(y, hy, ly), split(z, hz, lz);
+  d.nch[n] = make_float4(hx, hy, hz, d2f(A));
+  d.ncl[n] = make_float4(lx, ly, lz, 0.f);
 }
+
+// a x + b y + c z and a x - b y with their roundings fixed (two products contracted one way or the other
+// differ in the last bit, which the solvers amplify)
+__device__ __forceinline__ double dot3(double a, double x, double b, double y, double c, double z) {
+  return __fma_rn(c, z, __fma_rn(a, x, __dmul_rn(b, y)));
+}
+__device__ __forceinline__ double det2(double a, double x, double b, double y) { return __fma_rn(a, x, -__dmul_rn(b, y)); }
 
 // L2-coherent load of a node record written by another thread of the same launch.
 __device__ __forceinline__ double4 ldcg4(const double4 *p) {
@@ -48,23 +63,51 @@ __device__ __forceinline__ double4 ldcg4(const double4 *p) {
   return make_double4(a.x, a.y, b.x, b.y);
 }
 
-// One thread per leaf: FP64 face geometry of the leaf's faces (face_quantities,
-// RS/src/geometry.rs:33-39), the leaf's area and moment (Bvh::refit order, bvh.rs:226-260),
+// The refit of kRefitLeaves leaves per block: FP64 face geometry of their faces (face_quantities,
+// RS/src/geometry.rs:33-39), the leaves' areas and moments (Bvh::refit order, bvh.rs:226-260),
 // the packed FP32 face records relative to the leaf centroid, then the parents bottom-up: the
 // second child to arrive at a parent computes it (left + right), so every node is written once
 // with the crate's summation order.
-__global__ void refit_kernel(BhDev d, const double *__restrict__ pos) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= d.n_leaves) return;
-  uint32_t leaf = d.leaves[k];
-  uint32_t s0 = d.node_start[leaf], s1 = d.node_end[leaf];
-  double A = 0.0, M0 = 0.0, M1 = 0.0, M2 = 0.0;
-  double xb[8][3], ar[8], nr[8][3];
+//
+// Bound by FP64 instructions (sixteen cycles each for a warp, whatever its live lanes) on large meshes and by
+// the chain of a leaf's faces on small ones, so a thread takes a face (with a thread per leaf a
+// third of the lanes idled and eight faces followed one another), float pairs are split from
+// the bits, and the face records are written beside the climb. At 1,280 / 81,920 / 640,000 faces
+// a thread per leaf took 82 / 116 / 375 us.
+constexpr int kRefitLeaves = 32, kRefitThreads = 128;
+__global__ void __launch_bounds__(kRefitThreads) refit_kernel(BhDev d, const double *__restrict__ pos) {
+  __shared__ double fx[3][8 * kRefitLeaves], fn[3][8 * kRefitLeaves], fa[8 * kRefitLeaves];
+  __shared__ double cen[3][kRefitLeaves];
+  __shared__ uint32_t start[kRefitLeaves], first[kRefitLeaves];
+  __shared__ uint8_t map[8 * kRefitLeaves];  // leaf of every face of the block
+  __shared__ int total;
+  const int tid = threadIdx.x, lane = tid & 31, k = (int)(blockIdx.x * kRefitLeaves) + lane;
+  const bool mine = tid < 32 && k < d.n_leaves;
+  uint32_t leaf = 0;
+  int ns = 0, f0 = 0;
+  if (tid < 32) {
+    if (mine) {
+      leaf = d.leaves[k];
+      const uint32_t s0 = d.node_start[leaf];
+      ns = (int)min(8u, d.node_end[leaf] - s0);
+      start[lane] = s0;
+    }
+    f0 = ns;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    uint32_t p = s0 + i;
-    if (p >= s1) break;
-    uint32_t f = d.order[p];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, f0, o);
+      if (lane >= o) f0 += t;
+    }
+    if (lane == 31) total = f0;
+    f0 -= ns;
+    first[lane] = (uint32_t)f0;
+    for (int i = 0; i < ns; ++i) map[f0 + i] = (uint8_t)lane;
+  }
+  __syncthreads();
+  const int n = total;
+  for (int i = tid; i < n; i += kRefitThreads) {
+    const int l = map[i];
+    const uint32_t f = d.order[start[l] + (i - first[l])];
     const double *p0 = pos + 3 * (size_t)d.faces[3 * f];
     const double *p1 = pos + 3 * (size_t)d.faces[3 * f + 1];
     const double *p2 = pos + 3 * (size_t)d.faces[3 * f + 2];
@@ -75,54 +118,63 @@ __global__ void refit_kernel(BhDev d, const double *__restrict__ pos) {
     double c2 = __dsub_rn(__dmul_rn(u0, w1), __dmul_rn(u1, w0));
     double len = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(c0, c0), __dmul_rn(c1, c1)), __dmul_rn(c2, c2)));
     const double third = 1.0 / 3.0;
-    double x0 = __dmul_rn(__dadd_rn(__dadd_rn(p0[0], p1[0]), p2[0]), third);
-    double x1 = __dmul_rn(__dadd_rn(__dadd_rn(p0[1], p1[1]), p2[1]), third);
-    double x2 = __dmul_rn(__dadd_rn(__dadd_rn(p0[2], p1[2]), p2[2]), third);
-    double a = __dmul_rn(0.5, len);
+    fx[0][i] = __dmul_rn(__dadd_rn(__dadd_rn(p0[0], p1[0]), p2[0]), third);
+    fx[1][i] = __dmul_rn(__dadd_rn(__dadd_rn(p0[1], p1[1]), p2[1]), third);
+    fx[2][i] = __dmul_rn(__dadd_rn(__dadd_rn(p0[2], p1[2]), p2[2]), third);
+    fa[i] = __dmul_rn(0.5, len);
     double il = __drcp_rn(len);
-    nr[i][0] = __dmul_rn(c0, il);
-    nr[i][1] = __dmul_rn(c1, il);
-    nr[i][2] = __dmul_rn(c2, il);
-    xb[i][0] = x0, xb[i][1] = x1, xb[i][2] = x2, ar[i] = a;
-    A = __dadd_rn(A, a);
-    M0 = __dadd_rn(M0, __dmul_rn(a, x0));
-    M1 = __dadd_rn(M1, __dmul_rn(a, x1));
-    M2 = __dadd_rn(M2, __dmul_rn(a, x2));
+    fn[0][i] = __dmul_rn(c0, il), fn[1][i] = __dmul_rn(c1, il), fn[2][i] = __dmul_rn(c2, il);
   }
-  double cx = __ddiv_rn(M0, A), cy = __ddiv_rn(M1, A), cz = __ddiv_rn(M2, A);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    uint32_t p = s0 + i;
-    if (p >= s1) break;
-    double o0 = xb[i][0] - cx, o1 = xb[i][1] - cy, o2 = xb[i][2] - cz;
-    float h0 = (float)o0, h1 = (float)o1, h2 = (float)o2;
-    // alpha = N . (X - X_leaf) as a float pair: hi in fnl.w, lo in fol.w
-    double alpha = nr[i][0] * o0 + nr[i][1] * o1 + nr[i][2] * o2;
-    float al = (float)alpha;
-    d.fxa[p] = make_float4(h0, h1, h2, (float)ar[i]);
-    d.fol[p] = make_float4((float)(o0 - (double)h0), (float)(o1 - (double)h1), (float)(o2 - (double)h2),
-                           (float)(alpha - (double)al));
-    float n0 = (float)nr[i][0], n1 = (float)nr[i][1], n2 = (float)nr[i][2];
-    d.fnn[p] = make_float4(n0, n1, n2, 0.f);
-    d.fnl[p] = make_float4((float)(nr[i][0] - (double)n0), (float)(nr[i][1] - (double)n1),
-                           (float)(nr[i][2] - (double)n2), al);
+  __syncthreads();
+  double4 m = make_double4(0.0, 0.0, 0.0, 0.0);
+  if (mine) {
+    for (int i = f0; i < f0 + ns; ++i) {
+      const double a = fa[i];
+      m.w = __dadd_rn(m.w, a);
+      m.x = __dadd_rn(m.x, __dmul_rn(a, fx[0][i]));
+      m.y = __dadd_rn(m.y, __dmul_rn(a, fx[1][i]));
+      m.z = __dadd_rn(m.z, __dmul_rn(a, fx[2][i]));
+    }
+    const double cx = __ddiv_rn(m.x, m.w), cy = __ddiv_rn(m.y, m.w), cz = __ddiv_rn(m.z, m.w);
+    cen[0][lane] = cx, cen[1][lane] = cy, cen[2][lane] = cz;
+    d.nmom[leaf] = m;
+    store_centroid(d, leaf, cx, cy, cz, m.w);
   }
-  d.nmom[leaf] = make_double4(M0, M1, M2, A);
-  store_centroid(d, leaf, cx, cy, cz, A);
-  uint32_t n = leaf;
-  while (n != 0) {
-    uint32_t par = d.node_parent[n];
+  __syncthreads();
+  if (tid >= 32) {
+    for (int i = tid - 32; i < n; i += kRefitThreads - 32) {
+      const int l = map[i];
+      const uint32_t p = start[l] + (i - first[l]);
+      const double o0 = fx[0][i] - cen[0][l], o1 = fx[1][i] - cen[1][l], o2 = fx[2][i] - cen[2][l];
+      const double n0 = fn[0][i], n1 = fn[1][i], n2 = fn[2][i];
+      // alpha = N . (X - X_leaf) as a float pair: hi in fnl.w, lo in fol.w
+      const double alpha = dot3(n0, o0, n1, o1, n2, o2);
+      float al, all, h0, h1, h2, l0, l1, l2;
+      split(alpha, al, all);
+      split(o0, h0, l0), split(o1, h1, l1), split(o2, h2, l2);
+      d.fxa[p] = make_float4(h0, h1, h2, d2f(fa[i]));
+      d.fol[p] = make_float4(l0, l1, l2, all);
+      split(n0, h0, l0), split(n1, h1, l1), split(n2, h2, l2);
+      d.fnn[p] = make_float4(h0, h1, h2, 0.f);
+      d.fnl[p] = make_float4(l0, l1, l2, al);
+    }
+    return;
+  }
+  if (!mine) return;
+  uint32_t node = leaf;
+  while (node != 0) {
+    uint32_t par = d.node_parent[node];
     __threadfence();
     unsigned old = atomicAdd(&d.refit_count[par], 1u);
     if ((old & 1u) == 0u) return;  // first child here: the sibling completes the parent
     __threadfence();
     double4 l = ldcg4(&d.nmom[par + 1]);
     double4 r = ldcg4(&d.nmom[d.node_right[par]]);
-    double4 m = make_double4(__dadd_rn(l.x, r.x), __dadd_rn(l.y, r.y), __dadd_rn(l.z, r.z),
+    double4 s = make_double4(__dadd_rn(l.x, r.x), __dadd_rn(l.y, r.y), __dadd_rn(l.z, r.z),
                              __dadd_rn(l.w, r.w));
-    d.nmom[par] = m;
-    store_centroid(d, par, __ddiv_rn(m.x, m.w), __ddiv_rn(m.y, m.w), __ddiv_rn(m.z, m.w), m.w);
-    n = par;
+    d.nmom[par] = s;
+    store_centroid(d, par, __ddiv_rn(s.x, s.w), __ddiv_rn(s.y, s.w), __ddiv_rn(s.z, s.w), s.w);
+    node = par;
   }
 }
 
@@ -709,24 +761,39 @@ __global__ void node_sums_kernel(BhDev d) {
 }
 
 // Downward pass per leaf along its root -> leaf chain (barnes_hut.rs:521-538), in FP64 (about
-// 20 steps per leaf): beta_c = beta_p + U_p.(X_c - X_p) + b_c, U_c = U_p + u_c.
+// 20 steps per leaf, each record fetched four steps ahead): beta_c = beta_p + U_p.(X_c - X_p) + b_c, U_c = U_p + u_c.
 __global__ void downward_kernel(BhDev d) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= d.n_leaves) return;
   uint32_t c0 = d.chain_off[k], c1 = d.chain_off[k + 1];
   uint32_t p = d.chain[c0];
   float4 s = d.node_sum[p];
-  double beta = s.x, U0 = s.y, U1 = s.z, U2 = s.w;
+  double beta = f2d(s.x), U0 = f2d(s.y), U1 = f2d(s.z), U2 = f2d(s.w);
   double4 xp = d.ncA[p];
-  for (uint32_t i = c0 + 1; i < c1; ++i) {
-    uint32_t c = d.chain[i];
-    double4 xc = d.ncA[c];
-    float4 sc = d.node_sum[c];
-    beta = beta + (U0 * (xc.x - xp.x) + U1 * (xc.y - xp.y) + U2 * (xc.z - xp.z)) + (double)sc.x;
-    U0 += sc.y, U1 += sc.z, U2 += sc.w;
-    xp = xc;
+  constexpr int R = 4;  // records on the way
+  double4 xs[R];
+  float4 ss[R];
+  auto fetch = [&](uint32_t i, int j) {
+    if (i < c1) {
+      const uint32_t c = d.chain[i];
+      xs[j] = d.ncA[c], ss[j] = d.node_sum[c];
+    }
+  };
+#pragma unroll
+  for (int j = 0; j < R; ++j) fetch(c0 + 1 + j, j);
+  for (uint32_t i = c0 + 1; i < c1; i += R) {
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      if (i + j >= c1) break;
+      const double4 xc = xs[j];
+      const float4 sc = ss[j];
+      fetch(i + j + R, j);
+      beta = beta + dot3(U0, xc.x - xp.x, U1, xc.y - xp.y, U2, xc.z - xp.z) + f2d(sc.x);
+      U0 += f2d(sc.y), U1 += f2d(sc.z), U2 += f2d(sc.w);
+      xp = xc;
+    }
   }
-  d.leaf_bu[k] = make_float4((float)beta, (float)U0, (float)U1, (float)U2);
+  d.leaf_bu[k] = make_float4(d2f(beta), d2f(U0), d2f(U1), d2f(U2));
 }
 
 // Partner sums per chunk of a leaf's transposed exact list (one warp per chunk): lanes stride
@@ -743,8 +810,12 @@ __global__ void final_partial_kernel(BhDev d) {
   float acc[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+  // the places of the entries are found two rounds ahead (a chain of two loads)
+  auto place = [&](uint32_t e) { return e < ch.z ? d.partner_off[d.exact_t[e]] : 0u; };
+  uint32_t o0 = place(ch.y + lane), o1 = place(ch.y + lane + 32);
   for (uint32_t e = ch.y + lane; e < ch.z; e += 32) {
-    const float4 *pp = d.partner + d.partner_off[d.exact_t[e]];
+    const float4 *pp = d.partner + o0;
+    o0 = o1, o1 = place(e + 64);
 #pragma unroll
     for (int t = 0; t < 8; ++t)
       if ((uint32_t)t < ns) {
@@ -771,86 +842,126 @@ __global__ void final_partial_kernel(BhDev d) {
   d.fpart[32 * (size_t)w + lane] = (b0 ? r2[1] : r2[0]) + __shfl_xor_sync(0xffffffffu, b0 ? r2[0] : r2[1], 1);
 }
 
-// Per leaf (one warp, lane 4 t + c = component c of face t): own + partner (the leaf's chunks in
-// order) + cluster part (barnes_hut.rs:539-567), written by face id.
-__global__ void final_kernel(BhDev d) {
-  const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (k >= d.n_leaves) return;
-  const uint32_t leaf = d.leaves[k];
-  const uint32_t s0 = d.node_start[leaf];
-  const uint32_t ns = d.node_end[leaf] - s0;
-  const uint32_t t = lane >> 2, c = lane & 3;
-  if (t >= ns) return;
-  float part = 0.f;
-  for (uint32_t ch = d.fchunk_off[k]; ch < d.fchunk_off[k + 1]; ++ch) part += d.fpart[32 * (size_t)ch + lane];
-  const uint32_t p = s0 + t;
-  const float *ow = reinterpret_cast<const float *>(d.own);
-  float own = 0.f, ownn = 0.f;
-  for (uint32_t i = d.item_off[k]; i < d.item_off[k + 1]; ++i) {  // 64 floats per item
-    own += ow[64 * (size_t)i + 8 * t + c];
-    ownn += ow[64 * (size_t)i + 8 * t + 4 + c];
+// Per face: own + partner (the leaf's chunks in order) + cluster part (barnes_hut.rs:539-567), written
+// by face id; then the face's part of the differential at its three corners (face_pull_back,
+// RS/src/geometry.rs:87-110), in FP64: the face terms around a vertex cancel to a small
+// differential, so this O(F) step keeps FP64. The corners share the normal and the reciprocal
+// length (a pass per vertex formed them for every incident corner: 32 / 58 us at 1,280 / 81,920
+// faces, of which FP64 instructions 42 at the latter).
+template <bool CORNERS>
+__global__ void __launch_bounds__(128) final_kernel(BhDev d, const double *__restrict__ pos, double *__restrict__ corner) {
+  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= (uint32_t)d.n_faces) return;
+  const uint32_t k = d.leaf_of_pos[p], t = p - d.node_start[d.leaves[k]], f = d.order[p];
+  const float4 *fp = reinterpret_cast<const float4 *>(d.fpart);
+  float4 part = make_float4(0.f, 0.f, 0.f, 0.f), own = part, ownn = part;
+  for (uint32_t ch = d.fchunk_off[k]; ch < d.fchunk_off[k + 1]; ++ch) {
+    const float4 v = fp[8 * (size_t)ch + t];
+    part.x += v.x, part.y += v.y, part.z += v.z, part.w += v.w;
+  }
+  for (uint32_t i = d.item_off[k]; i < d.item_off[k + 1]; ++i) {
+    const float4 v = d.own[16 * (size_t)i + 2 * t], w = d.own[16 * (size_t)i + 2 * t + 1];
+    own.x += v.x, own.y += v.y, own.z += v.z, own.w += v.w;
+    ownn.x += w.x, ownn.y += w.y, ownn.z += w.z, ownn.w += w.w;
   }
   const float4 bu = d.leaf_bu[k];
   const float4 xa = d.fxa[p];  // offset X_T - X_leaf and a_T
-  float cl;
-  if (c == 0) cl = bu.x + (bu.y * xa.x + bu.z * xa.y + bu.w * xa.z);
-  else cl = xa.w * (c == 1 ? bu.y : (c == 2 ? bu.z : bu.w));
-  const uint32_t f = d.order[p];
-  float *out = reinterpret_cast<float *>(d.partials);
-  out[8 * (size_t)f + c] = (own + part) + cl;
-  out[8 * (size_t)f + 4 + c] = ownn;
+  const float cl = __fadd_rn(bu.x, __fmaf_rn(bu.w, xa.z, __fmaf_rn(bu.z, xa.y, __fmul_rn(bu.y, xa.x))));
+  float q[7];
+  q[0] = __fadd_rn(own.x + part.x, cl);
+  q[1] = __fadd_rn(own.y + part.y, __fmul_rn(xa.w, bu.y));
+  q[2] = __fadd_rn(own.z + part.z, __fmul_rn(xa.w, bu.z));
+  q[3] = __fadd_rn(own.w + part.w, __fmul_rn(xa.w, bu.w));
+  q[4] = ownn.x, q[5] = ownn.y, q[6] = ownn.z;
+  d.partials[2 * (size_t)f] = make_float4(q[0], q[1], q[2], q[3]);
+  d.partials[2 * (size_t)f + 1] = make_float4(q[4], q[5], q[6], ownn.w);
+  if constexpr (CORNERS) {
+    const uint32_t *t3 = d.faces + 3 * (size_t)f;
+    double P[3][3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int a = 0; a < 3; ++a) P[c][a] = pos[3 * (size_t)t3[c] + a];
+    double u0 = P[1][0] - P[0][0], u1 = P[1][1] - P[0][1], u2 = P[1][2] - P[0][2];
+    double w0 = P[2][0] - P[0][0], w1 = P[2][1] - P[0][1], w2 = P[2][2] - P[0][2];
+    double n0 = det2(u1, w2, u2, w1), n1 = det2(u2, w0, u0, w2), n2 = det2(u0, w1, u1, w0);
+    double len = sqrt(dot3(n0, n0, n1, n1, n2, n2));
+    double il = 1.0 / len;
+    n0 *= il, n1 *= il, n2 *= il;
+    const double third = 1.0 / 3.0;
+    const double q4 = f2d(q[4]), q5 = f2d(q[5]), q6 = f2d(q[6]);
+    double ha = 0.5 * f2d(q[0]);
+    double q1 = f2d(q[1]), q2 = f2d(q[2]), q3 = f2d(q[3]);
+    double *out = corner + 9 * (size_t)f;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      // edge opposite corner c: e_jk = p2 - p1, e_ki = p0 - p2, e_ij = p1 - p0
+      const double(&pa)[3] = P[(c + 1) % 3], (&pb)[3] = P[(c + 2) % 3];
+      double e0 = pb[0] - pa[0], e1 = pb[1] - pa[1], e2 = pb[2] - pa[2];
+      double c0 = det2(n1, e2, n2, e1), c1 = det2(n2, e0, n0, e2), c2 = det2(n0, e1, n1, e0);  // N x e
+      double dotn = -dot3(c0, q4, c1, q5, c2, q6) * il;
+      out[3 * c] = dot3(ha, c0, q1, third, n0, dotn);
+      out[3 * c + 1] = dot3(ha, c1, q2, third, n1, dotn);
+      out[3 * c + 2] = dot3(ha, c2, q3, third, n2, dotn);
+    }
+  }
 }
 
-// Pull-back to the vertices (face_pull_back, RS/src/geometry.rs:87-110, summed over the
-// incident faces in increasing face order, geometry.rs:172-188), in FP64: the face terms
-// around a vertex cancel to a small differential, so this O(F) step keeps FP64.
-__global__ void pull_back_kernel(BhDev d, const double *__restrict__ pos, double *__restrict__ dE) {
+// The differential: the corners' parts summed over the faces around a vertex in increasing face
+// order (geometry.rs:172-188).
+__global__ void pull_back_kernel(BhDev d, const double *__restrict__ corner, double *__restrict__ dE) {
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= d.n_vertices) return;
   double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-  const float *pa_ = reinterpret_cast<const float *>(d.partials);
-  for (uint32_t e = d.inc_off[v]; e < d.inc_off[v + 1]; ++e) {
-    uint32_t fc = d.inc[e];
-    uint32_t f = fc >> 2, c = fc & 3;
-    const uint32_t *t = d.faces + 3 * (size_t)f;
-    const double *p0 = pos + 3 * (size_t)t[0];
-    const double *p1 = pos + 3 * (size_t)t[1];
-    const double *p2 = pos + 3 * (size_t)t[2];
-    double u0 = p1[0] - p0[0], u1 = p1[1] - p0[1], u2 = p1[2] - p0[2];
-    double w0 = p2[0] - p0[0], w1 = p2[1] - p0[1], w2 = p2[2] - p0[2];
-    double n0 = u1 * w2 - u2 * w1, n1 = u2 * w0 - u0 * w2, n2 = u0 * w1 - u1 * w0;
-    double len = sqrt(n0 * n0 + n1 * n1 + n2 * n2);
-    double il = 1.0 / len;
-    n0 *= il, n1 *= il, n2 *= il;
-    // edge opposite corner c: e_jk = p2 - p1, e_ki = p0 - p2, e_ij = p1 - p0
-    const double *pa = c == 0 ? p1 : (c == 1 ? p2 : p0);
-    const double *pb = c == 0 ? p2 : (c == 1 ? p0 : p1);
-    double e0 = pb[0] - pa[0], e1 = pb[1] - pa[1], e2 = pb[2] - pa[2];
-    const float *q = pa_ + 8 * (size_t)f;
-    double ha = 0.5 * (double)q[0];
-    double c0 = n1 * e2 - n2 * e1, c1 = n2 * e0 - n0 * e2, c2 = n0 * e1 - n1 * e0;  // N x e
-    double dotn = -(c0 * (double)q[4] + c1 * (double)q[5] + c2 * (double)q[6]) * il;
-    const double third = 1.0 / 3.0;
-    g0 += ha * c0 + (double)q[1] * third + n0 * dotn;
-    g1 += ha * c1 + (double)q[2] * third + n1 * dotn;
-    g2 += ha * c2 + (double)q[3] * third + n2 * dotn;
+  const uint32_t e1 = d.inc_off[v + 1];
+#pragma unroll 4
+  for (uint32_t e = d.inc_off[v]; e < e1; ++e) {
+    const uint32_t fc = d.inc[e];
+    const double *q = corner + 9 * (size_t)(fc >> 2) + 3 * (fc & 3);
+    g0 += q[0], g1 += q[1], g2 += q[2];
   }
-  dE[3 * v] = g0, dE[3 * v + 1] = g1, dE[3 * v + 2] = g2;
+  dE[3 * (size_t)v] = g0, dE[3 * (size_t)v + 1] = g1, dE[3 * (size_t)v + 2] = g2;
 }
 
-// Energy over the leaves in FP64: fixed strided partial sums, then a fixed tree.
-__global__ void energy_reduce_kernel(const double *leaf_energy, int n, double *out) {
-  __shared__ double sh[1024];
+// Energy over the work items in FP64: 1024 strided partial sums over a cluster of eight blocks, then a
+// fixed tree in the first (one block of 1024 threads is bound by its SM's FP64 rate: 21 us at 81,920 faces,
+// 172 at 640,000).
+constexpr int kEnergyBlocks = 8, kEnergyThreads = 1024 / kEnergyBlocks;
+__global__ void __cluster_dims__(kEnergyBlocks) __launch_bounds__(kEnergyThreads)
+    energy_reduce_kernel(const double *leaf_energy, int n, double *out) {
+  __shared__ double part[kEnergyThreads], sh[1024];
   double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) acc += leaf_energy[i];
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int m = blockDim.x / 2; m > 0; m >>= 1) {
-    if ((int)threadIdx.x < m) sh[threadIdx.x] += sh[threadIdx.x + m];
-    __syncthreads();
+  int i = (int)(blockIdx.x * kEnergyThreads + threadIdx.x);
+  for (; i + 7 * 1024 < n; i += 8 * 1024) {
+    double v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = leaf_energy[i + 1024 * j];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc += v[j];
   }
-  if (threadIdx.x == 0) *out = sh[0];
+  for (; i < n; i += 1024) acc += leaf_energy[i];
+  part[threadIdx.x] = acc;
+  auto barrier = [] {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  };
+  barrier();
+  if (blockIdx.x == 0) {
+    const unsigned own = (unsigned)__cvta_generic_to_shared(part + threadIdx.x);
+#pragma unroll
+    for (int b = 0; b < kEnergyBlocks; ++b) {
+      unsigned at;
+      double v;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(own), "r"(b));
+      asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(at) : "memory");
+      sh[b * kEnergyThreads + threadIdx.x] = v;
+    }
+    for (int m = 512; m > 0; m >>= 1) {
+      __syncthreads();
+      for (int t = threadIdx.x; t < m; t += kEnergyThreads) sh[t] += sh[t + m];
+    }
+    if (threadIdx.x == 0) *out = sh[0];
+  }
+  barrier();  // no block leaves while the first may read its shared memory
 }
 
 // First exact pair in leaf, list, s, t order whose FP32 term is non-finite (culprit_pair,
@@ -921,7 +1032,7 @@ struct rs_bh {
   DevBuf<double4> ncA, nmom;
   DevBuf<float4> nch, ncl;
   DevBuf<uint32_t> refit_count;
-  DevBuf<double> item_energy, energy, dE;
+  DevBuf<double> item_energy, energy, dE, corner;
   DevBuf<unsigned int> ticket;
   DevBuf<unsigned long long> culprit_key;
   bool positions_current = false;
@@ -1048,6 +1159,7 @@ void upload_topology(rs_bh *h) {
   h->fol.alloc(h->nf);
   h->fnl.alloc(h->nf);
   h->partials.alloc(2 * (size_t)h->nf);
+  h->corner.alloc(9 * (size_t)h->nf);
   h->ncA.alloc(nn);
   h->nmom.alloc(nn);
   h->nch.alloc(nn);
@@ -1267,7 +1379,7 @@ void build_lists_device(rs_bh *h) {
 void refit_device(rs_bh *h) {
   BhDev d = h->dev();
   size_t nl = h->tree.leaves.size();
-  refit_kernel<<<blocks(nl, 128), 128, 0, h->st()>>>(d, h->pos.p);
+  refit_kernel<<<blocks(nl, kRefitLeaves), kRefitThreads, 0, h->st()>>>(d, h->pos.p);
   RSG_LAUNCHED(h->ctx, "refit");
   h->positions_current = true;
 }
@@ -1329,18 +1441,19 @@ void evaluate(rs_bh *h, const Pow &pw, bool fast, bool grad, double *energy_dev,
     P.begin(s, "final");
     final_partial_kernel<<<blocks((size_t)h->n_fchunks * 32, 256), 256, 0, s>>>(d);
     RSG_LAUNCHED(h->ctx, "final");
-    final_kernel<<<blocks(nl * 32, 256), 256, 0, s>>>(d);
+    if (dE_dev) final_kernel<true><<<blocks(h->nf, 128), 128, 0, s>>>(d, h->pos.p, h->corner.p);
+    else final_kernel<false><<<blocks(h->nf, 128), 128, 0, s>>>(d, h->pos.p, nullptr);
     RSG_LAUNCHED(h->ctx, "final");
     P.end(s);
     if (dE_dev) {
       P.begin(s, "pull_back");
-      pull_back_kernel<<<blocks(h->nv, 256), 256, 0, s>>>(d, h->pos.p, dE_dev);
+      pull_back_kernel<<<blocks(h->nv, 128), 128, 0, s>>>(d, h->corner.p, dE_dev);
       RSG_LAUNCHED(h->ctx, "pull_back");
       P.end(s);
     }
   }
   P.begin(s, "energy_reduce");
-  energy_reduce_kernel<<<1, 1024, 0, s>>>(h->item_energy.p, (int)h->n_items, energy_dev);
+  energy_reduce_kernel<<<kEnergyBlocks, kEnergyThreads, 0, s>>>(h->item_energy.p, (int)h->n_items, energy_dev);
   RSG_LAUNCHED(h->ctx, "energy_reduce");
   P.end(s);
 }

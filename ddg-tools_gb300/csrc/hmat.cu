@@ -35,6 +35,7 @@
 
 #include "block_tree.hpp"
 #include "common.hpp"
+#include "fp64_bits.cuh"
 #include "host_tree.hpp"
 #include "hmat.hpp"
 #include "profile.hpp"
@@ -127,20 +128,6 @@ __device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
   return r;
 }
 constexpr f32x2 kF2Sign = 0x8000000080000000ull;  // both halves' sign bits
-
-// Conversions between FP32 and FP64 from the bits. GB300 converts at its FP64 rate, two lanes per
-// clock and SM, which bounded every pass around the near field; integer instructions run at 64.
-__device__ __forceinline__ double f2d(float x) {  // (double)x
-  const unsigned b = __float_as_uint(x), e = (b >> 23) & 0xffu;
-  if (e - 1u >= 254u) return (double)x;  // zero, subnormal, infinity, NaN
-  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
-}
-__device__ __forceinline__ double rn24(double x) {  // (double)(float)x
-  const unsigned hi = (unsigned)__double2hiint(x), e = (hi >> 20) & 0x7ffu;
-  if (e - 897u >= 253u) return (double)(float)x;  // not a normal float
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  return __longlong_as_double((long long)((b + 0x0fffffffull + ((b >> 29) & 1ull)) & ~0x1fffffffull));
-}
 
 // v as a float pair: hi = v rounded to FP32, lo = the rest rounded
 __device__ __forceinline__ float2 to_pair(double v) {
