@@ -72,22 +72,33 @@ __device__ __forceinline__ double4 ldcg4(const double4 *p) {
 // Bound by FP64 instructions (sixteen cycles each for a warp, whatever its live lanes) on large meshes and by
 // the chain of a leaf's faces on small ones, so a thread takes a face (with a thread per leaf a
 // third of the lanes idled and eight faces followed one another), float pairs are split from
-// the bits, and the face records are written beside the climb. At 1,280 / 81,920 / 640,000 faces
-// a thread per leaf took 82 / 116 / 375 us.
+// the bits, and the face records are written beside the climb. The climb starts in shared
+// memory: the nodes over a block's leaves alone are summed there and divided afterwards a
+// lane per node; only the nodes above them take a fence and an atomic per level in global memory. At 1,280 /
+// 81,920 / 640,000 faces a thread per leaf and a climb through global memory took 82 / 116 /
+// 375 us, a thread per face 62 / 103 / 292.
 constexpr int kRefitLeaves = 32, kRefitThreads = 128;
+constexpr uint32_t kNoSlot = ~0u;
 __global__ void __launch_bounds__(kRefitThreads) refit_kernel(BhDev d, const double *__restrict__ pos) {
   __shared__ double fx[3][8 * kRefitLeaves], fn[3][8 * kRefitLeaves], fa[8 * kRefitLeaves];
   __shared__ double cen[3][kRefitLeaves];
   __shared__ uint32_t start[kRefitLeaves], first[kRefitLeaves];
   __shared__ uint8_t map[8 * kRefitLeaves];  // leaf of every face of the block
   __shared__ int total;
+  // per node over leaves of the block alone (its slot: the ordinal of its right child's first leaf): the
+  // moments of its children, how many are there, and where it climbs to
+  __shared__ double kid[2][4][kRefitLeaves];
+  __shared__ uint32_t arrived[kRefitLeaves], id[kRefitLeaves], up[kRefitLeaves];
   const int tid = threadIdx.x, lane = tid & 31, k = (int)(blockIdx.x * kRefitLeaves) + lane;
   const bool mine = tid < 32 && k < d.n_leaves;
   uint32_t leaf = 0;
+  uint4 climb = make_uint4(kNoSlot, kNoSlot, kNoSlot, 0u);
   int ns = 0, f0 = 0;
   if (tid < 32) {
+    arrived[lane] = 0u;
     if (mine) {
       leaf = d.leaves[k];
+      climb = d.climb[k];
       const uint32_t s0 = d.node_start[leaf];
       ns = (int)min(8u, d.node_end[leaf] - s0);
       start[lane] = s0;
@@ -101,6 +112,7 @@ __global__ void __launch_bounds__(kRefitThreads) refit_kernel(BhDev d, const dou
     if (lane == 31) total = f0;
     f0 -= ns;
     first[lane] = (uint32_t)f0;
+    id[lane] = climb.y, up[lane] = climb.z;
     for (int i = 0; i < ns; ++i) map[f0 + i] = (uint8_t)lane;
   }
   __syncthreads();
@@ -137,7 +149,6 @@ __global__ void __launch_bounds__(kRefitThreads) refit_kernel(BhDev d, const dou
     }
     const double cx = __ddiv_rn(m.x, m.w), cy = __ddiv_rn(m.y, m.w), cz = __ddiv_rn(m.z, m.w);
     cen[0][lane] = cx, cen[1][lane] = cy, cen[2][lane] = cz;
-    d.nmom[leaf] = m;
     store_centroid(d, leaf, cx, cy, cz, m.w);
   }
   __syncthreads();
@@ -160,22 +171,45 @@ __global__ void __launch_bounds__(kRefitThreads) refit_kernel(BhDev d, const dou
     }
     return;
   }
-  if (!mine) return;
-  uint32_t node = leaf;
+  // in the block: the second child to arrive goes on with the sum
+  uint32_t node = leaf, to = climb.x;  // to: slot of the parent, times two, plus one for a right child
+  bool live = mine;
+  while (live && to != kNoSlot) {
+    const uint32_t slot = to >> 1, side = to & 1u;
+    kid[side][0][slot] = m.x, kid[side][1][slot] = m.y, kid[side][2][slot] = m.z, kid[side][3][slot] = m.w;
+    __threadfence_block();
+    if (atomicAdd(&arrived[slot], 1u) == 0u) {
+      live = false;
+    } else {
+      __threadfence_block();
+      m.x = __dadd_rn(m.x, kid[side ^ 1u][0][slot]), m.y = __dadd_rn(m.y, kid[side ^ 1u][1][slot]);
+      m.z = __dadd_rn(m.z, kid[side ^ 1u][2][slot]), m.w = __dadd_rn(m.w, kid[side ^ 1u][3][slot]);
+      node = id[slot], to = up[slot];
+    }
+  }
+  __syncwarp();
+  // the centroids of those nodes
+  if (climb.y != kNoSlot && arrived[lane] == 2u) {
+    const double x = __dadd_rn(kid[0][0][lane], kid[1][0][lane]), y = __dadd_rn(kid[0][1][lane], kid[1][1][lane]);
+    const double z = __dadd_rn(kid[0][2][lane], kid[1][2][lane]), A = __dadd_rn(kid[0][3][lane], kid[1][3][lane]);
+    store_centroid(d, climb.y, __ddiv_rn(x, A), __ddiv_rn(y, A), __ddiv_rn(z, A), A);
+  }
+  if (!live) return;
+  // above
+  bool done = true;  // its centroid is stored
   while (node != 0) {
-    uint32_t par = d.node_parent[node];
+    const uint32_t par = d.node_parent[node], right = d.node_right[par];
+    d.nmom[node] = m;
     __threadfence();
-    unsigned old = atomicAdd(&d.refit_count[par], 1u);
+    const unsigned old = atomicAdd(&d.refit_count[par], 1u);
+    if (!done) store_centroid(d, node, __ddiv_rn(m.x, m.w), __ddiv_rn(m.y, m.w), __ddiv_rn(m.z, m.w), m.w);
     if ((old & 1u) == 0u) return;  // first child here: the sibling completes the parent
     __threadfence();
-    double4 l = ldcg4(&d.nmom[par + 1]);
-    double4 r = ldcg4(&d.nmom[d.node_right[par]]);
-    double4 s = make_double4(__dadd_rn(l.x, r.x), __dadd_rn(l.y, r.y), __dadd_rn(l.z, r.z),
-                             __dadd_rn(l.w, r.w));
-    d.nmom[par] = s;
-    store_centroid(d, par, __ddiv_rn(s.x, s.w), __ddiv_rn(s.y, s.w), __ddiv_rn(s.z, s.w), s.w);
-    node = par;
+    const double4 o = ldcg4(&d.nmom[node == right ? par + 1 : right]);
+    m = make_double4(__dadd_rn(m.x, o.x), __dadd_rn(m.y, o.y), __dadd_rn(m.z, o.z), __dadd_rn(m.w, o.w));
+    node = par, done = false;
   }
+  if (!done) store_centroid(d, 0, __ddiv_rn(m.x, m.w), __ddiv_rn(m.y, m.w), __ddiv_rn(m.z, m.w), m.w);
 }
 
 // ------------------------------------------------------------------ interaction lists
@@ -510,15 +544,31 @@ struct PairStage {
 // nu = alpha_S - N_S.y_T with y_T = X_T - X_L held as a float pair and a compensated dot
 // product, and v = X_S - X_T is summed with its rounding error (leaf offsets can be large next
 // to |v| in a stretched leaf). alpha_S = N_S.(X_S - X_L) is a float pair from the FP64 refit.
-template <bool GRAD, bool FAST>
-__global__ void __launch_bounds__(128, 6) bh_pair_kernel(BhDev d, Pow pw) {
+//
+// COOP: a block's four warps share a work item, a batch each in turn (every warp finds the
+// batches by itself); the batches' sums go through shared memory and are added in batch order, two of
+// the eight accumulators per warp, so the result is the same bits. For meshes of few items,
+// whose time is that of one item: 1,280 faces 55 us with a warp per item.
+template <bool GRAD, bool FAST, bool COOP>
+__global__ void __launch_bounds__(128, COOP ? 4 : 6) bh_pair_kernel(BhDev d, Pow pw) {
   __shared__ PairStage stage[4];
+  __shared__ float sums[COOP ? 2 : 1][COOP ? 4 : 1][COOP ? 8 : 1][32];
+  __shared__ unsigned int next;
   PairStage &st = stage[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, W = COOP ? (int)(threadIdx.x >> 5) : 0;
+  constexpr int NW = COOP ? 4 : 1;  // batches at a time
+  int turn = 0;
   for (;;) {
     unsigned int w = 0;
-    if (lane == 0) w = atomicAdd(d.ticket, 1u);
-    w = __shfl_sync(0xffffffffu, w, 0);
+    if (COOP) {
+      __syncthreads();
+      if (threadIdx.x == 0) next = atomicAdd(d.ticket, 1u);
+      __syncthreads();
+      w = next;
+    } else {
+      if (lane == 0) w = atomicAdd(d.ticket, 1u);
+      w = __shfl_sync(0xffffffffu, w, 0);
+    }
     if (w >= (unsigned)d.n_items) return;
     const uint32_t item = d.schedule[w];
     const uint4 it = d.items[item];  // lumped [x, y), exact [z, w) entry ranges
@@ -535,12 +585,38 @@ __global__ void __launch_bounds__(128, 6) bh_pair_kernel(BhDev d, Pow pw) {
     const float4 xsl = act ? d.fol[s0 + s] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 cLh = d.nch[leaf], cLl = d.ncl[leaf];
     const float a_s = xs.w;
-    Kahan e_acc, da_acc, dx0, dx1, dx2, dn0, dn1, dn2;
+    // energy, d_a, d_x, d_n (COOP: the warp's two of them)
+    Kahan acc[COOP ? 2 : 8];
+    // adds the sums v of a batch, of which all but d_a's are still to be multiplied by f when SCALE;
+    // COOP: of `count` batches in order
+    auto push = [&](auto scale, const float (&v)[8], float f, int count) {
+      constexpr bool SCALE = decltype(scale)::value;
+      if constexpr (COOP) {
+#pragma unroll
+        for (int i = 0; i < (GRAD ? 8 : 1); ++i) sums[turn][W][i][lane] = v[i];
+        __syncthreads();
+        if (GRAD || W == 0) {
+          for (int b = 0; b < count; ++b) {
+            const float x = sums[turn][b][2 * W][lane];
+            SCALE ? acc[0].add(f, x) : acc[0].add(x);
+            if (GRAD) {
+              const float y = sums[turn][b][2 * W + 1][lane];
+              SCALE && W != 0 ? acc[1].add(f, y) : acc[1].add(y);
+            }
+          }
+        }
+        turn ^= 1;
+      } else {
+#pragma unroll
+        for (int i = 0; i < (GRAD ? 8 : 1); ++i) SCALE && i != 1 ? acc[i].add(f, v[i]) : acc[i].add(v[i]);
+      }
+    };
 
     // ---- lumped nodes
     const uint32_t llo = it.x, lhi = it.y;
-    for (uint32_t base = llo; base < lhi; base += B) {
-      const int cnt = (int)min((uint32_t)B, lhi - base);
+    for (uint32_t r0 = llo; r0 < lhi; r0 += NW * B) {
+      const uint32_t base = r0 + W * B;
+      const int cnt = base < lhi ? (int)min((uint32_t)B, lhi - base) : 0;
       __syncwarp();
       for (int e = lane; e < cnt; e += 32) {
         const uint32_t c = d.lumped[base + e];
@@ -576,11 +652,9 @@ __global__ void __launch_bounds__(128, 6) bh_pair_kernel(BhDev d, Pow pw) {
           st.red[s * RS + e] = make_float4(a_s * K, -a_s * dv0, -a_s * dv1, -a_s * dv2);
         }
       }
-      e_acc.add(be);
+      const float bs[8] = {be, bda, bx0, bx1, bx2, bn0, bn1, bn2};
+      push(std::false_type{}, bs, a_s, min(NW, (int)((lhi - r0 + B - 1) / B)));
       if (GRAD) {
-        da_acc.add(bda);
-        dx0.add(bx0), dx1.add(bx1), dx2.add(bx2);
-        dn0.add(bn0), dn1.add(bn1), dn2.add(bn2);
         __syncwarp();
         for (int e = lane; e < cnt; e += 32) {
           float4 t = st.red[e];
@@ -622,8 +696,8 @@ __global__ void __launch_bounds__(128, 6) bh_pair_kernel(BhDev d, Pow pw) {
         st.ent_first[lane] = incl - nc;
         for (uint32_t t = 0; t < nc; ++t) st.fmap[incl - nc + t] = (uint8_t)lane;
       }
-      for (int fb = 0; fb < FT; fb += B) {
-        const int cnt = min(B, FT - fb);
+      for (int fr = 0; fr < FT; fr += NW * B) {
+        const int fb = fr + W * B, cnt = max(0, min(B, FT - fb));
         __syncwarp();
         for (int f = lane; f < cnt; f += 32) {
           const int i = st.fmap[fb + f];
@@ -677,11 +751,9 @@ __global__ void __launch_bounds__(128, 6) bh_pair_kernel(BhDev d, Pow pw) {
             st.red[s * RS + f] = make_float4(a_s * K, aa * dv0, aa * dv1, aa * dv2);
           }
         }
-        e_acc.add(a_s * row);
+        const float rs[8] = {row, row, rx0, rx1, rx2, rn0, rn1, rn2};
+        push(std::true_type{}, rs, a_s, min(NW, (FT - fr + B - 1) / B));
         if (GRAD) {
-          da_acc.add(row);
-          dx0.add(a_s * rx0), dx1.add(a_s * rx1), dx2.add(a_s * rx2);
-          dn0.add(a_s * rn0), dn1.add(a_s * rn1), dn2.add(a_s * rn2);
           __syncwarp();
           for (int f = lane; f < cnt; f += 32) {
             float4 t = st.red[f];
@@ -698,12 +770,20 @@ __global__ void __launch_bounds__(128, 6) bh_pair_kernel(BhDev d, Pow pw) {
     // ---- own partials summed over the groups in order; lanes 0..7 write the item's slots
     if (GRAD) {
       __syncwarp();
-      if (act) {
-        st.red[2 * (g * 8 + s)] = make_float4(da_acc.value(), dx0.value(), dx1.value(), dx2.value());
-        st.red[2 * (g * 8 + s) + 1] = make_float4(dn0.value(), dn1.value(), dn2.value(), 0.f);
+      if constexpr (COOP) {
+        __syncthreads();  // the last batches' red is done with
+        if (act) {  // into the first warp's red: (d_a, d_x), (d_n, -) of a lane, warp W the floats 2 W - 1 and 2 W
+          float *o = reinterpret_cast<float *>(stage[0].red + 2 * (g * 8 + s));
+          if (W != 0) o[2 * W - 1] = acc[0].value();
+          o[2 * W] = acc[1].value();
+        }
+        __syncthreads();
+      } else if (act) {
+        st.red[2 * (g * 8 + s)] = make_float4(acc[1].value(), acc[2].value(), acc[3].value(), acc[4].value());
+        st.red[2 * (g * 8 + s) + 1] = make_float4(acc[5].value(), acc[6].value(), acc[7].value(), 0.f);
       }
       __syncwarp();
-      if (lane < 8) {
+      if (W == 0 && lane < 8) {
         float4 o0 = make_float4(0.f, 0.f, 0.f, 0.f), o1 = o0;
         if (lane < ns) {
           o0 = st.red[2 * lane], o1 = st.red[2 * lane + 1];
@@ -717,10 +797,12 @@ __global__ void __launch_bounds__(128, 6) bh_pair_kernel(BhDev d, Pow pw) {
         d.own[16 * (size_t)item + 2 * lane + 1] = o1;
       }
     }
-    double e = (double)e_acc.s - (double)e_acc.c;
+    if (W == 0) {
+      double e = (double)acc[0].s - (double)acc[0].c;
 #pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) e += __shfl_xor_sync(0xffffffffu, e, m);
-    if (lane == 0) d.item_energy[item] = e;
+      for (int m = 16; m >= 1; m >>= 1) e += __shfl_xor_sync(0xffffffffu, e, m);
+      if (lane == 0) d.item_energy[item] = e;
+    }
   }
 }
 
@@ -1030,6 +1112,7 @@ struct rs_bh {
   DevBuf<double> pos;
   DevBuf<float4> fxa, fnn, fol, fnl, own, node_term, partner, node_sum, leaf_bu, partials;
   DevBuf<double4> ncA, nmom;
+  DevBuf<uint4> climb;
   DevBuf<float4> nch, ncl;
   DevBuf<uint32_t> refit_count;
   DevBuf<double> item_energy, energy, dE, corner;
@@ -1055,6 +1138,7 @@ struct rs_bh {
     d.n_vertices = nv, d.n_faces = nf, d.n_nodes = (int)tree.n_nodes();
     d.n_leaves = (int)tree.leaves.size();
     d.fxa = fxa.p, d.fnn = fnn.p, d.ncA = ncA.p, d.nmom = nmom.p, d.refit_count = refit_count.p;
+    d.climb = climb.p;
     d.nch = nch.p, d.ncl = ncl.p;
     d.own = own.p, d.node_term = node_term.p, d.partner = partner.p, d.node_sum = node_sum.p;
     d.leaf_bu = leaf_bu.p, d.partials = partials.p, d.item_energy = item_energy.p;
@@ -1131,6 +1215,32 @@ void upload_topology(rs_bh *h) {
     if (T.end[l] - T.start[l] > 8)
       fail(RS_INVALID_OPTION, "InvalidOption", "upload", "a leaf holds more than 8 faces");
   }
+  // The refit's climb within blocks of kRefitLeaves leaves, per leaf: where it climbs to, the node whose
+  // right child's leaves begin at it when that node's leaves are those of one block, and where that one
+  // climbs to (2 slot + side of the parent, or none).
+  std::vector<uint32_t> lo(nn), hi(nn);
+  std::vector<uint8_t> inside(nn, 0);
+  std::vector<uint4> climb(nl, make_uint4(kNoSlot, kNoSlot, kNoSlot, 0u));
+  for (size_t i = nn; i-- > 0;) {
+    const uint32_t l = (uint32_t)i + 1, r = T.right[i];
+    if (r == 0) {
+      lo[i] = hi[i] = T.leaf_ordinal[i];
+      inside[i] = 1;
+      continue;
+    }
+    lo[i] = std::min(lo[l], lo[r]), hi[i] = std::max(hi[l], hi[r]);
+    inside[i] = l != r && parent[l] == i && parent[r] == i && inside[l] && inside[r] && hi[l] + 1 == lo[r] &&
+                lo[i] / kRefitLeaves == hi[i] / kRefitLeaves;
+    if (inside[i]) climb[lo[r]].y = (uint32_t)i;
+  }
+  auto target = [&](uint32_t i) {
+    const uint32_t p = parent[i];
+    return i != 0 && inside[p] ? 2 * (lo[T.right[p]] % kRefitLeaves) + (i == T.right[p] ? 1u : 0u) : kNoSlot;
+  };
+  for (size_t k = 0; k < nl; ++k) {
+    climb[k].x = target(T.leaves[k]);
+    if (climb[k].y != kNoSlot) climb[k].z = target(climb[k].y);
+  }
   // vertex -> (face, corner), faces ascending
   std::vector<uint32_t> ioff((size_t)h->nv + 1, 0), inc(3 * (size_t)h->nf);
   for (int f = 0; f < h->nf; ++f)
@@ -1151,6 +1261,7 @@ void upload_topology(rs_bh *h) {
   upload_vec(h->leaf_of_pos, leaf_of_pos, s);
   upload_vec(h->chain_off, coff, s);
   upload_vec(h->chain, chain, s);
+  upload_vec(h->climb, climb, s);
   upload_vec(h->inc_off, ioff, s);
   upload_vec(h->inc, inc, s);
   upload_vec(h->leaf_ordinal, T.leaf_ordinal, s);
@@ -1393,15 +1504,23 @@ void check_positions_host(rs_bh *h, const double *pos) {
         fail(RS_NONFINITE_POSITION, "NonFinitePosition", "energy", "vertex " + std::to_string(v));
 }
 
-// Resident 256-thread blocks per SM of the pair kernel (a persistent grid: one wave).
+constexpr size_t kCoopItems = 4;
+using PairKernel = void (*)(BhDev, Pow);
+PairKernel pair_kernel(bool grad, bool fast, bool coop) {
+  static const PairKernel k[8] = {bh_pair_kernel<false, false, false>, bh_pair_kernel<false, true, false>,
+                                  bh_pair_kernel<true, false, false>,  bh_pair_kernel<true, true, false>,
+                                  bh_pair_kernel<false, false, true>,  bh_pair_kernel<false, true, true>,
+                                  bh_pair_kernel<true, false, true>,   bh_pair_kernel<true, true, true>};
+  return k[(coop ? 4 : 0) + (grad ? 2 : 0) + (fast ? 1 : 0)];
+}
+
+// Resident blocks per SM of the pair kernel with a warp per item (a persistent grid: one wave).
 int pair_blocks_per_sm(bool grad, bool fast) {
   static int cache[4] = {0, 0, 0, 0};
   int &c = cache[(grad ? 2 : 0) + (fast ? 1 : 0)];
   if (c == 0) {
-    const void *fn = grad ? (fast ? (const void *)bh_pair_kernel<true, true> : (const void *)bh_pair_kernel<true, false>)
-                          : (fast ? (const void *)bh_pair_kernel<false, true> : (const void *)bh_pair_kernel<false, false>);
     int b = 0;
-    RSG_CUDA("launch", cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, 128, 0));
+    RSG_CUDA("launch", cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (const void *)pair_kernel(grad, fast, false), 128, 0));
     c = b > 0 ? b : 1;
   }
   return c;
@@ -1415,16 +1534,13 @@ void evaluate(rs_bh *h, const Pow &pw, bool fast, bool grad, double *energy_dev,
   size_t nl = h->tree.leaves.size(), nn = h->tree.n_nodes();
   Profiler &P = h->prof;
   RSG_CUDA("launch", cudaMemsetAsync(h->ticket.p, 0, sizeof(unsigned), s));
-  unsigned grid = (unsigned)std::min<size_t>((size_t)h->ctx->sm_count * pair_blocks_per_sm(grad, fast),
-                                             blocks(h->n_items, 4));
+  // four warps to an item where there are at most kCoopItems of them per SM
+  const bool coop = h->n_items <= kCoopItems * (size_t)h->ctx->sm_count;
+  const unsigned grid = coop ? (unsigned)h->n_items
+                             : (unsigned)std::min<size_t>((size_t)h->ctx->sm_count * pair_blocks_per_sm(grad, fast),
+                                                          blocks(h->n_items, 4));
   P.begin(s, grad ? "bh_pair_grad" : "bh_pair_value");
-  if (grad) {
-    if (fast) bh_pair_kernel<true, true><<<grid, 128, 0, s>>>(d, pw);
-    else bh_pair_kernel<true, false><<<grid, 128, 0, s>>>(d, pw);
-  } else {
-    if (fast) bh_pair_kernel<false, true><<<grid, 128, 0, s>>>(d, pw);
-    else bh_pair_kernel<false, false><<<grid, 128, 0, s>>>(d, pw);
-  }
+  pair_kernel(grad, fast, coop)<<<grid, 128, 0, s>>>(d, pw);
   RSG_LAUNCHED(h->ctx, "bh_pair");
   P.end(s);
   if (grad) {

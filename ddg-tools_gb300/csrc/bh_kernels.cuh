@@ -33,6 +33,7 @@ struct BhDev {
   const uint32_t *node_end;    // N
   const uint32_t *node_right;  // N
   const uint32_t *node_parent; // N (root: 0)
+  const uint4 *climb;          // L: the refit's climb within a block of leaves (upload_topology)
   const uint32_t *leaves;      // L: node id of each leaf
   const uint32_t *leaf_of_pos; // F: leaf ordinal of each BVH position
   const uint32_t *schedule;    // work items, most work first
@@ -133,8 +134,9 @@ __device__ __forceinline__ void kernel_k(const Pow &p, float nu, float r2, float
 // Kahan-compensated FP32 accumulator.
 struct Kahan {
   float s = 0.f, c = 0.f;
-  __device__ __forceinline__ void add(float x) {
-    float y = x - c;
+  __device__ __forceinline__ void add(float x) { put(x - c); }
+  __device__ __forceinline__ void add(float a, float b) { put(__fmaf_rn(a, b, -c)); }  // a b, rounded once
+  __device__ __forceinline__ void put(float y) {
     float t = s + y;
     c = (t - s) - y;
     s = t;
