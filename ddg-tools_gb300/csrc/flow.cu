@@ -94,22 +94,36 @@ void volume_gradient(int nv, int nf, const uint32_t *f, const double *p, double 
   }
 }
 
-double mean_edge_length(int nf, const uint32_t *f, const double *p) {
-  std::vector<std::pair<uint32_t, uint32_t>> e;
-  e.reserve(3 * (size_t)nf);
-  for (int i = 0; i < nf; ++i)
-    for (int c = 0; c < 3; ++c) {
-      uint32_t a = f[3 * i + c], b = f[3 * i + (c + 1) % 3];
-      e.push_back({std::min(a, b), std::max(a, b)});
-    }
-  std::sort(e.begin(), e.end());
-  e.erase(std::unique(e.begin(), e.end()), e.end());
-  double s = 0.0;
-  for (auto [a, b] : e) {
-    const double *x = p + 3 * (size_t)a, *y = p + 3 * (size_t)b;
-    s += std::sqrt((x[0] - y[0]) * (x[0] - y[0]) + (x[1] - y[1]) * (x[1] - y[1]) + (x[2] - y[2]) * (x[2] - y[2]));
+// over the edges in increasing order of their lower, then their higher vertex
+double mean_edge_length(int nv, int nf, const uint32_t *f, const double *p) {
+  // the higher vertices of the edges of every lower vertex, an edge of two faces twice
+  std::vector<uint32_t> ptr((size_t)nv + 1, 0), far(3 * (size_t)nf);
+  auto edges = [&](auto visit) {
+    for (int i = 0; i < nf; ++i)
+      for (int c = 0; c < 3; ++c) {
+        const uint32_t a = f[3 * (size_t)i + c], b = f[3 * (size_t)i + (c + 1) % 3];
+        visit(std::min(a, b), std::max(a, b));
+      }
+  };
+  edges([&](uint32_t a, uint32_t) { ptr[a + 1]++; });
+  for (int v = 0; v < nv; ++v) ptr[v + 1] += ptr[v];
+  {
+    std::vector<uint32_t> fill(ptr.begin(), ptr.end() - 1);
+    edges([&](uint32_t a, uint32_t b) { far[fill[a]++] = b; });
   }
-  return s / (double)e.size();
+  double s = 0.0;
+  size_t n = 0;
+  for (int a = 0; a < nv; ++a) {
+    uint32_t *b = far.data() + ptr[a], *e = far.data() + ptr[a + 1];
+    std::sort(b, e);
+    e = std::unique(b, e);
+    n += (size_t)(e - b);
+    for (const double *x = p + 3 * (size_t)a; b < e; ++b) {
+      const double *y = p + 3 * (size_t)*b;
+      s += std::sqrt((x[0] - y[0]) * (x[0] - y[0]) + (x[1] - y[1]) * (x[1] - y[1]) + (x[2] - y[2]) * (x[2] - y[2]));
+    }
+  }
+  return s / (double)n;
 }
 
 template <class T>
@@ -208,7 +222,7 @@ int rs_flow_create(rs_ctx *ctx, int nv, int nf, const uint32_t *faces, const dou
       fail(RS_INVALID_OPTION, "InvalidOption", "flow", "start values must be finite and positive");
     if (!(o.tau_min_rel > 0.0 && std::isfinite(o.tau_min_rel)) || !(o.newton_tolerance > 0.0) || o.newton_max < 0)
       fail(RS_INVALID_OPTION, "InvalidOption", "flow", "tau_min_rel, newton_tolerance > 0, newton_max >= 0");
-    F->l0 = mean_edge_length(nf, faces, positions_host);
+    F->l0 = mean_edge_length(nv, nf, faces, positions_host);
     F->area_t = std::isnan(o.area_target) ? total_area(nf, faces, positions_host) : o.area_target;
     F->vol_t = std::isnan(o.volume_target) ? total_volume(nf, faces, positions_host) : o.volume_target;
     // barycenter groups numbered as the solver's positional rows: one global group, or one per

@@ -14,6 +14,8 @@
 #include "host_tree.hpp"
 
 #include <algorithm>
+#include <array>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <future>
@@ -52,6 +54,65 @@ TrustedTopology::TrustedTopology() : prev(g_topology_trusted) { g_topology_trust
 TrustedTopology::~TrustedTopology() { g_topology_trusted = prev; }
 bool topology_trusted() { return g_topology_trusted; }
 
+// Whether the faces around every vertex are one fan with at most kMaxFan of them, no two with the same
+// vertices: then every edge has one or two faces and the surface is valid. Faces of distinct
+// vertices in range. Each vertex is decided from its own corners, by walking from face to face over the
+// shared neighbours (the sorts of all faces and of all edges below take ten times as long: at 204,800 faces 41 against
+// 4.2 ms). A
+// false only says that the general checks have to decide, and name the fault.
+constexpr uint32_t kMaxFan = 64;
+static bool one_fan_everywhere(int nv, int nf, const uint32_t *faces) {
+  std::vector<uint32_t> ptr((size_t)nv + 1, 0);
+  for (size_t i = 0; i < 3 * (size_t)nf; ++i) ptr[faces[i] + 1]++;
+  for (int v = 0; v < nv; ++v) {
+    if (ptr[v + 1] == 0 || ptr[v + 1] > kMaxFan) return false;
+    ptr[v + 1] += ptr[v];
+  }
+  std::vector<std::array<uint32_t, 2>> corner(3 * (size_t)nf);  // the two other vertices of a face
+  {
+    std::vector<uint32_t> fill(ptr.begin(), ptr.end() - 1);
+    for (int f = 0; f < nf; ++f) {
+      const uint32_t *t = faces + 3 * (size_t)f;
+      corner[fill[t[0]]++] = {t[1], t[2]};
+      corner[fill[t[1]]++] = {t[2], t[0]};
+      corner[fill[t[2]]++] = {t[0], t[1]};
+    }
+  }
+  std::atomic<bool> good{true};
+  parallel_for((size_t)nv, [&](size_t v0, size_t v1) {
+    for (size_t v = v0; v < v1; ++v) {
+      const std::array<uint32_t, 2> *c = corner.data() + ptr[v];
+      const uint32_t m = ptr[v + 1] - ptr[v];
+      uint32_t mate[kMaxFan][2];  // the face beyond each of a face's two edges at v, or m
+      uint32_t first = 0;
+      for (uint32_t i = 0; i < m; ++i)
+        for (int k = 0; k < 2; ++k) {
+          uint32_t found = m, n = 0;
+          for (uint32_t j = 0; j < m; ++j)
+            if (j != i && (c[j][0] == c[i][k] || c[j][1] == c[i][k])) found = j, ++n;
+          if (n > 1) {
+            good.store(false, std::memory_order_relaxed);
+            return;
+          }
+          mate[i][k] = found;
+          if (found == m) first = i;  // the fan is open: walk from an end
+        }
+      uint32_t seen = 1, at = first, from = m;
+      int k = mate[first][0] == m ? 1 : 0;
+      while (mate[at][k] != m && mate[at][k] != first && seen < m) {
+        if (mate[at][0] == mate[at][1]) break;  // two faces with the same vertices
+        from = at, at = mate[at][k], ++seen;
+        k = mate[at][0] == from ? 1 : 0;
+      }
+      if (seen != m) {
+        good.store(false, std::memory_order_relaxed);
+        return;
+      }
+    }
+  });
+  return good;
+}
+
 void validate_topology(int nv, int nf, const uint32_t *faces) {
   if (g_topology_trusted) return;
   if (nf <= 0) fail(RS_TOPOLOGY, "NoFaces", "surface", "the face list is empty");
@@ -66,6 +127,7 @@ void validate_topology(int nv, int nf, const uint32_t *faces) {
     if (t[0] == t[1] || t[1] == t[2] || t[0] == t[2])
       fail(RS_TOPOLOGY, "RepeatedVertex", "surface", "face " + s(f) + " repeats a vertex");
   }
+  if (one_fan_everywhere(nv, nf, faces)) return;
   {  // duplicates, surface.rs:163-196
     std::vector<std::pair<std::array<uint32_t, 3>, uint32_t>> keys((size_t)nf);
     for (int f = 0; f < nf; ++f) {
