@@ -5,8 +5,10 @@
 #include "krylov.hpp"
 #include "profile.hpp"
 
+#include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <type_traits>
 
 namespace rsg {
 
@@ -16,43 +18,79 @@ constexpr int RB = 256;  // reduction blocks of the dot products (fixed: determi
 
 inline unsigned nb_(size_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
-// Partial sums of v_i . w over a fixed row split: block b owns rows [b c, (b+1) c).
 constexpr int kDotVecs = 8;  // vectors per pass over w
+constexpr int kMaxRhs = 4;   // right-hand sides of a launch
 
-// out[i] = v_i . w (sqrt of it with `root`) for i < nvec, v_i = vs[i] (or v1 when given, nvec =
-// 1). Each block takes a fixed row range and up to kDotVecs vectors per pass over it (w read
-// once per pass), reduces by warp shuffles and then over the warps in order, and writes its
-// partials; the last block to finish (a ticket counter, reset by that block) adds the
-// partials of every vector in block order, a warp per vector. Deterministic: the grid, the
-// row ranges and every reduction order are fixed.
-__global__ void __launch_bounds__(256) dots_kernel(const double *const *vs, const double *v1, int nvec,
-                                                   const double *__restrict__ w, size_t n, double *part,
-                                                   unsigned *ticket, double *out, int root) {
+// What a launch does for one right-hand side: the vectors v[i], i < nvec (or v1, nvec = 1), against w
+// (w also receives: axpy), and the scalars, out of the dots and into the axpy.
+struct RhsVecs {
+  const double *const *vs;
+  const double *v1;
+  int nvec;
+  double *w;
+  double *h;
+};
+struct RhsList {
+  RhsVecs r[kMaxRhs];
+};
+
+// The sums over a warp of eight values per lane, by a butterfly whose steps share the lanes
+// between the values: 9 FP64 additions (sixteen cycles each for a warp) instead of 40. Lane l
+// ends with value (l >> 4 & 1) + 2 (l >> 3 & 1) + 4 (l >> 2 & 1). Every addition joins the same two numbers as
+// a butterfly of its own would.
+__device__ __forceinline__ double warp_sums8(const double (&v)[8], int lane) {
+  const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
+  double a[4], b[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    a[i] = (u16 ? v[2 * i + 1] : v[2 * i]) + __shfl_xor_sync(0xffffffffu, u16 ? v[2 * i] : v[2 * i + 1], 16);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    b[i] = (u8 ? a[2 * i + 1] : a[2 * i]) + __shfl_xor_sync(0xffffffffu, u8 ? a[2 * i] : a[2 * i + 1], 8);
+  double c = (u4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, u4 ? b[0] : b[1], 4);
+  c += __shfl_xor_sync(0xffffffffu, c, 2);
+  return c + __shfl_xor_sync(0xffffffffu, c, 1);
+}
+
+// h[i] = v_i . w (sqrt of it with `root`) for every right-hand side (blockIdx.y). Each block takes a
+// fixed row range and up to kDotVecs vectors per pass over it (w read once per pass), reduces by warp
+// shuffles and then over the warps in order, and writes its partials; the last block of the
+// right-hand side to finish (a ticket counter, reset by that block) adds the partials of every
+// vector in block order, a warp per vector. Deterministic: the grid, the row ranges and every
+// reduction order are fixed.
+//
+// Bound by FP64: 307,200 rows and 15 vectors are 8 us of fused multiply-adds at two lanes per clock and
+// SM. A launch per right-hand side with a butterfly per vector took 33 us (the butterflies 9, and
+// 256 blocks of 8 warps leave most of an SM's FP64 time to latency).
+__global__ void __launch_bounds__(256) dots_kernel(const __grid_constant__ RhsList L, size_t n, double *part_all,
+                                                   unsigned *tickets, int root) {
   __shared__ double sh[8][kDotVecs];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const RhsVecs &Q = L.r[blockIdx.y];
+  const int nvec = Q.nvec;
+  const double *__restrict__ w = Q.w;
+  double *part = part_all + (size_t)blockIdx.y * RB * 64;
   const size_t chunk = (n + gridDim.x - 1) / gridDim.x;
   const size_t r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk);
-  for (int i0 = 0; i0 < nvec; i0 += kDotVecs) {
+  auto pass = [&](auto full, int i0) {
+    constexpr bool FULL = decltype(full)::value;
     const double *vp[kDotVecs];
     double acc[kDotVecs];
 #pragma unroll
     for (int j = 0; j < kDotVecs; ++j) {
-      vp[j] = (i0 + j < nvec) ? (v1 ? v1 : vs[i0 + j]) : nullptr;
+      vp[j] = (FULL || i0 + j < nvec) ? (Q.v1 ? Q.v1 : Q.vs[i0 + j]) : nullptr;
       acc[j] = 0.0;
     }
+#pragma unroll 2
     for (size_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
       const double wr = w[r];
 #pragma unroll
       for (int j = 0; j < kDotVecs; ++j)
-        if (vp[j]) acc[j] = fma(vp[j][r], wr, acc[j]);
+        if (FULL || vp[j]) acc[j] = fma(vp[j][r], wr, acc[j]);
     }
-#pragma unroll
-    for (int j = 0; j < kDotVecs; ++j) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-      if (lane == 0) sh[wid][j] = acc[j];
-    }
+    const double t8 = warp_sums8(acc, lane);
+    if ((lane & 3) == 0) sh[wid][(lane >> 4 & 1) + 2 * (lane >> 3 & 1) + 4 * (lane >> 2 & 1)] = t8;
     __syncthreads();
     if ((int)threadIdx.x < kDotVecs && i0 + (int)threadIdx.x < nvec) {
       double t = 0.0;
@@ -60,33 +98,43 @@ __global__ void __launch_bounds__(256) dots_kernel(const double *const *vs, cons
       part[(size_t)blockIdx.x * nvec + i0 + threadIdx.x] = t;
     }
     __syncthreads();
+  };
+  for (int i0 = 0; i0 < nvec; i0 += kDotVecs) {
+    if (i0 + kDotVecs <= nvec) pass(std::true_type{}, i0);
+    else pass(std::false_type{}, i0);
   }
   if (threadIdx.x == 0) {
     __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    last = atomicAdd(tickets + blockIdx.y, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
   for (int i = wid; i < nvec; i += (int)(blockDim.x >> 5)) {
-    double t = 0.0;
-    for (unsigned b = lane; b < gridDim.x; b += 32) t += __ldcg(part + (size_t)b * nvec + i);
+    double p[RB / 32], t = 0.0;
+#pragma unroll
+    for (int b = 0; b < RB / 32; ++b) p[b] = __ldcg(part + (size_t)(lane + 32 * b) * nvec + i);
+#pragma unroll
+    for (int b = 0; b < RB / 32; ++b) t += p[b];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) out[i] = root ? sqrt(t) : t;
+    if (lane == 0) Q.h[i] = root ? sqrt(t) : t;
   }
-  if (threadIdx.x == 0) *ticket = 0u;
+  if (threadIdx.x == 0) tickets[blockIdx.y] = 0u;
 }
 
-// w -= sum_i h_i v_i (sign = -1) or x += sum_i h_i v_i (sign = +1).
-__global__ void axpy_many_kernel(const double *const *vs, int nvec, const double *__restrict__ h,
-                                 double sign, double *w, size_t n) {
+// w -= sum_i h_i v_i (sign = -1) or w += sum_i h_i v_i (sign = +1), per right-hand side (blockIdx.y).
+__global__ void __launch_bounds__(256) axpy_many_kernel(const __grid_constant__ RhsList L, double sign, size_t n) {
   __shared__ double hs[64];
   __shared__ const double *vp[64];
-  if (threadIdx.x < nvec) hs[threadIdx.x] = h[threadIdx.x], vp[threadIdx.x] = vs[threadIdx.x];
+  const RhsVecs &Q = L.r[blockIdx.y];
+  const int nvec = Q.nvec;
+  if ((int)threadIdx.x < nvec) hs[threadIdx.x] = Q.h[threadIdx.x], vp[threadIdx.x] = Q.vs[threadIdx.x];
   __syncthreads();
+  double *w = Q.w;
   for (size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x; r < n; r += (size_t)gridDim.x * blockDim.x) {
     double acc = 0.0;
+#pragma unroll 4
     for (int i = 0; i < nvec; ++i) acc = fma(hs[i], vp[i][r], acc);
     w[r] = fma(sign, acc, w[r]);
   }
@@ -106,17 +154,34 @@ __global__ void sub_kernel(const double *a, const double *b, double *y, size_t n
 
 }  // namespace
 
-void dev_dots(rs_ctx *ctx, const double *const *vs, int nvec, const double *w, size_t n,
-              double *out_dev, const double *v1, bool root) {
+namespace {
+
+// the dots of `count` right-hand sides in one launch
+void launch_dots(rs_ctx *ctx, const RhsList &L, int count, size_t n, bool root) {
   static thread_local DevBuf<double> partial;
   static thread_local DevBuf<unsigned> ticket;
-  if (nvec < 1 || nvec > 64) fail(RS_INTERNAL, "Internal", "gmres", "1 to 64 vectors per dot-product launch");
-  if (partial.n < (size_t)RB * 64) {
-    partial.alloc((size_t)RB * 64), ticket.alloc(1);
-    RSG_CUDA("gmres", cudaMemsetAsync(ticket.p, 0, sizeof(unsigned), ctx->stream));
+  for (int q = 0; q < count; ++q)
+    if (L.r[q].nvec < 1 || L.r[q].nvec > 64) fail(RS_INTERNAL, "Internal", "gmres", "1 to 64 vectors per dot-product launch");
+  if (partial.n < (size_t)RB * 64 * kMaxRhs) {
+    partial.alloc((size_t)RB * 64 * kMaxRhs), ticket.alloc(kMaxRhs);
+    RSG_CUDA("gmres", cudaMemsetAsync(ticket.p, 0, kMaxRhs * sizeof(unsigned), ctx->stream));
   }
-  dots_kernel<<<RB, 256, 0, ctx->stream>>>(vs, v1, nvec, w, n, partial.p, ticket.p, out_dev, root ? 1 : 0);
+  dots_kernel<<<dim3(RB, (unsigned)count), 256, 0, ctx->stream>>>(L, n, partial.p, ticket.p, root ? 1 : 0);
   RSG_LAUNCHED(ctx, "dots");
+}
+
+void launch_axpy(rs_ctx *ctx, const RhsList &L, int count, size_t n, double sign) {
+  axpy_many_kernel<<<dim3(nb_(n, 256), (unsigned)count), 256, 0, ctx->stream>>>(L, sign, n);
+  RSG_LAUNCHED(ctx, "axpy_many");
+}
+
+}  // namespace
+
+void dev_dots(rs_ctx *ctx, const double *const *vs, int nvec, const double *w, size_t n,
+              double *out_dev, const double *v1, bool root) {
+  RhsList L = {};
+  L.r[0] = RhsVecs{vs, v1, nvec, const_cast<double *>(w), out_dev};
+  launch_dots(ctx, L, 1, n, root);
 }
 
 namespace {
@@ -267,20 +332,23 @@ void gmres_batch(rs_ctx *ctx, const Operator &A, const Operator *P, int nb, cons
     }
     // classical Gram-Schmidt, twice; h = h1 + h2, then |w|
     if (opt.prof) opt.prof->begin(s, "gmres_orthogonalize");
-    for (int i = 0; i < na; ++i) {
-      Rhs &Q = R[act[i]];
-      Q.rep.operator_applications++;
-      const int k = Q.j + 1;
-      double *w = Q.w.p;
-      RSG_CUDA("gmres", cudaMemcpyAsync(w, ybuf.p + (size_t)i * n, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-      double *h1 = Q.h.p, *h2 = Q.h.p + (m + 2);
-      dev_dots(ctx, Q.vptr.p, k, w, n, h1);
-      axpy_many_kernel<<<nb_(n, 256), 256, 0, s>>>(Q.vptr.p, k, h1, -1.0, w, n);
-      RSG_LAUNCHED(ctx, "axpy_many");
-      dev_dots(ctx, Q.vptr.p, k, w, n, h2);
-      axpy_many_kernel<<<nb_(n, 256), 256, 0, s>>>(Q.vptr.p, k, h2, -1.0, w, n);
-      RSG_LAUNCHED(ctx, "axpy_many");
-      norm_dev(Q, w, Q.h.p + 2 * (m + 2));
+    for (int i = 0; i < na; ++i) R[act[i]].rep.operator_applications++;
+    for (int i0 = 0; i0 < na; i0 += kMaxRhs) {  // up to kMaxRhs right-hand sides per launch
+      const int c = std::min(kMaxRhs, na - i0);
+      RhsList h1 = {}, h2 = {}, nrm = {};
+      for (int i = 0; i < c; ++i) {
+        Rhs &Q = R[act[i0 + i]];
+        RSG_CUDA("gmres", cudaMemcpyAsync(Q.w.p, ybuf.p + (size_t)(i0 + i) * n, n * sizeof(double),
+                                          cudaMemcpyDeviceToDevice, s));
+        h1.r[i] = h2.r[i] = RhsVecs{Q.vptr.p, nullptr, Q.j + 1, Q.w.p, Q.h.p};
+        h2.r[i].h = Q.h.p + (m + 2);
+        nrm.r[i] = RhsVecs{nullptr, Q.w.p, 1, Q.w.p, Q.h.p + 2 * (m + 2)};
+      }
+      launch_dots(ctx, h1, c, n, false);
+      launch_axpy(ctx, h1, c, n, -1.0);
+      launch_dots(ctx, h2, c, n, false);
+      launch_axpy(ctx, h2, c, n, -1.0);
+      launch_dots(ctx, nrm, c, n, true);
     }
     if (opt.prof) opt.prof->end(s);
     std::vector<double> hh((size_t)na * (2 * (m + 2) + 1));
@@ -334,8 +402,9 @@ void gmres_batch(rs_ctx *ctx, const Operator &A, const Operator *P, int nb, cons
         y[t] = d != 0.0 ? sum / d : 0.0;
       }
       RSG_CUDA("gmres", rsg::copy_async(Q.h.p, y.data(), kk * sizeof(double), cudaMemcpyHostToDevice, s));
-      axpy_many_kernel<<<nb_(n, 256), 256, 0, s>>>(Q.zptr.p, kk, Q.h.p, 1.0, x + (size_t)act[i] * n, n);
-      RSG_LAUNCHED(ctx, "axpy_many");
+      RhsList xz = {};
+      xz.r[0] = RhsVecs{Q.zptr.p, nullptr, kk, x + (size_t)act[i] * n, Q.h.p};
+      launch_axpy(ctx, xz, 1, n, 1.0);
       RSG_CUDA("gmres", cudaStreamSynchronize(s));  // y lives on the host stack
       Q.active = false;
       Q.j = -1;  // cycle ended
