@@ -30,6 +30,7 @@
 #include "krylov.hpp"
 #include "learned.hpp"
 #include "dense.hpp"
+#include "fp64_bits.cuh"
 #include "profile.hpp"
 
 namespace rsg {
@@ -39,22 +40,60 @@ namespace {
 inline unsigned nblk(size_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 constexpr int GB = 128;  // reduction blocks of the group sums
 
-// The end of a group-sum launch: the block's K partials are in part; the last block to finish
-// (a ticket counter, reset by that block) adds every entry's partials in block order, a warp
-// per entry with the lanes strided over the blocks, and writes out.
-__device__ __forceinline__ void finish_group_sums(const double *part, int K, unsigned *ticket, double *out) {
+// out[q][3 g + k] = sum over the vertices v of group g of w_v x_q[3 v + k], load(q, v, w, x) giving the
+// weight and the three values. Blocks (b, y): the b-th share of the vertices, the vectors and groups
+// y, y + gridDim.y, ... A thread accumulates over a strided subset, a fixed tree adds a warp's threads, the
+// warps are added in order, and the last block to finish (a ticket counter, reset by that block)
+// adds every entry's partials in block order, a warp per entry with the lanes strided over the
+// blocks. The three axes share a sweep and the lanes of a tree (6 FP64 additions, sixteen cycles each for a
+// warp, instead of 15); with a sweep per vector and axis one after another the launch took 32 us for three vectors at
+// 102,400 vertices.
+constexpr int kGroupBlocks = 64;  // at most that many in y
+template <class Load>
+__device__ __forceinline__ void group_sums(Load load, int nb, int nv, const uint32_t *__restrict__ group, int G,
+                                           double *part, unsigned *ticket, double *out) {
+  __shared__ double wsum[8][4];
   __shared__ bool last;
-  __syncthreads();
+  const int K = 3 * G * nb, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const size_t chunk = (nv + gridDim.x - 1) / gridDim.x;
+  const size_t v0 = blockIdx.x * chunk, v1 = min((size_t)nv, v0 + chunk);
+  for (int qg = blockIdx.y; qg < nb * G; qg += gridDim.y) {
+    const int q = qg / G, g = qg - q * G;
+    double acc[3] = {0.0, 0.0, 0.0};
+    for (size_t v = v0 + threadIdx.x; v < v1; v += blockDim.x)
+      if ((int)group[v] == g) {
+        double w, x[3];
+        load(q, v, w, x);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) acc[k] = __fma_rn(w, x[k], acc[k]);
+      }
+    // 16 apart: lanes 0-15 keep axes 0 and 2, the others axis 1; 8 apart likewise
+    const bool u16 = lane & 16, u8 = lane & 8;
+    double a = u16 ? acc[1] : acc[0], b = u16 ? 0.0 : acc[2];
+    a += __shfl_xor_sync(0xffffffffu, u16 ? acc[0] : acc[1], 16);
+    b += __shfl_xor_sync(0xffffffffu, u16 ? acc[2] : 0.0, 16);
+    double c = (u8 ? b : a) + __shfl_xor_sync(0xffffffffu, u8 ? a : b, 8);
+#pragma unroll
+    for (int m = 4; m >= 1; m >>= 1) c += __shfl_xor_sync(0xffffffffu, c, m);
+    if ((lane & 7) == 0) wsum[wid][(lane >> 4) + 2 * ((lane >> 3) & 1)] = c;
+    __syncthreads();
+    if (threadIdx.x < 3) {
+      double t = 0.0;
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += wsum[w][threadIdx.x];
+      part[(size_t)blockIdx.x * K + 3 * qg + threadIdx.x] = t;
+    }
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
     __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    last = atomicAdd(ticket, 1u) == gridDim.x * gridDim.y - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  const int lane = threadIdx.x & 31;
-  for (int i = threadIdx.x >> 5; i < K; i += (int)(blockDim.x >> 5)) {
+  for (int i = wid; i < K; i += (int)(blockDim.x >> 5)) {
     double t = 0.0;
+#pragma unroll 4
     for (unsigned b = lane; b < gridDim.x; b += 32) t += __ldcg(part + (size_t)b * K + i);
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (lane == 0) out[i] = t;
@@ -62,40 +101,17 @@ __device__ __forceinline__ void finish_group_sums(const double *part, int K, uns
   if (threadIdx.x == 0) *ticket = 0u;
 }
 
-// part[b][q][3 g + k] = sum over the block's vertices v of group g of wgt_v x_q[3 v + k]
-// (wgt = null: weight 1). x has leading dimension ld; G groups.
-__global__ void group_sums_partial(const double *__restrict__ x, size_t ld, int nb, int nv,
-                                   const uint32_t *__restrict__ group, const double *__restrict__ wgt,
-                                   int G, double *part, unsigned *ticket, double *out) {
-  extern __shared__ double sh[];  // 3 G nb per block
-  const int K = 3 * G * nb;
-  for (int i = threadIdx.x; i < K; i += blockDim.x) sh[i] = 0.0;
-  __syncthreads();
-  const size_t chunk = (nv + gridDim.x - 1) / gridDim.x;
-  const size_t v0 = blockIdx.x * chunk, v1 = min((size_t)nv, v0 + chunk);
-  // each thread accumulates privately over a strided subset, then a fixed-order tree
-  for (int q = 0; q < nb; ++q)
-    for (int g = 0; g < G; ++g)
-      for (int k = 0; k < 3; ++k) {
-        double acc = 0.0;
-        for (size_t v = v0 + threadIdx.x; v < v1; v += blockDim.x)
-          if ((int)group[v] == g) acc += (wgt ? wgt[v] : 1.0) * x[q * ld + 3 * v + k];
-        // warp tree then lane-0 adds in warp order
-        for (int m = 16; m >= 1; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-        __shared__ double wsum[32];
-        if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-          double t = 0.0;
-          for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += wsum[w];
-          sh[(q * G + g) * 3 + k] = t;
-        }
-        __syncthreads();
-      }
-  for (int i = threadIdx.x; i < K; i += blockDim.x) part[(size_t)blockIdx.x * K + i] = sh[i];
-  finish_group_sums(part, K, ticket, out);
+// of nb vectors of leading dimension ld, weighted by wgt (null: 1)
+__global__ void __launch_bounds__(256) group_sums_kernel(const double *__restrict__ x, size_t ld, int nb, int nv,
+                                                         const uint32_t *__restrict__ group,
+                                                         const double *__restrict__ wgt, int G, double *part,
+                                                         unsigned *ticket, double *out) {
+  group_sums([&](int q, size_t v, double &w, double (&o)[3]) {
+    w = wgt ? wgt[v] : 1.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) o[k] = x[q * ld + 3 * v + k];
+  }, nb, nv, group, G, part, ticket, out);
 }
-
 
 // Operator tail: y_pos += c_v l_{g(v)} and y_mult = C_Q x (from the group sums `cx`).
 __global__ void cq_apply_kernel(const double *__restrict__ x, double *__restrict__ y, size_t ld,
@@ -361,8 +377,8 @@ struct rs_solver {
                      double *out) {
     int K = 3 * ng * nb;
     if (part.n < (size_t)GB * K) part.alloc((size_t)GB * K);
-    group_sums_partial<<<GB, 256, (size_t)K * sizeof(double), st()>>>(x, ld, nb, nv, grp, wgt, ng, part.p,
-                                                                      gs_ticket.p, out);
+    group_sums_kernel<<<dim3(GB, (unsigned)std::min(nb * ng, kGroupBlocks)), 256, 0, st()>>>(
+        x, ld, nb, nv, grp, wgt, ng, part.p, gs_ticket.p, out);
     RSG_LAUNCHED(ctx, "group_sums");
   }
 
@@ -516,29 +532,15 @@ __global__ void add_kernel(size_t m, const double *x, double *y) {
   if (i < m) y[i] += x[i];
 }
 // cy[q][3g + k] = sum_{v in g} c_v yy[v][3q + k]  (weighted group sums on the multigrid layout)
-__global__ void mg_group_partial(const mgreal *__restrict__ yy, int nb, int nv,
-                                 const uint32_t *__restrict__ group, const double *__restrict__ c,
-                                 int G, double *part, unsigned *ticket, double *out) {
-  const int K = 3 * G * nb;
-  const size_t chunk = (nv + gridDim.x - 1) / gridDim.x;
-  const size_t v0 = blockIdx.x * chunk, v1 = min((size_t)nv, v0 + chunk);
-  __shared__ double wsum[32];
-  for (int i = 0; i < K; ++i) {
-    int q = i / (3 * G), g = (i % (3 * G)) / 3, k = i % 3;
-    double acc = 0.0;
-    for (size_t v = v0 + threadIdx.x; v < v1; v += blockDim.x)
-      if ((int)group[v] == g) acc += c[v] * (double)yy[v * 3 * nb + 3 * q + k];
-    for (int m = 16; m >= 1; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += wsum[w];
-      part[(size_t)blockIdx.x * K + i] = t;
-    }
-    __syncthreads();
-  }
-  finish_group_sums(part, K, ticket, out);
+__global__ void __launch_bounds__(256) mg_group_kernel(const mgreal *__restrict__ yy, int nb, int nv,
+                                                       const uint32_t *__restrict__ group,
+                                                       const double *__restrict__ c, int G, double *part,
+                                                       unsigned *ticket, double *out) {
+  group_sums([&](int q, size_t v, double &w, double (&o)[3]) {
+    w = c[v];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) o[k] = f2d(yy[v * 3 * nb + 3 * q + k]);
+  }, nb, nv, group, G, part, ticket, out);
 }
 
 }  // namespace
@@ -555,7 +557,8 @@ void rs_solver::add_into(size_t m, const double *x, double *y) {
 void rs_solver::pos_copy_weighted(int nb) {
   int K = 3 * G * nb;
   if (part.n < (size_t)GB * K) part.alloc((size_t)GB * K);
-  mg_group_partial<<<GB, 256, 0, st()>>>(mg_out.p, nb, nv, group.p, c.p, G, part.p, gs_ticket.p, cy.p);
+  mg_group_kernel<<<dim3(GB, (unsigned)std::min(nb * G, kGroupBlocks)), 256, 0, st()>>>(mg_out.p, nb, nv, group.p, c.p,
+                                                                                        G, part.p, gs_ticket.p, cy.p);
   RSG_LAUNCHED(ctx, "mg_group");
 }
 
