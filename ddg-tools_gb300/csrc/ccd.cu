@@ -21,9 +21,11 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "common.hpp"
+#include "fp64_bits.cuh"
 
 namespace rsg {
 namespace {
@@ -116,15 +118,38 @@ struct Tally {
   unsigned long long pairs = 0, close = 0, touching = 0, evals = 0;
 };
 
+struct Params {
+  const double3 *start, *vel;
+  const double *speed;
+  const uint32_t *faces;  // 3 per face
+  const uint32_t *edges;  // 2 per edge
+  const DBox *vbox;
+  const uint8_t *band;    // exempt band per vertex, or null
+  int nv, ne, nf, max_iterations;
+  double gap_abs, close_factor, h, lo, hi;
+  unsigned long long *best;   // bits of the earliest contact time (+inf: none)
+  unsigned long long *tally;  // pairs, close, touching, evaluations, exempt
+  int *overflow;
+};
+
+constexpr double kMargin = 1.0 + 1e-12;  // ccd.rs:498-499
+
+__device__ __forceinline__ double horizon(const Params &P) {
+  const double b = __longlong_as_double((long long)*(volatile unsigned long long *)P.best);
+  return fmin(b, P.hi);
+}
+
 // Conservative advancement of one pair on [lo, hz] (advance, RS/src/ccd.rs:529-592); returns
 // the contact time or -1 for none. When a step would pass hz with the cheap bound, the
 // reference retries with the refined bound l' and takes min(l, l'); that step is at least as
 // long, so it passes hz too and the pair has no contact before hz. The retry is therefore
 // left out: the result is the same. Every iterate that stays below hz is the reference's, so
 // a contact time below the horizon does not depend on the horizon.
-template <class Dist>
-__device__ double advance(const Dist &dist, double l, double gap_abs, int max_iterations, double close_factor,
-                          double lo, double hz, Tally &tally) {
+// no_contact(target) may decide after the first distance that no iterate below the horizon ends the
+// loop. The horizon is read at every step: it only falls.
+template <class Dist, class Early>
+__device__ double advance(const Dist &dist, const Early &no_contact, const Params &P, double l, Tally &tally) {
+  const double gap_abs = P.gap_abs, lo = P.lo;
   const double d0 = dist(0.0);
   tally.pairs += 1;
   tally.evals += 1;
@@ -137,15 +162,17 @@ __device__ double advance(const Dist &dist, double l, double gap_abs, int max_it
   } else if (d0 <= 1e-12 * gap_abs) {
     return -1.0;
   }
-  const double target = d0 > gap_abs ? gap_abs : close_factor * d0;
+  const double target = d0 > gap_abs ? gap_abs : P.close_factor * d0;
   const double slack = 1e-9 * d0;
+  if (no_contact(target)) return -1.0;
   double tau = lo;
   double d = d0;
   if (lo != 0.0) {
     d = dist(lo);
     tally.evals += 1;
   }
-  for (int it = 0; it < max_iterations; ++it) {
+  for (int it = 0; it < P.max_iterations; ++it) {
+    const double hz = horizon(P);
     if (isnan(d) || d - target <= slack) return tau;
     const double next = tau + (d - target) / l;
     if (next >= hz || isnan(next)) return -1.0;
@@ -219,23 +246,26 @@ __global__ void prim_box_kernel(int n, const uint32_t *verts, const DBox *vbox, 
   idx[i] = (uint32_t)i;
 }
 
-__global__ void gather_boxes_kernel(int n, const uint32_t *order, const DBox *box, DBox *sbox) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) sbox[i] = box[order[i]];
-}
 
 // Node boxes of the walk in FP32, rounded outward: a node box contains the FP64 union of its
 // elements' boxes, so the walk visits every leaf block the FP64 tree would (it may visit more;
 // the element test below is exact).
-struct FBox {
-  float lo[3], hi[3];
+struct alignas(32) FBox {  // two 16-byte loads
+  float lo[3], pad0, hi[3], pad1;
 };
 
 __device__ __forceinline__ FBox outward(const DBox &b) {
   FBox r;
+  r.pad0 = r.pad1 = 0.f;
 #pragma unroll
   for (int k = 0; k < 3; ++k) r.lo[k] = __double2float_rd(b.lo[k]), r.hi[k] = __double2float_ru(b.hi[k]);
   return r;
+}
+
+__device__ __forceinline__ FBox load_box(const FBox *p) {
+  const float4 *q = reinterpret_cast<const float4 *>(p);
+  const float4 a = __ldg(q), b = __ldg(q + 1);
+  return FBox{{a.x, a.y, a.z}, 0.f, {b.x, b.y, b.z}, 0.f};
 }
 
 __device__ __forceinline__ bool overlaps_f(const FBox &a, const FBox &b) {
@@ -243,6 +273,11 @@ __device__ __forceinline__ bool overlaps_f(const FBox &a, const FBox &b) {
   for (int k = 0; k < 3; ++k)
     if (!(a.lo[k] <= b.hi[k] && b.lo[k] <= a.hi[k])) return false;
   return true;
+}
+
+__global__ void gather_boxes_kernel(int n, const uint32_t *order, const DBox *box, DBox *sbox) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) sbox[i] = box[order[i]];
 }
 
 // level 0: unions of blocks of 8 sorted element boxes (FP64, then rounded outward)
@@ -269,63 +304,53 @@ __global__ void level_kernel(int n_out, const FBox *in, int n_in, FBox *out) {
   out[i] = r;
 }
 
+constexpr int kMaxLevels = 62;
+constexpr int kLeaf = 8;  // elements of a block (level0_kernel)
+
 struct Tree {
   const DBox *sbox;      // sorted element boxes (FP64, the exact test)
   const uint32_t *order; // sorted position -> element
   const FBox *levels;    // all levels, level 0 first
-  const int *lvl_off;    // offset of each level in `levels`
-  const int *lvl_len;
-  int n, n_levels, leaf;
+  int n, n_levels;
+  int lvl_off[kMaxLevels], lvl_len[kMaxLevels];  // place of each level in `levels`, its nodes
 };
 
 constexpr int kStack = 64;
 
-// Calls f(element) for every element whose FP64 box overlaps q (query, ccd.rs:359-389).
-// Returns false if the stack would overflow (not reachable: a depth-first walk of a tree of
-// n_levels <= 62 levels holds at most n_levels + 1 entries).
+// Calls f(element) for every element at a sorted place >= from whose FP64 box overlaps q (query,
+// ccd.rs:359-389). Returns false if the stack would overflow (not reachable: a depth-first walk of a
+// tree of n_levels <= 62 levels holds at most n_levels + 1 entries). A node is tested when its
+// parent is opened, so both children's boxes are loaded together.
 template <class F>
-__device__ bool query(const Tree &t, const DBox &q, F &&f) {
+__device__ __forceinline__ bool query(const Tree &t, bool mine, const DBox &q, int from, F &&f) {
+  __shared__ int off[kMaxLevels], len[kMaxLevels];  // indexed by a lane's own level
+  for (int k = threadIdx.x; k < t.n_levels; k += blockDim.x) off[k] = t.lvl_off[k], len[k] = t.lvl_len[k];
+  __syncthreads();
+  if (!mine) return true;
   const FBox qf = outward(q);
-  int2 stack[kStack];
+  uint32_t stack[kStack];  // overlapping nodes: the level above 26 bits of place
   int sp = 0;
-  stack[sp++] = make_int2(t.n_levels - 1, 0);
+  if (overlaps_f(load_box(t.levels + off[t.n_levels - 1]), qf)) stack[sp++] = (uint32_t)(t.n_levels - 1) << 26;
   while (sp > 0) {
-    const int2 e = stack[--sp];
-    if (!overlaps_f(t.levels[t.lvl_off[e.x] + e.y], qf)) continue;
-    if (e.x == 0) {
-      const int b = e.y * t.leaf, end = min(b + t.leaf, t.n);
-      for (int pos = b; pos < end; ++pos)
+    const uint32_t e = stack[--sp];
+    const int l = (int)(e >> 26), at = (int)(e & 0x3ffffffu);
+    if (l == 0) {
+      const int end = min((at + 1) * kLeaf, t.n);
+#pragma unroll 4
+      for (int pos = max(at * kLeaf, from); pos < end; ++pos)
         if (overlaps(t.sbox[pos], q)) f(t.order[pos]);
     } else {
       if (sp + 2 > kStack) return false;
-      stack[sp++] = make_int2(e.x - 1, 2 * e.y);
-      if (2 * e.y + 1 < t.lvl_len[e.x - 1]) stack[sp++] = make_int2(e.x - 1, 2 * e.y + 1);
+      const FBox *c = t.levels + off[l - 1] + 2 * at;
+      const bool two = 2 * at + 1 < len[l - 1];
+      const bool one = ((long long)(2 * at + 1) * kLeaf << (l - 1)) > from;  // reaches past `from`
+      const FBox c0 = load_box(one ? c : c + 1), c1 = load_box(two ? c + 1 : c);
+      const uint32_t e0 = (uint32_t)(l - 1) << 26 | (uint32_t)(2 * at);
+      if (one && overlaps_f(c0, qf)) stack[sp++] = e0;
+      if (two && overlaps_f(c1, qf)) stack[sp++] = e0 + 1;
     }
   }
   return true;
-}
-
-struct Params {
-  const double3 *start, *vel;
-  const double *speed;
-  const uint32_t *faces;  // 3 per face
-  const uint32_t *edges;  // 2 per edge
-  const DBox *vbox;
-  const DBox *ebox;       // inflated, element order
-  const DBox *fbox;       // face boxes, element order (the band's face-face walk)
-  const uint8_t *band;    // exempt band per vertex, or null
-  int nv, ne, nf, max_iterations;
-  double gap_abs, close_factor, h, lo, hi;
-  unsigned long long *best;   // bits of the earliest contact time (+inf: none)
-  unsigned long long *tally;  // pairs, close, touching, evaluations, exempt
-  int *overflow;
-};
-
-constexpr double kMargin = 1.0 + 1e-12;  // ccd.rs:498-499
-
-__device__ __forceinline__ double horizon(const Params &P) {
-  const double b = __longlong_as_double((long long)*(volatile unsigned long long *)P.best);
-  return fmin(b, P.hi);
 }
 
 __device__ void flush_tally(const Params &P, const Tally &t) {
@@ -340,10 +365,16 @@ __device__ void flush_tally(const Params &P, const Tally &t) {
 
 // Broad phase, one thread per query: KIND 0 a vertex against the face tree (the vertex not in
 // the face, ccd.rs:937-985), KIND 1 an edge against the edge tree (partners e2 > e without a
-// common vertex, ccd.rs:987-1038). FILL 0 counts each query's candidates; FILL 1 writes them
-// as (query, element) from the query's offset, in the walk's order.
+// common vertex, ccd.rs:987-1038).
 // KIND 2 (the band): a face against the face tree of the static hulls, partners g > f
 // (intersecting_pairs, ccd.rs:1229-1279); the intersection test runs per pair afterwards.
+// Within one kind the thread of a sorted place takes the places after it, so that every pair is
+// met once, half of the tree is never opened and a warp's queries are neighbours on the curve; the
+// pair is stored by increasing element.
+// Bound by the scattered box loads and the FP64 tests of the elements. Edges of 204,800 faces: 2.0 ms
+// with the queries in element order, half of the partners met twice, and a node tested when it was
+// popped; 1.4 with children tested together. An FP32 test before the FP64 one costs more in
+// loads than it saves (1.7).
 // A pair whose two elements both have a vertex in the band is exempt (ccd.rs:947-950,
 // 1001-1004): it is not a candidate, and it is counted in `counters[1]`.
 // Candidates are appended as (query, element) to `pairs`: each thread buffers up to 16 and
@@ -353,12 +384,12 @@ __device__ void flush_tally(const Params &P, const Tally &t) {
 constexpr int kAppend = 16;
 
 template <int KIND>
-__global__ void __launch_bounds__(128) walk_kernel(Params P, Tree t, unsigned long long *counters, uint2 *pairs,
+__global__ void __launch_bounds__(128) walk_kernel(Params P, const __grid_constant__ Tree t, unsigned long long *counters, uint2 *pairs,
                                                    unsigned long long cap) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
   const int nq = KIND == 0 ? P.nv : (KIND == 1 ? P.ne : P.nf);
-  if (q >= nq) return;
-  const DBox qb = KIND == 0 ? inflate(P.vbox[q], P.h) : (KIND == 1 ? P.ebox[q] : P.fbox[q]);
+  const int q0 = blockIdx.x * blockDim.x + threadIdx.x, place = min(q0, nq - 1);
+  const uint32_t q = KIND == 0 ? (uint32_t)place : t.order[place];
+  const DBox qb = KIND == 0 ? inflate(P.vbox[q], P.h) : t.sbox[place];
   uint32_t a = 0, b = 0;
   if (KIND == 1) a = P.edges[2 * q], b = P.edges[2 * q + 1];
   const bool qband = P.band && (KIND == 0 ? P.band[q] : (KIND == 1 ? (P.band[a] || P.band[b]) : false));
@@ -368,27 +399,24 @@ __global__ void __launch_bounds__(128) walk_kernel(Params P, Tree t, unsigned lo
   auto flush = [&]() {
     const unsigned long long base = atomicAdd(counters, (unsigned long long)nb);
     for (int i = 0; i < nb; ++i)
-      if (base + i < cap) pairs[base + i] = make_uint2((uint32_t)q, buf[i]);
+      if (base + i < cap) pairs[base + i] = KIND == 0 ? make_uint2(q, buf[i]) : make_uint2(min(q, buf[i]), max(q, buf[i]));
     nb = 0;
   };
-  const bool ok = query(t, qb, [&](uint32_t el) {
+  const bool ok = query(t, q0 < nq, qb, KIND == 0 ? 0 : place + 1, [&](uint32_t el) {
     if (KIND == 0) {
       const uint32_t fa = P.faces[3 * el], fb = P.faces[3 * el + 1], fc = P.faces[3 * el + 2];
-      if (fa == (uint32_t)q || fb == (uint32_t)q || fc == (uint32_t)q) return;
+      if (fa == q || fb == q || fc == q) return;
       if (qband && (P.band[fa] || P.band[fb] || P.band[fc])) {
         ++exempt;
         return;
       }
     } else if (KIND == 1) {
-      if (el <= (uint32_t)q) return;
       const uint32_t c = P.edges[2 * el], d = P.edges[2 * el + 1];
       if (c == a || c == b || d == a || d == b) return;
       if (qband && (P.band[c] || P.band[d])) {
         ++exempt;
         return;
       }
-    } else {
-      if (el <= (uint32_t)q) return;
     }
     buf[nb++] = el;
     if (nb == kAppend) flush();
@@ -453,40 +481,233 @@ __global__ void count_flags_kernel(int n, const uint8_t *flag, unsigned long lon
   if ((threadIdx.x & 31) == 0 && m) atomicAdd(count, (unsigned long long)__popc(m));
 }
 
-// Narrow phase, one thread per candidate pair: the lanes of a warp evaluate their distances
-// together. KIND 0: (vertex, face); KIND 1: (edge, edge).
+// ---- narrow phase
+//
+// The contact times are the reference's FP64 advancement, whose distances cost a warp some 300 FP64
+// instructions of sixteen cycles each: 560,000 vertex-face and 1.8 million edge-edge pairs took 3.3 and 2.3
+// ms, nearly all of them to find no contact before the horizon. filter_kernel decides those in FP32:
+//
+// * A lower bound of the distance at time t: for any direction u, the gap between the two elements'
+//   projections on u. u points between the FP32 closest points; where they are wrong the bound is only
+//   weaker. The relative positions carry 4 2^-24 M per component (M: the largest component until the
+//   horizon), a projection 25 2^-24 M between two elements, and u is at most 2^-21 too long:
+//   2^-19 M and a factor 1 - 2^-20 are taken off, and 2^-44 of the positions for the FP64 distance's own
+//   rounding. The FP64 point-plane distance loses digits on slivers: those go to FP64 at once.
+// * The bound advanced as the reference's distance is, t <- t + (bound - gap) / l, rounded down. By
+//   induction each iterate is at most the reference's: the distance changes by at most l dt, and
+//   the margin is above its slack of 1e-9 d. So when an iterate passes the horizon within as many steps as the
+//   reference may take, the reference finds no contact.
+//
+// The pairs left, with their last iterate, are advanced in FP64 (narrow_kernel): first those whose
+// iterate is within a thousandth of the least, then the others, most of which begin past the contact
+// found. Filters 0.09 and 0.19 ms, the advancement of what is left 1.0.
+struct F3 {
+  float x, y, z;
+};
+__device__ __forceinline__ F3 operator+(F3 a, F3 b) { return F3{a.x + b.x, a.y + b.y, a.z + b.z}; }
+__device__ __forceinline__ F3 operator-(F3 a, F3 b) { return F3{a.x - b.x, a.y - b.y, a.z - b.z}; }
+__device__ __forceinline__ F3 operator*(float s, F3 a) { return F3{s * a.x, s * a.y, s * a.z}; }
+__device__ __forceinline__ float dot(F3 a, F3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ F3 cross(F3 a, F3 b) {
+  return F3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+}
+__device__ __forceinline__ F3 narrow3(double3 a, double3 b) { return F3{d2f(a.x - b.x), d2f(a.y - b.y), d2f(a.z - b.z)}; }
+__device__ __forceinline__ float largest(F3 a) { return fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)); }
+__device__ __forceinline__ float largest(double3 a) {
+  return fmaxf(fmaxf(fabsf(d2f(a.x)), fabsf(d2f(a.y))), fabsf(d2f(a.z)));
+}
+__device__ __forceinline__ float unit(float x) { return fminf(fmaxf(x, 0.f), 1.f); }
+
+// The gap between the projections on the direction of v of 0 and the triangle r (KIND 0), or of the
+// segments 0 r[0] and r[1] r[2] (KIND 1); NaN where v is too short for its length.
 template <int KIND>
-__global__ void __launch_bounds__(128) narrow_kernel(Params P, const uint2 *pairs, unsigned long long n) {
-  const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ float separation(const F3 (&r)[3], F3 v) {
+  const float q = dot(v, v);
+  if (!(q > 0x1p-100f)) return __int_as_float(0x7fffffff);
+  const F3 u = rsqrtf(q) * v;
+  const float a = dot(u, r[0]), b = dot(u, r[1]), c = dot(u, r[2]);
+  return KIND == 0 ? fminf(fminf(a, b), c) : fminf(b, c) - fmaxf(a, 0.f);
+}
+__device__ __forceinline__ float triangle_bound(const F3 (&r)[3]) {
+  const F3 ab = r[1] - r[0], ac = r[2] - r[0], bc = r[2] - r[1];
+  auto foot = [](F3 a, F3 d) {  // the point of the segment a, a + d closest to 0
+    const float e = dot(d, d);
+    return a + (e > 0.f ? unit(__fdividef(-dot(a, d), e)) : 0.f) * d;
+  };
+  F3 v = foot(r[0], ab), w = foot(r[1], bc);
+  if (dot(w, w) < dot(v, v)) v = w;
+  w = foot(r[0], ac);
+  if (dot(w, w) < dot(v, v)) v = w;
+  const F3 n = cross(ab, ac);
+  const float nn = dot(n, n), ee = dot(ab, ab) * dot(ac, ac);
+  if (!(ee > 0x1p-110f && nn > 0x1p-30f * ee)) return __int_as_float(0x7fffffff);  // a sliver
+  const float i = __fdividef(1.f, nn), s = -dot(cross(r[0], ac), n) * i, t = -dot(cross(ab, r[0]), n) * i;
+  if (s >= 0.f && t >= 0.f && s + t <= 1.f) v = (dot(r[0], n) * i) * n;
+  return separation<0>(r, v);
+}
+__device__ __forceinline__ float segment_bound(const F3 (&r)[3]) {
+  // the closest points s d1 and r[1] + t d2 (C. Ericson, Real-Time Collision Detection, 5.1.9)
+  const F3 d1 = r[0], d2 = r[2] - r[1];
+  const float a = dot(d1, d1), e = dot(d2, d2), f = -dot(d2, r[1]), c = -dot(d1, r[1]), b = dot(d1, d2), m = a * e - b * b;
+  float s = m > 0.f ? unit(__fdividef(b * f - c * e, m)) : 0.f;
+  const float t0 = __fdividef(b * s + f, e), t = unit(t0);
+  if (t != t0) s = unit(__fdividef(b * t - c, a));
+  return separation<1>(r, (r[1] + t * d2) - s * d1);
+}
+
+struct Survivors {
+  uint2 *list;      // the pair's place and the bits of its last iterate (0: to be advanced in any case)
+  unsigned *count;  // of the two kinds, then the bits of the least iterate above zero
+};
+constexpr int kFilterSteps = 128;
+
+// pair (KIND 0: vertex, face; KIND 1: edge, edge): its vertices, and the speed bound l
+template <int KIND>
+__device__ __forceinline__ void pair_vertices(const Params &P, uint2 pr, uint32_t (&v)[4], double &l) {
+  if (KIND == 0) {
+    v[0] = pr.x, v[1] = P.faces[3 * pr.y], v[2] = P.faces[3 * pr.y + 1], v[3] = P.faces[3 * pr.y + 2];
+    l = (P.speed[v[0]] + fmax(fmax(P.speed[v[1]], P.speed[v[2]]), P.speed[v[3]])) * kMargin;
+  } else {
+    v[0] = P.edges[2 * pr.x], v[1] = P.edges[2 * pr.x + 1], v[2] = P.edges[2 * pr.y], v[3] = P.edges[2 * pr.y + 1];
+    l = (fmax(P.speed[v[0]], P.speed[v[1]]) + fmax(P.speed[v[2]], P.speed[v[3]])) * kMargin;
+  }
+}
+
+// The FP32 form of a pair: positions and velocities relative to its first vertex.
+template <int KIND>
+struct NarrowPair {
+  F3 x[3], w[3];
+  float il, err;
+  __device__ __forceinline__ void load(const Params &P, const uint32_t (&v)[4], double l, float hz) {
+    const double3 p = P.start[v[0]], u = P.vel[v[0]];
+    float M = 0.f, W = 0.f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      x[k] = narrow3(P.start[v[k + 1]], p), w[k] = narrow3(P.vel[v[k + 1]], u);
+      M = fmaxf(M, largest(x[k])), W = fmaxf(W, largest(w[k]));
+    }
+    il = __fdiv_rd(1.f, __double2float_ru(l));
+    err = 0x1p-19f * (M + hz * W) + 0x1p-43f * (largest(p) + M + hz * (largest(u) + W));
+  }
+  __device__ __forceinline__ float bound(float t) const {
+    F3 r[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) r[k] = x[k] + t * w[k];
+    return (1.f - 0x1p-20f) * (KIND == 0 ? triangle_bound(r) : segment_bound(r)) - err;
+  }
+  // From t with the bound d towards `target`: true when an iterate passes hz within `steps`; else
+  // t is the last iterate.
+  __device__ __forceinline__ bool passes(float &t, float d, float target, float hz, int steps, Tally &tally) const {
+    for (int it = 0; it < steps && d > target; ++it) {
+      const float next = __fadd_rd(t, __fmul_rd(__fsub_rd(d, target), il));
+      if (next >= hz) return true;
+      if (!(next > t + 0x1p-18f * t)) break;
+      t = next;
+      d = bound(t);
+      tally.evals += 1;
+    }
+    return false;
+  }
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(128) filter_kernel(Params P, const uint2 *pairs, unsigned n, Survivors S) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
   Tally tally;
-  if (i < n) {
-    const uint2 pr = pairs[i];
-    double r;
+  bool left = i < n;
+  float t = 0.f;
+  if (left) {
+    uint32_t v[4];
+    double l;
+    pair_vertices<KIND>(P, pairs[i], v, l);
+    NarrowPair<KIND> q;
+    const float hz = __double2float_ru(P.hi), gap = __double2float_ru(P.gap_abs);
+    q.load(P, v, l, hz);
+    float d = q.bound(0.f);
+    tally.evals += 1;
+    if (d > gap) {  // neither touching nor close at the start
+      if (P.lo != 0.0) t = __double2float_rd(P.lo), d = q.bound(t);
+      left = !q.passes(t, d, gap, hz, min(kFilterSteps, P.max_iterations), tally);
+    }
+    if (!left) tally.pairs += 1;
+  }
+  // the survivors of a warp side by side, and the least iterate
+  const unsigned m = __ballot_sync(0xffffffffu, left);
+  if (m) {
+    unsigned base = 0, least = left && t > 0.f ? __float_as_uint(t) : 0x7f800000u;
+    if (lane == 0) base = atomicAdd(S.count + KIND, (unsigned)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (left) S.list[base + __popc(m & ((1u << lane) - 1u))] = make_uint2(i, __float_as_uint(t));
+    least = __reduce_min_sync(0xffffffffu, least);
+    if (lane == 0 && least != 0x7f800000u) atomicMin(S.count + 2, least);
+  }
+  flush_tally(P, tally);
+}
+
+// FP64 advancement of the pairs left, a block of either kind: FIRST those whose iterate is near the
+// least one and those that are close at the start, else the others. A launch lasts as long as its longest
+// chain of distances (up to max_iterations of 8 to 11 us each), so the chains of both kinds run
+// beside one another, and with at most kFewLeft pairs all go first (204,800 faces, a few hundred pairs:
+// 1.0 ms for one launch, 2.1 for two).
+constexpr unsigned kFewLeft = 4096;
+struct PairsLeft {
+  const uint2 *pairs[2];
+  Survivors left[2];
+  unsigned blocks[2];
+};
+
+template <int KIND, bool FIRST>
+__device__ __forceinline__ void narrow(const Params &P, const PairsLeft &L, unsigned block, Tally &tally) {
+  const uint2 *pairs = L.pairs[KIND];
+  const Survivors S = L.left[KIND];
+  const unsigned n = S.count[KIND];
+  const float lim = S.count[0] + S.count[1] <= kFewLeft ? INFINITY : __uint_as_float(S.count[2]) * (1.f + 0x1p-10f);
+  for (unsigned i = block * blockDim.x + threadIdx.x; i < n; i += L.blocks[KIND] * blockDim.x) {
+    const uint2 e = S.list[i];
+    const float t = __uint_as_float(e.y);
+    if (FIRST != (t <= lim)) continue;
+    const double hz = horizon(P);
+    if (t > 0.f && (double)t >= hz) {
+      tally.pairs += 1;
+      continue;
+    }
+    uint32_t v[4];
+    double lc, r;
+    pair_vertices<KIND>(P, pairs[e.x], v, lc);
+    // a pair that is close at the start has a target of its own, known only now
+    auto no_contact = [&](double target) {
+      if (t > 0.f || P.lo != 0.0) return false;
+      NarrowPair<KIND> q;
+      const float hzf = __double2float_ru(hz);
+      q.load(P, v, lc, hzf);
+      float at = 0.f;
+      return q.passes(at, q.bound(0.f), __double2float_ru(target), hzf, min(kFilterSteps, P.max_iterations), tally);
+    };
     if (KIND == 0) {
-      const uint32_t v = pr.x, f = pr.y;
-      const uint32_t a = P.faces[3 * f], b = P.faces[3 * f + 1], c = P.faces[3 * f + 2];
-      const double3 p = P.start[v], u = P.vel[v];
-      const double3 ta = at3(P.start[a], P.vel[a], 0.0), tb = at3(P.start[b], P.vel[b], 0.0),
-                    tc = at3(P.start[c], P.vel[c], 0.0);
-      const double3 ua = P.vel[a], ub = P.vel[b], uc = P.vel[c];
-      const double lc = (P.speed[v] + fmax(fmax(P.speed[a], P.speed[b]), P.speed[c])) * kMargin;
-      auto dist = [&](double t) {
-        return point_triangle_distance(at3(p, u, t), at3(ta, ua, t), at3(tb, ub, t), at3(tc, uc, t));
+      const double3 p = P.start[v[0]], u = P.vel[v[0]], ua = P.vel[v[1]], ub = P.vel[v[2]], uc = P.vel[v[3]];
+      const double3 ta = at3(P.start[v[1]], ua, 0.0), tb = at3(P.start[v[2]], ub, 0.0), tc = at3(P.start[v[3]], uc, 0.0);
+      auto dist = [&](double at) {
+        return point_triangle_distance(at3(p, u, at), at3(ta, ua, at), at3(tb, ub, at), at3(tc, uc, at));
       };
-      r = advance(dist, lc, P.gap_abs, P.max_iterations, P.close_factor, P.lo, horizon(P), tally);
+      r = advance(dist, no_contact, P, lc, tally);
     } else {
-      const uint32_t a = P.edges[2 * pr.x], b = P.edges[2 * pr.x + 1];
-      const uint32_t c = P.edges[2 * pr.y], d = P.edges[2 * pr.y + 1];
-      const double3 pa = P.start[a], pb = P.start[b], ua = P.vel[a], ub = P.vel[b];
-      const double3 pc = P.start[c], pd = P.start[d], uc = P.vel[c], ud = P.vel[d];
-      const double lc = (fmax(P.speed[a], P.speed[b]) + fmax(P.speed[c], P.speed[d])) * kMargin;
-      auto dist = [&](double t) {
-        return segment_segment_distance(at3(pa, ua, t), at3(pb, ub, t), at3(pc, uc, t), at3(pd, ud, t));
+      const double3 pa = P.start[v[0]], pb = P.start[v[1]], ua = P.vel[v[0]], ub = P.vel[v[1]];
+      const double3 pc = P.start[v[2]], pd = P.start[v[3]], uc = P.vel[v[2]], ud = P.vel[v[3]];
+      auto dist = [&](double at) {
+        return segment_segment_distance(at3(pa, ua, at), at3(pb, ub, at), at3(pc, uc, at), at3(pd, ud, at));
       };
-      r = advance(dist, lc, P.gap_abs, P.max_iterations, P.close_factor, P.lo, horizon(P), tally);
+      r = advance(dist, no_contact, P, lc, tally);
     }
     if (r >= 0.0) atomicMin(P.best, (unsigned long long)__double_as_longlong(r));
   }
+}
+
+template <bool FIRST>
+__global__ void __launch_bounds__(128) narrow_kernel(Params P, const __grid_constant__ PairsLeft L) {
+  Tally tally;
+  if (blockIdx.x < L.blocks[0]) narrow<0, FIRST>(P, L, blockIdx.x, tally);
+  else narrow<1, FIRST>(P, L, blockIdx.x - L.blocks[0], tally);
   flush_tally(P, tally);
 }
 
@@ -494,6 +715,9 @@ __global__ void __launch_bounds__(128) narrow_kernel(Params P, const uint2 *pair
 __global__ void reset_kernel(unsigned long long *best, unsigned long long *tally) {
   if (threadIdx.x == 0) *best = 0x7FF0000000000000ull;
   if (threadIdx.x < 5) tally[threadIdx.x] = 0;
+}
+__global__ void reset_survivors_kernel(unsigned *count) {
+  if (threadIdx.x < 3) count[threadIdx.x] = threadIdx.x == 2 ? 0x7f800000u : 0u;
 }
 
 inline unsigned blocks(long long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -504,9 +728,8 @@ struct TreeBufs {
   DevBuf<DBox> box, sbox;
   DevBuf<FBox> levels;
   DevBuf<uint32_t> key, key_sorted, idx, order;
-  DevBuf<int> lvl_off, lvl_len;
   std::vector<int> off, len;
-  void init(int n_, cudaStream_t s) {
+  void init(int n_) {
     n = n_;
     box.alloc(n), sbox.alloc(n), key.alloc(n), key_sorted.alloc(n), idx.alloc(n), order.alloc(n);
     off.clear(), len.clear();
@@ -517,12 +740,14 @@ struct TreeBufs {
       if (m <= 1) break;
       m = (m + 1) / 2;
     }
-    if (off.size() > 62) fail(RS_INTERNAL, "Internal", "ccd", "box tree deeper than 62 levels");
+    // a place of a level is below 2^26 (nodes of 8 elements, which are numbered by an int, three a face)
+    if (off.size() > (size_t)kMaxLevels || len[0] > (1 << 26)) fail(RS_INTERNAL, "Internal", "ccd", "box tree deeper than 62 levels");
     levels.alloc(total);
-    lvl_off.upload(off, s), lvl_len.upload(len, s);
   }
   Tree view() const {
-    return Tree{sbox.p, order.p, levels.p, lvl_off.p, lvl_len.p, n, (int)off.size(), 8};
+    Tree t{sbox.p, order.p, levels.p, n, (int)off.size(), {}, {}};
+    std::copy(off.begin(), off.end(), t.lvl_off), std::copy(len.begin(), len.end(), t.lvl_len);
+    return t;
   }
 };
 
@@ -544,6 +769,8 @@ struct rs_ccd {
   DevBuf<uint2> pairs;                // candidate pairs of a window (or of the band's walk)
   DevBuf<uint8_t> hit, core, band;    // the band: intersection flags per candidate, per vertex
   bool has_band = false;
+  DevBuf<uint2> left;            // the pairs a window advances in FP64
+  DevBuf<unsigned> left_count;
   DevBuf<unsigned char> cub_tmp;
   DevBuf<unsigned long long> scratch;  // best, 5 tally counters, overflow flag, band hits
   double last_seconds = 0.0;
@@ -620,7 +847,7 @@ Params make_params(rs_ccd *c, double gap_abs, double close_factor, int max_itera
                    double hi, const uint8_t *band) {
   Params P;
   P.start = c->start.p, P.vel = c->vel.p, P.speed = c->speed.p, P.faces = c->faces.p, P.edges = c->edges.p;
-  P.vbox = c->vbox.p, P.ebox = c->et.box.p, P.fbox = c->ft.box.p, P.band = band;
+  P.vbox = c->vbox.p, P.band = band;
   P.nv = c->nv, P.ne = c->ne, P.nf = c->nf, P.max_iterations = max_iterations;
   P.gap_abs = gap_abs, P.close_factor = close_factor, P.h = h, P.lo = lo, P.hi = hi;
   P.best = c->scratch.p, P.tally = c->scratch.p + 1;
@@ -703,7 +930,7 @@ int rs_ccd_create(rs_ctx *ctx, int nv, int nf, const uint32_t *faces, rs_ccd **o
     c->edges.upload(c->edges_h, s);
     c->start.alloc(nv), c->vel.alloc(nv), c->speed.alloc(nv), c->vbox.alloc(nv);
     c->core.alloc(nv), c->band.alloc(nv);
-    c->ft.init(nf, s), c->et.init(c->ne, s);
+    c->ft.init(nf), c->et.init(c->ne);
     size_t t1 = 0, t2 = 0, t3 = 0;
     RSG_CUDA("ccd", cub::DeviceRadixSort::SortPairs(nullptr, t1, c->ft.key.p, c->ft.key_sorted.p, c->ft.idx.p,
                                                     c->ft.order.p, nf, 0, 30, s));
@@ -713,6 +940,7 @@ int rs_ccd_create(rs_ctx *ctx, int nv, int nf, const uint32_t *faces, rs_ccd **o
     c->pairs.alloc((size_t)8 * (nv + c->ne));  // grown on demand
     c->cub_tmp.alloc(std::max<size_t>(std::max(std::max(t1, t2), t3), 16));
     c->scratch.alloc(8);
+    c->left_count.alloc(3);
     RSG_CUDA("ccd", cudaStreamSynchronize(s));
     ctx_retain(ctx);
     *out = c.release();
@@ -851,14 +1079,30 @@ int rs_ccd_first_contact(rs_ccd *c, const double *start, const double *velocity,
       int64_t exempt_w = 0;
       const unsigned long long n_vt = collect<0>(c, P, c->ft.view(), nv, 0, false, s, &exempt_w);
       const unsigned long long n_ee = collect<1>(c, P, c->et.view(), c->ne, n_vt, true, s, &exempt_w);
-      // narrow phase, one thread per candidate pair
-      if (n_vt) {
-        narrow_kernel<0><<<blocks((long long)n_vt, 128), 128, 0, s>>>(P, c->pairs.p, n_vt);
-        RSG_LAUNCHED(ctx, "ccd vertex-triangle");
-      }
-      if (n_ee) {
-        narrow_kernel<1><<<blocks((long long)n_ee, 128), 128, 0, s>>>(P, c->pairs.p + n_vt, n_ee);
-        RSG_LAUNCHED(ctx, "ccd edge-edge");
+      // narrow phase, in slices whose places fit 32 bits
+      constexpr unsigned long long kSlice = 1ull << 30;
+      for (unsigned long long at = 0; at < std::max(n_vt, n_ee); at += kSlice) {
+        const unsigned vt = at < n_vt ? (unsigned)std::min(kSlice, n_vt - at) : 0u;
+        const unsigned ee = at < n_ee ? (unsigned)std::min(kSlice, n_ee - at) : 0u;
+        const uint2 *pv = c->pairs.p + at, *pe = c->pairs.p + n_vt + at;
+        if (c->left.n < (size_t)vt + ee) c->left.alloc(((size_t)vt + ee) * 5 / 4 + 1024);
+        const Survivors sv{c->left.p, c->left_count.p}, se{c->left.p + vt, c->left_count.p};
+        reset_survivors_kernel<<<1, 32, 0, s>>>(c->left_count.p);
+        RSG_LAUNCHED(ctx, "ccd reset");
+        if (vt) {
+          filter_kernel<0><<<blocks(vt, 128), 128, 0, s>>>(P, pv, vt, sv);
+          RSG_LAUNCHED(ctx, "ccd filter");
+        }
+        if (ee) {
+          filter_kernel<1><<<blocks(ee, 128), 128, 0, s>>>(P, pe, ee, se);
+          RSG_LAUNCHED(ctx, "ccd filter");
+        }
+        const unsigned wave = 4u * (unsigned)ctx->sm_count;
+        const PairsLeft L{{pv, pe}, {sv, se}, {std::min(wave, blocks(vt, 128)), std::min(wave, blocks(ee, 128))}};
+        narrow_kernel<true><<<L.blocks[0] + L.blocks[1], 128, 0, s>>>(P, L);
+        RSG_LAUNCHED(ctx, "ccd advancement");
+        narrow_kernel<false><<<L.blocks[0] + L.blocks[1], 128, 0, s>>>(P, L);
+        RSG_LAUNCHED(ctx, "ccd advancement");
       }
       unsigned long long res[8];
       c->scratch.download(res, 8, s);
