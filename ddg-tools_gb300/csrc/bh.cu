@@ -23,6 +23,7 @@
 
 #include "bh_kernels.cuh"
 #include "common.hpp"
+#include "f32x2.cuh"
 #include "fp64_bits.cuh"
 #include "host_tree.hpp"
 #include "profile.hpp"
@@ -471,32 +472,56 @@ __global__ void offsets_from_sorted(const uint32_t *key, uint32_t n, uint32_t m,
 
 // ------------------------------------------------------------------ the pair kernel
 
-// Error-free product and sum (Dekker/Knuth with FMA): a*b = p + e, a+b = s + t exactly.
-__device__ __forceinline__ void two_prod(float a, float b, float &p, float &e) {
-  p = a * b;
-  e = fmaf(a, b, -p);
-}
+// Error-free sum (Knuth): a + b = s + t exactly.
 __device__ __forceinline__ void two_sum(float a, float b, float &s, float &t) {
   s = a + b;
   float bv = s - a;
   t = (a - (s - bv)) + (b - bv);
 }
 
+// Packed FP32: two sources at once. The contractions of these and of the pair terms below are fixed:
+// the energies of earlier builds keep their bits.
+__device__ __forceinline__ f32x2 f2_neg(f32x2 a) { return a ^ kF2Sign; }
+__device__ __forceinline__ void two_sum2(f32x2 a, f32x2 b, f32x2 &s, f32x2 &t) {
+  s = f2_add(a, b);
+  const f32x2 bv = f2_sub(s, a);
+  t = f2_add(f2_sub(a, f2_sub(s, bv)), f2_sub(b, bv));
+}
+template <bool SECOND = false>  // the product that is rounded alone: the first or the second
+__device__ __forceinline__ f32x2 dot3x2(f32x2 a, f32x2 x, f32x2 b, f32x2 y, f32x2 c, f32x2 z) {
+  return f2_fma(c, z, SECOND ? f2_fma(a, x, f2_mul(b, y)) : f2_fma(b, y, f2_mul(a, x)));
+}
 // N . o for a unit normal and an offset both held as float pairs (hi + lo), compensated
 // (the Dot2 scheme of Ogita, Rump and Oishi, 2005): the sum of the three products carries its
 // rounding errors, which matters because it nearly cancels for a smooth surface.
 // The result is left unrounded as u + lo.
-__device__ __forceinline__ void dot2(float nx, float ny, float nz, float lx, float ly, float lz,
-                                     float ox, float oy, float oz, float px, float py, float pz,
-                                     float &u, float &lo) {
-  float p0, e0, p1, e1, p2, e2, s, t0, t1;
-  two_prod(nx, ox, p0, e0);
-  two_prod(ny, oy, p1, e1);
-  two_prod(nz, oz, p2, e2);
-  two_sum(p0, p1, s, t0);
-  two_sum(s, p2, u, t1);
-  lo = ((e0 + e1) + (e2 + t0)) + t1;
-  lo += (nx * px + ny * py + nz * pz) + (lx * ox + ly * oy + lz * oz);
+__device__ __forceinline__ void dot2x2(const f32x2 (&n)[3], const f32x2 (&l)[3], const f32x2 (&o)[3], const f32x2 (&p)[3],
+                                       f32x2 &u, f32x2 &lo) {
+  f32x2 q[3], e[3], s, t0, t1;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) q[k] = f2_mul(n[k], o[k]), e[k] = f2_fma(n[k], o[k], f2_neg(q[k]));
+  two_sum2(q[0], q[1], s, t0);
+  two_sum2(s, q[2], u, t1);
+  lo = f2_add(f2_add(f2_add(e[0], e[1]), f2_add(e[2], t0)), t1);
+  lo = f2_add(lo, f2_add(dot3x2(n[0], p[0], n[1], p[1], n[2], p[2]), dot3x2(l[0], o[0], l[1], o[1], l[2], o[2])));
+}
+// K and c_n of two sources; gg = beta K / r^2
+template <bool FAST>
+__device__ __forceinline__ void kernel_k2(const Pow &pw, f32x2 nu, f32x2 r2, f32x2 &K, f32x2 &cn, f32x2 &gg) {
+  const float2 r = f2_unpack(r2);
+  const f32x2 ir2 = f2_pack(__fdividef(1.f, r.x), __fdividef(1.f, r.y));
+  if constexpr (FAST) {
+    const f32x2 q = f2_mul(f2_mul(nu, nu), ir2), q2 = f2_mul(q, q), i3 = f2_mul(f2_mul(ir2, ir2), ir2);
+    const f32x2 t = f2_mul(q2, i3);
+    K = f2_mul(t, q);
+    cn = f2_mul(f2_mul(f2_mul(f2_dup(6.f), nu), t), ir2);
+  } else {
+    const float2 n = f2_unpack(nu), i = f2_unpack(ir2);
+    float k0, k1, c0, c1;
+    kernel_k<false>(pw, n.x, r.x, i.x, k0, c0), kernel_k<false>(pw, n.y, r.y, i.y, k1, c1);
+    K = f2_pack(k0, k1), cn = f2_pack(c0, c1);
+  }
+  gg = f2_mul(f2_mul(f2_dup(pw.beta), K), ir2);
 }
 
 // X_L - X_C from two centroids held as float pairs, as a float pair (h + l) per axis.
@@ -511,13 +536,21 @@ __device__ __forceinline__ void pair_diff(const float4 &ah, const float4 &al, co
   l[2] = t2 + (al.z - bl.z);
 }
 
-// Per-warp staging of the pair kernel in shared memory (one batch of up to kBatch sources).
 constexpr int kBatch = 64;
+// the float of component c of source e in src
+__device__ __forceinline__ int src_at(int e, int G, float rG, int c) {
+  const int i = (int)(((float)e + 0.5f) * rG);  // e / G: exact for these sizes
+  return ((c >> 1) * (kBatch / 2) + (i >> 1) * G + (e - i * G)) * 4 + (c & 1) * 2 + (i & 1);
+}
+
+// Per-warp staging of the pair kernel in shared memory (one batch of up to kBatch sources).
 struct PairStage {
   // lumped: per node entry, X_L - X_C rounded to FP32 (xyz) and A_C (w);
   // exact: per source face T, y_T = X_T - X_L as a float pair: hi (xyz) with a_T (w), lo (xyz)
   // with T's slot in the target leaf when C = L, else -1 (w, integer bits)
-  float4 src_hi[kBatch], src_lo[kBatch];
+  // (hi xyzw, lo xyzw), two sources e and e + G of a group side by side: plane p of pair
+  // (e / G / 2) G + e % G holds components 2 p and 2 p + 1 of both
+  float4 src[4][kBatch / 2];
   uint32_t src_slot[kBatch];            // exact: partner slot of each staged face
   float4 ent_h[32], ent_l[32];          // exact: X_L - X_C of each entry as a float pair
   uint32_t ent_cs[32], ent_po[32], ent_first[32];
@@ -545,12 +578,17 @@ struct PairStage {
 // product, and v = X_S - X_T is summed with its rounding error (leaf offsets can be large next
 // to |v| in a stretched leaf). alpha_S = N_S.(X_S - X_L) is a float pair from the FP64 refit.
 //
+// Bound by instruction issue (80 % of the slots, FMA pipe 50 %, with a source at a time), so a lane
+// evaluates its sources g + G i and g + G (i + 1) together in packed FP32, from records that lie side by
+// side; only the sums, whose order is kept, take them one by one. Value alone at 640,000 faces
+// 5.15 to 4.64 ms, with the differential at 81,920 faces 0.745 to 0.714 ms.
+//
 // COOP: a block's four warps share a work item, a batch each in turn (every warp finds the
 // batches by itself); the batches' sums go through shared memory and are added in batch order, two of
 // the eight accumulators per warp, so the result is the same bits. For meshes of few items,
 // whose time is that of one item: 1,280 faces 55 us with a warp per item.
 template <bool GRAD, bool FAST, bool COOP>
-__global__ void __launch_bounds__(128, COOP ? 4 : 6) bh_pair_kernel(BhDev d, Pow pw) {
+__global__ void __launch_bounds__(128, 4) bh_pair_kernel(BhDev d, Pow pw) {
   __shared__ PairStage stage[4];
   __shared__ float sums[COOP ? 2 : 1][COOP ? 4 : 1][COOP ? 8 : 1][32];
   __shared__ unsigned int next;
@@ -584,7 +622,15 @@ __global__ void __launch_bounds__(128, COOP ? 4 : 6) bh_pair_kernel(BhDev d, Pow
     const float4 nL = act ? d.fnl[s0 + s] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 xsl = act ? d.fol[s0 + s] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 cLh = d.nch[leaf], cLl = d.ncl[leaf];
-    const float a_s = xs.w;
+    const float a_s = xs.w, rG = 1.f / (float)G;
+    float *const src = reinterpret_cast<float *>(st.src);
+    const f32x2 Xh[3] = {f2_dup(xs.x), f2_dup(xs.y), f2_dup(xs.z)}, Xl[3] = {f2_dup(xsl.x), f2_dup(xsl.y), f2_dup(xsl.z)};
+    const f32x2 Nh[3] = {f2_dup(nS.x), f2_dup(nS.y), f2_dup(nS.z)}, Nl[3] = {f2_dup(nL.x), f2_dup(nL.y), f2_dup(nL.z)};
+    const f32x2 ah = f2_dup(nL.w), al = f2_dup(xsl.w);
+    // the differential's direction of one component, c_n N - gg v
+    auto dv2 = [&](f32x2 cn, f32x2 n, f32x2 gg, f32x2 v) {
+      return f2_fma(cn, n, f2_neg(f2_mul(gg, v)));
+    };
     // energy, d_a, d_x, d_n (COOP: the warp's two of them)
     Kahan acc[COOP ? 2 : 8];
     // adds the sums v of a batch, of which all but d_a's are still to be multiplied by f when SCALE;
@@ -623,33 +669,48 @@ __global__ void __launch_bounds__(128, COOP ? 4 : 6) bh_pair_kernel(BhDev d, Pow
         const float4 ch = d.nch[c], cl = d.ncl[c];
         float h[3], l[3];
         pair_diff(cLh, cLl, ch, cl, h, l);
-        st.src_hi[e] = make_float4(h[0] + l[0], h[1] + l[1], h[2] + l[2], ch.w);
+        const int at = src_at(e, G, rG, 0);  // components 0 and 1, then 2 and 3 in the next plane
+        src[at] = h[0] + l[0], src[at + 2] = h[1] + l[1];
+        src[at + 2 * kBatch] = h[2] + l[2], src[at + 2 * kBatch + 2] = ch.w;
       }
       __syncwarp();
       float bda = 0.f, be = 0.f, bx0 = 0.f, bx1 = 0.f, bx2 = 0.f, bn0 = 0.f, bn1 = 0.f, bn2 = 0.f;
 #pragma unroll 2
-      for (int i = 0; i < 8; ++i) {
-        const int e = g + G * i;
+      for (int i = 0; i < 4; ++i) {  // sources e and e + G
+        const int e = g + 2 * G * i;
         if (!act || e >= cnt) continue;
-        const float4 nd = st.src_hi[e];
-        const float v0 = xs.x + nd.x, v1 = xs.y + nd.y, v2 = xs.z + nd.z;
-        const float u = fmaf(nS.z, nd.z, fmaf(nS.y, nd.y, nS.x * nd.x));
-        const float nu = nL.w + (u + xsl.w);
-        const float r2 = v0 * v0 + v1 * v1 + v2 * v2;
-        const float ir2 = __fdividef(1.f, r2);
-        float K, cn;
-        kernel_k<FAST>(pw, nu, r2, ir2, K, cn);
-        const float Ac = nd.w;
-        be += a_s * K * Ac;
+        const bool both = e + G < cnt;
+        const ulonglong2 s0_ = reinterpret_cast<const ulonglong2 *>(st.src[0])[i * G + g];
+        const ulonglong2 s1_ = reinterpret_cast<const ulonglong2 *>(st.src[1])[i * G + g];
+        const f32x2 nd[3] = {s0_.x, s0_.y, s1_.x}, Ac = s1_.y;
+        f32x2 v[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[k] = f2_add(Xh[k], nd[k]);
+        const f32x2 u = f2_fma(Nh[2], nd[2], f2_fma(Nh[1], nd[1], f2_mul(Nh[0], nd[0])));
+        const f32x2 nu = f2_add(ah, f2_add(u, al));
+        const f32x2 r2 = dot3x2<true>(v[0], v[0], v[1], v[1], v[2], v[2]);
+        f32x2 K, cn, gg;
+        kernel_k2<FAST>(pw, nu, r2, K, cn, gg);
+        const f32x2 A = f2_dup(a_s), aK = f2_mul(A, K);
+        const float2 aK_ = f2_unpack(aK), Ac_ = f2_unpack(Ac);
+        be = __fmaf_rn(aK_.x, Ac_.x, be);
+        if (both) be = __fmaf_rn(aK_.y, Ac_.y, be);
         if (GRAD) {
-          const float gg = pw.beta * K * ir2;
-          const float dv0 = cn * nS.x - gg * v0, dv1 = cn * nS.y - gg * v1, dv2 = cn * nS.z - gg * v2;
-          bda += K * Ac;
-          const float aa = a_s * Ac;
-          bx0 += aa * dv0, bx1 += aa * dv1, bx2 += aa * dv2;
-          const float ac = aa * cn;
-          bn0 += ac * v0, bn1 += ac * v1, bn2 += ac * v2;
-          st.red[s * RS + e] = make_float4(a_s * K, -a_s * dv0, -a_s * dv1, -a_s * dv2);
+          const f32x2 aa = f2_mul(A, Ac), ac = f2_mul(aa, cn);
+          float2 d[3], w[3];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) d[k] = f2_unpack(dv2(cn, Nh[k], gg, v[k])), w[k] = f2_unpack(v[k]);
+          const float2 K_ = f2_unpack(K), aa_ = f2_unpack(aa), ac_ = f2_unpack(ac);
+          bda = __fmaf_rn(K_.x, Ac_.x, bda);
+          bx0 = __fmaf_rn(aa_.x, d[0].x, bx0), bx1 = __fmaf_rn(aa_.x, d[1].x, bx1), bx2 = __fmaf_rn(aa_.x, d[2].x, bx2);
+          bn0 = __fmaf_rn(ac_.x, w[0].x, bn0), bn1 = __fmaf_rn(ac_.x, w[1].x, bn1), bn2 = __fmaf_rn(ac_.x, w[2].x, bn2);
+          st.red[s * RS + e] = make_float4(aK_.x, -a_s * d[0].x, -a_s * d[1].x, -a_s * d[2].x);
+          if (both) {
+            bda = __fmaf_rn(K_.y, Ac_.y, bda);
+            bx0 = __fmaf_rn(aa_.y, d[0].y, bx0), bx1 = __fmaf_rn(aa_.y, d[1].y, bx1), bx2 = __fmaf_rn(aa_.y, d[2].y, bx2);
+            bn0 = __fmaf_rn(ac_.y, w[0].y, bn0), bn1 = __fmaf_rn(ac_.y, w[1].y, bn1), bn2 = __fmaf_rn(ac_.y, w[2].y, bn2);
+            st.red[s * RS + e + G] = make_float4(aK_.y, -a_s * d[0].y, -a_s * d[1].y, -a_s * d[2].y);
+          }
         }
       }
       const float bs[8] = {be, bda, bx0, bx1, bx2, bn0, bn1, bn2};
@@ -710,45 +771,68 @@ __global__ void __launch_bounds__(128, COOP ? 4 : 6) bh_pair_kernel(BhDev d, Pow
           two_sum(xt.x, -hh.x, y0, e0);
           two_sum(xt.y, -hh.y, y1, e1);
           two_sum(xt.z, -hh.z, y2, e2);
-          st.src_hi[f] = make_float4(y0, y1, y2, xt.w);
-          st.src_lo[f] = make_float4(e0 + (xl.x - ll.x), e1 + (xl.y - ll.y), e2 + (xl.z - ll.z),
-                                     __int_as_float(__float_as_int(ll.w) ? (int)t : -1));
+          const int at = src_at(f, G, rG, 0);  // a plane per two components
+          src[at] = y0, src[at + 2] = y1;
+          src[at + 2 * kBatch] = y2, src[at + 2 * kBatch + 2] = xt.w;
+          src[at + 4 * kBatch] = e0 + (xl.x - ll.x), src[at + 4 * kBatch + 2] = e1 + (xl.y - ll.y);
+          src[at + 6 * kBatch] = e2 + (xl.z - ll.z);
+          src[at + 6 * kBatch + 2] = __int_as_float(__float_as_int(ll.w) ? (int)t : -1);
           st.src_slot[f] = st.ent_po[i] + t;
         }
         __syncwarp();
         float row = 0.f, rx0 = 0.f, rx1 = 0.f, rx2 = 0.f, rn0 = 0.f, rn1 = 0.f, rn2 = 0.f;
 #pragma unroll 2
-        for (int i = 0; i < 8; ++i) {
-          const int f = g + G * i;
+        for (int i = 0; i < 4; ++i) {  // sources f and f + G
+          const int f = g + 2 * G * i;
           if (!act || f >= cnt) continue;
-          const float4 yh = st.src_hi[f], yl = st.src_lo[f];
-          const float a_t = yh.w;
-          float K = 0.f, cn = 0.f, gg = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f;
-          if (__float_as_int(yl.w) != s) {
-            float w0, w1, w2, e0, e1, e2;
-            two_sum(xs.x, -yh.x, w0, e0);
-            two_sum(xs.y, -yh.y, w1, e1);
-            two_sum(xs.z, -yh.z, w2, e2);
-            v0 = w0 + (e0 + (xsl.x - yl.x));
-            v1 = w1 + (e1 + (xsl.y - yl.y));
-            v2 = w2 + (e2 + (xsl.z - yl.z));
-            const float r2 = v0 * v0 + v1 * v1 + v2 * v2;
-            const float ir2 = __fdividef(1.f, r2);
-            float ph, pl, sh, se;
-            dot2(nS.x, nS.y, nS.z, nL.x, nL.y, nL.z, yh.x, yh.y, yh.z, yl.x, yl.y, yl.z, ph, pl);
-            two_sum(nL.w, -ph, sh, se);
-            const float nu = sh + (se + (xsl.w - pl));
-            kernel_k<FAST>(pw, nu, r2, ir2, K, cn);
-            gg = pw.beta * K * ir2;
+          const bool both = f + G < cnt;
+          ulonglong2 sp[4];
+#pragma unroll
+          for (int p = 0; p < 4; ++p) sp[p] = reinterpret_cast<const ulonglong2 *>(st.src[p])[i * G + g];
+          const f32x2 yh[3] = {sp[0].x, sp[0].y, sp[1].x}, yl[3] = {sp[2].x, sp[2].y, sp[3].x}, at2 = sp[1].y;
+          f32x2 v[3];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            f32x2 w, e;
+            two_sum2(Xh[k], f2_neg(yh[k]), w, e);
+            v[k] = f2_add(w, f2_add(e, f2_sub(Xl[k], yl[k])));
           }
-          row += a_t * K;
+          const f32x2 r2 = dot3x2(v[0], v[0], v[1], v[1], v[2], v[2]);
+          f32x2 ph, pl, sh, se, K, cn, gg;
+          dot2x2(Nh, Nl, yh, yl, ph, pl);
+          two_sum2(ah, f2_neg(ph), sh, se);
+          const f32x2 nu = f2_add(sh, f2_add(se, f2_sub(al, pl)));
+          kernel_k2<FAST>(pw, nu, r2, K, cn, gg);
+          // the face itself: no terms
+          const float2 slot = f2_unpack(sp[3].y);
+          if (__float_as_int(slot.x) == s) {
+            const unsigned long long m = 0xffffffff00000000ull;
+            K &= m, cn &= m, gg &= m, v[0] &= m, v[1] &= m, v[2] &= m;
+          }
+          if (__float_as_int(slot.y) == s) {
+            const unsigned long long m = 0x00000000ffffffffull;
+            K &= m, cn &= m, gg &= m, v[0] &= m, v[1] &= m, v[2] &= m;
+          }
+          const float2 a_ = f2_unpack(at2), K_ = f2_unpack(K);
+          row = __fmaf_rn(a_.x, K_.x, row);
+          if (both) row = __fmaf_rn(a_.y, K_.y, row);
           if (GRAD) {
-            const float dv0 = cn * nS.x - gg * v0, dv1 = cn * nS.y - gg * v1, dv2 = cn * nS.z - gg * v2;
-            rx0 += a_t * dv0, rx1 += a_t * dv1, rx2 += a_t * dv2;
-            const float tc = a_t * cn;
-            rn0 += tc * v0, rn1 += tc * v1, rn2 += tc * v2;
-            const float aa = -a_s * a_t;
-            st.red[s * RS + f] = make_float4(a_s * K, aa * dv0, aa * dv1, aa * dv2);
+            const f32x2 aa = f2_mul(f2_dup(-a_s), at2), tc = f2_mul(at2, cn);
+            float2 d[3], w[3], b[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+              const f32x2 dk = dv2(cn, Nh[k], gg, v[k]);
+              d[k] = f2_unpack(dk), w[k] = f2_unpack(v[k]), b[k] = f2_unpack(f2_mul(aa, dk));
+            }
+            const float2 tc_ = f2_unpack(tc), aK = f2_unpack(f2_mul(f2_dup(a_s), K));
+            rx0 = __fmaf_rn(a_.x, d[0].x, rx0), rx1 = __fmaf_rn(a_.x, d[1].x, rx1), rx2 = __fmaf_rn(a_.x, d[2].x, rx2);
+            rn0 = __fmaf_rn(tc_.x, w[0].x, rn0), rn1 = __fmaf_rn(tc_.x, w[1].x, rn1), rn2 = __fmaf_rn(tc_.x, w[2].x, rn2);
+            st.red[s * RS + f] = make_float4(aK.x, b[0].x, b[1].x, b[2].x);
+            if (both) {
+              rx0 = __fmaf_rn(a_.y, d[0].y, rx0), rx1 = __fmaf_rn(a_.y, d[1].y, rx1), rx2 = __fmaf_rn(a_.y, d[2].y, rx2);
+              rn0 = __fmaf_rn(tc_.y, w[0].y, rn0), rn1 = __fmaf_rn(tc_.y, w[1].y, rn1), rn2 = __fmaf_rn(tc_.y, w[2].y, rn2);
+              st.red[s * RS + f + G] = make_float4(aK.y, b[0].y, b[1].y, b[2].y);
+            }
           }
         }
         const float rs[8] = {row, row, rx0, rx1, rx2, rn0, rn1, rn2};

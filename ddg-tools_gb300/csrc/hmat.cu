@@ -35,6 +35,7 @@
 
 #include "block_tree.hpp"
 #include "common.hpp"
+#include "f32x2.cuh"
 #include "fp64_bits.cuh"
 #include "host_tree.hpp"
 #include "hmat.hpp"
@@ -94,40 +95,6 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &t) {
   t = (a - (s - bv)) + (b - bv);
 }
 
-// Two FP32 values in one 64-bit register (first in the low half) and the packed FP32 pair
-// arithmetic of sm_100 and later (each half rounded to nearest, as the scalar operations).
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 f2_pack(float a, float b) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 f2_unpack(f32x2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-constexpr f32x2 kF2Sign = 0x8000000080000000ull;  // both halves' sign bits
 
 // v as a float pair: hi = v rounded to FP32, lo = the rest rounded
 __device__ __forceinline__ float2 to_pair(double v) {
