@@ -5,9 +5,10 @@
 // Per step:   host BVH build (host_tree.cpp) -> device list build (lists_count/lists_fill,
 //             radix-sorted transposes).
 // Per energy: refit (FP64 face geometry + bottom-up node aggregates, packs FP32 offsets)
-//             -> bh_pair (the pair kernel, warp per target leaf)
+//             -> bh_pair (the pair kernel, warp per work item of a target leaf)
 //             -> node_sums -> downward (per-leaf chain walk) -> final (own + partner +
-//             cluster) -> pull_back (per-vertex gather) -> energy reduction (FP64).
+//             cluster, per face, and its FP64 corner terms) -> pull_back (per-vertex
+//             gather) -> energy reduction (FP64).
 // Every reduction has a fixed order (gathers over the transposed lists, fixed shuffle
 // trees), so results are bitwise reproducible run to run.
 #include <cub/device/device_radix_sort.cuh>

@@ -11,9 +11,10 @@
 //   2. a box tree per primitive kind, as the reference builds it: boxes sorted along a Morton
 //      curve of their centres, blocks of 8 united, blocks merged pairwise up to one root;
 //   3. one thread per query (a vertex against the face tree, an edge against the edge tree)
-//      walks the tree and runs the narrow phase on every element whose own box overlaps the
-//      query box (so the candidate pairs are exactly those of the reference, whatever the
-//      tree's shape), keeping the earliest contact in one global atomic minimum.
+//      walks the tree and lists every element whose own box overlaps the query box (so the
+//      candidate pairs are exactly those of the reference, whatever the tree's shape);
+//   4. a filter drops the pairs that cannot meet before the horizon, the others are advanced,
+//      keeping the earliest contact in one global atomic minimum.
 // A pair's contact time does not depend on the horizon it is given (see advance()), so the
 // global minimum used as horizon only skips pairs that cannot lower the result.
 #include <cub/cub.cuh>
@@ -328,12 +329,12 @@ __device__ __forceinline__ bool query(const Tree &t, bool mine, const DBox &q, i
   __syncthreads();
   if (!mine) return true;
   const FBox qf = outward(q);
-  uint32_t stack[kStack];  // overlapping nodes: the level above 26 bits of place
+  int2 stack[kStack];  // overlapping nodes: level, place
   int sp = 0;
-  if (overlaps_f(load_box(t.levels + off[t.n_levels - 1]), qf)) stack[sp++] = (uint32_t)(t.n_levels - 1) << 26;
+  if (overlaps_f(load_box(t.levels + off[t.n_levels - 1]), qf)) stack[sp++] = make_int2(t.n_levels - 1, 0);
   while (sp > 0) {
-    const uint32_t e = stack[--sp];
-    const int l = (int)(e >> 26), at = (int)(e & 0x3ffffffu);
+    const int2 e = stack[--sp];
+    const int l = e.x, at = e.y;
     if (l == 0) {
       const int end = min((at + 1) * kLeaf, t.n);
 #pragma unroll 4
@@ -345,9 +346,8 @@ __device__ __forceinline__ bool query(const Tree &t, bool mine, const DBox &q, i
       const bool two = 2 * at + 1 < len[l - 1];
       const bool one = ((long long)(2 * at + 1) * kLeaf << (l - 1)) > from;  // reaches past `from`
       const FBox c0 = load_box(one ? c : c + 1), c1 = load_box(two ? c + 1 : c);
-      const uint32_t e0 = (uint32_t)(l - 1) << 26 | (uint32_t)(2 * at);
-      if (one && overlaps_f(c0, qf)) stack[sp++] = e0;
-      if (two && overlaps_f(c1, qf)) stack[sp++] = e0 + 1;
+      if (one && overlaps_f(c0, qf)) stack[sp++] = make_int2(l - 1, 2 * at);
+      if (two && overlaps_f(c1, qf)) stack[sp++] = make_int2(l - 1, 2 * at + 1);
     }
   }
   return true;
@@ -740,8 +740,7 @@ struct TreeBufs {
       if (m <= 1) break;
       m = (m + 1) / 2;
     }
-    // a place of a level is below 2^26 (nodes of 8 elements, which are numbered by an int, three a face)
-    if (off.size() > (size_t)kMaxLevels || len[0] > (1 << 26)) fail(RS_INTERNAL, "Internal", "ccd", "box tree deeper than 62 levels");
+    if (off.size() > (size_t)kMaxLevels) fail(RS_INTERNAL, "Internal", "ccd", "box tree deeper than 62 levels");
     levels.alloc(total);
   }
   Tree view() const {

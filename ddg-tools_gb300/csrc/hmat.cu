@@ -4,10 +4,8 @@
 // behind rs_metric_* / rs_vfrac_* of include/rsgpu.h.
 //
 // Both are kernel-matrix forms L u = 2 M^T diag(a) (diag(H~a) M u - H~(a M u)) with a block
-// cluster tree H~: rank-one far blocks (cluster data) and exact near blocks. The near entries
-// are NOT stored: every product evaluates them from the element records (FP32 offsets from the
-// leaf centroid, normals) while it streams the columns, which costs less than reading a stored
-// near field from HBM (0.3 G entries x 2 kernels at 204,800 faces).
+// cluster tree H~: rank-one far blocks (cluster data) and exact near blocks, whose FP32 weights are
+// evaluated once per set-up and streamed by every product.
 //
 // Per product (C channels per element: 9 gradient + 3 average per input vector for faces, 3
 // per vector for vertices):
