@@ -719,9 +719,9 @@ def bench_ccd(args, rank, world, local):
                 "d2h_bytes_per_step": 64 * int(r["windows"])},
         "pairs_per_s": r["pairs_tested"] * value, "evaluations_per_s": r["evaluations"] * value,
         "roofline": None,
-        "roofline_note": ("the narrow phase (64 % of the GPU time) is bound by the FP64 pipe, ~70 % active "
-                          "where it runs (ncu, profiles/ccd_first_contact.md); no FP64 peak is measured "
-                          "on this pool, so no fraction is reported"),
+        "roofline_note": ("bound by latency: the longest chain of FP64 distances of a pair (41 % of the GPU "
+                          "time) and the tree walks (41 %) (profiles/ccd_first_contact.md); no FP64 peak is "
+                          "measured, so no fraction is reported"),
         "gpu_launches": launches,
         "clocks": clk.summary(),
     }
