@@ -929,8 +929,7 @@ __global__ void node_sums_kernel(BhDev d) {
 
 // Downward pass per leaf along its root -> leaf chain (barnes_hut.rs:521-538), in FP64 (about
 // 20 steps per leaf, each record fetched four steps ahead): beta_c = beta_p + U_p.(X_c - X_p) + b_c, U_c = U_p + u_c.
-__global__ void downward_kernel(BhDev d) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void downward(const BhDev &d, int k) {
   if (k >= d.n_leaves) return;
   uint32_t c0 = d.chain_off[k], c1 = d.chain_off[k + 1];
   uint32_t p = d.chain[c0];
@@ -967,8 +966,7 @@ __global__ void downward_kernel(BhDev d) {
 // over the chunk's entries, each summing the leaf's (<= 8) partner slots of an entry into
 // 8 x 4 registers; a transposing reduce over the 32 lanes leaves lane 4 t + c with component c
 // of face t, written to the chunk's 32 partial sums.
-__global__ void final_partial_kernel(BhDev d) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ void final_partial(const BhDev &d, int w) {
   const int lane = threadIdx.x & 31;
   if (w >= d.n_fchunks) return;
   const uint4 ch = d.fchunk[w];
@@ -1007,6 +1005,14 @@ __global__ void final_partial_kernel(BhDev d) {
   for (int i = 0; i < 2; ++i)
     r2[i] = (b1 ? r4[2 + i] : r4[i]) + __shfl_xor_sync(0xffffffffu, b1 ? r4[i] : r4[2 + i], 2);
   d.fpart[32 * (size_t)w + lane] = (b0 ? r2[1] : r2[0]) + __shfl_xor_sync(0xffffffffu, b0 ? r2[0] : r2[1], 1);
+}
+
+// Both, which do not depend on one another: the first blocks walk the chains (bound by FP64 and the records'
+// latency on few warps: 14 us at 1,280 faces), the others sum the partners (17 us).
+constexpr int kWalkThreads = 128;
+__global__ void __launch_bounds__(kWalkThreads) walks_kernel(BhDev d, unsigned n_down) {
+  if (blockIdx.x < n_down) downward(d, (int)(blockIdx.x * kWalkThreads + threadIdx.x));
+  else final_partial(d, (int)(((blockIdx.x - n_down) * kWalkThreads + threadIdx.x) >> 5));
 }
 
 // Per face: own + partner (the leaf's chunks in order) + cluster part (barnes_hut.rs:539-567), written
@@ -1635,13 +1641,12 @@ void evaluate(rs_bh *h, const Pow &pw, bool fast, bool grad, double *energy_dev,
     node_sums_kernel<<<blocks(nn, 256), 256, 0, s>>>(d);
     RSG_LAUNCHED(h->ctx, "node_sums");
     P.end(s);
-    P.begin(s, "downward");
-    downward_kernel<<<blocks(nl, 128), 128, 0, s>>>(d);
+    P.begin(s, "downward_and_partners");
+    const unsigned n_down = blocks(nl, kWalkThreads);
+    walks_kernel<<<n_down + blocks((size_t)h->n_fchunks * 32, kWalkThreads), kWalkThreads, 0, s>>>(d, n_down);
     RSG_LAUNCHED(h->ctx, "downward");
     P.end(s);
     P.begin(s, "final");
-    final_partial_kernel<<<blocks((size_t)h->n_fchunks * 32, 256), 256, 0, s>>>(d);
-    RSG_LAUNCHED(h->ctx, "final");
     if (dE_dev) final_kernel<true><<<blocks(h->nf, 128), 128, 0, s>>>(d, h->pos.p, h->corner.p);
     else final_kernel<false><<<blocks(h->nf, 128), 128, 0, s>>>(d, h->pos.p, nullptr);
     RSG_LAUNCHED(h->ctx, "final");
