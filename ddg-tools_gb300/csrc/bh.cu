@@ -1007,12 +1007,52 @@ __device__ __forceinline__ void final_partial(const BhDev &d, int w) {
   d.fpart[32 * (size_t)w + lane] = (b0 ? r2[1] : r2[0]) + __shfl_xor_sync(0xffffffffu, b0 ? r2[0] : r2[1], 1);
 }
 
-// Both, which do not depend on one another: the first blocks walk the chains (bound by FP64 and the records'
-// latency on few warps: 14 us at 1,280 faces), the others sum the partners (17 us).
+// Energy over the work items in FP64: 1024 strided partial sums over eight blocks, then a fixed tree in the
+// last of them to finish (a ticket that it resets). One block of 1024 threads is bound by its SM's FP64
+// rate: 21 us at 81,920 faces, 172 at 640,000.
 constexpr int kWalkThreads = 128;
-__global__ void __launch_bounds__(kWalkThreads) walks_kernel(BhDev d, unsigned n_down) {
-  if (blockIdx.x < n_down) downward(d, (int)(blockIdx.x * kWalkThreads + threadIdx.x));
-  else final_partial(d, (int)(((blockIdx.x - n_down) * kWalkThreads + threadIdx.x) >> 5));
+constexpr unsigned kEnergyBlocks = 1024 / kWalkThreads;
+__device__ __forceinline__ void energy_sum(const BhDev &d, unsigned block, double *out) {
+  __shared__ double sh[1024];
+  __shared__ bool last;
+  const double *__restrict__ e = d.item_energy;
+  const int n = d.n_items, t0 = (int)(block * kWalkThreads + threadIdx.x);
+  double acc = 0.0;
+  int i = t0;
+  for (; i + 7 * 1024 < n; i += 8 * 1024) {
+    double v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = e[i + 1024 * j];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc += v[j];
+  }
+  for (; i < n; i += 1024) acc += e[i];
+  d.energy_part[t0] = acc;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(d.energy_ticket, 1u) == kEnergyBlocks - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+#pragma unroll
+  for (int j = 0; j < 1024 / kWalkThreads; ++j) sh[j * kWalkThreads + threadIdx.x] = __ldcg(d.energy_part + j * kWalkThreads + threadIdx.x);
+  for (int m = 512; m > 0; m >>= 1) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < m; t += kWalkThreads) sh[t] += sh[t + m];
+  }
+  if (threadIdx.x == 0) *out = sh[0], *d.energy_ticket = 0u;
+}
+
+// Three passes that do not depend on one another: the first blocks add up the energy, the next walk the chains (bound by FP64 and the records'
+// latency on few warps: 14 us at 1,280 faces), the others sum the partners (17 us).
+__global__ void __launch_bounds__(kWalkThreads) walks_kernel(BhDev d, unsigned n_down, double *energy) {
+  if (blockIdx.x < kEnergyBlocks) {
+    energy_sum(d, blockIdx.x, energy);
+    return;
+  }
+  const unsigned b = blockIdx.x - kEnergyBlocks;
+  if (b < n_down) downward(d, (int)(b * kWalkThreads + threadIdx.x));
+  else final_partial(d, (int)(((b - n_down) * kWalkThreads + threadIdx.x) >> 5));
 }
 
 // Per face: own + partner (the leaf's chunks in order) + cluster part (barnes_hut.rs:539-567), written
@@ -1096,46 +1136,8 @@ __global__ void pull_back_kernel(BhDev d, const double *__restrict__ corner, dou
   dE[3 * (size_t)v] = g0, dE[3 * (size_t)v + 1] = g1, dE[3 * (size_t)v + 2] = g2;
 }
 
-// Energy over the work items in FP64: 1024 strided partial sums over a cluster of eight blocks, then a
-// fixed tree in the first (one block of 1024 threads is bound by its SM's FP64 rate: 21 us at 81,920 faces,
-// 172 at 640,000).
-constexpr int kEnergyBlocks = 8, kEnergyThreads = 1024 / kEnergyBlocks;
-__global__ void __cluster_dims__(kEnergyBlocks) __launch_bounds__(kEnergyThreads)
-    energy_reduce_kernel(const double *leaf_energy, int n, double *out) {
-  __shared__ double part[kEnergyThreads], sh[1024];
-  double acc = 0.0;
-  int i = (int)(blockIdx.x * kEnergyThreads + threadIdx.x);
-  for (; i + 7 * 1024 < n; i += 8 * 1024) {
-    double v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = leaf_energy[i + 1024 * j];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc += v[j];
-  }
-  for (; i < n; i += 1024) acc += leaf_energy[i];
-  part[threadIdx.x] = acc;
-  auto barrier = [] {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  };
-  barrier();
-  if (blockIdx.x == 0) {
-    const unsigned own = (unsigned)__cvta_generic_to_shared(part + threadIdx.x);
-#pragma unroll
-    for (int b = 0; b < kEnergyBlocks; ++b) {
-      unsigned at;
-      double v;
-      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(own), "r"(b));
-      asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(at) : "memory");
-      sh[b * kEnergyThreads + threadIdx.x] = v;
-    }
-    for (int m = 512; m > 0; m >>= 1) {
-      __syncthreads();
-      for (int t = threadIdx.x; t < m; t += kEnergyThreads) sh[t] += sh[t + m];
-    }
-    if (threadIdx.x == 0) *out = sh[0];
-  }
-  barrier();  // no block leaves while the first may read its shared memory
-}
+// The energy alone (the value path).
+__global__ void __launch_bounds__(kWalkThreads) energy_reduce_kernel(BhDev d, double *out) { energy_sum(d, blockIdx.x, out); }
 
 // First exact pair in leaf, list, s, t order whose FP32 term is non-finite (culprit_pair,
 // barnes_hut.rs:693-724): the smallest (entry << 8 | s << 4 | t) rank.
@@ -1206,7 +1208,8 @@ struct rs_bh {
   DevBuf<uint4> climb;
   DevBuf<float4> nch, ncl;
   DevBuf<uint32_t> refit_count;
-  DevBuf<double> item_energy, energy, dE, corner;
+  DevBuf<double> item_energy, energy, energy_part, dE, corner;
+  DevBuf<unsigned> energy_ticket;
   DevBuf<unsigned int> ticket;
   DevBuf<unsigned long long> culprit_key;
   bool positions_current = false;
@@ -1229,7 +1232,7 @@ struct rs_bh {
     d.n_vertices = nv, d.n_faces = nf, d.n_nodes = (int)tree.n_nodes();
     d.n_leaves = (int)tree.leaves.size();
     d.fxa = fxa.p, d.fnn = fnn.p, d.ncA = ncA.p, d.nmom = nmom.p, d.refit_count = refit_count.p;
-    d.climb = climb.p;
+    d.climb = climb.p, d.energy_part = energy_part.p, d.energy_ticket = energy_ticket.p;
     d.nch = nch.p, d.ncl = ncl.p;
     d.own = own.p, d.node_term = node_term.p, d.partner = partner.p, d.node_sum = node_sum.p;
     d.leaf_bu = leaf_bu.p, d.partials = partials.p, d.item_energy = item_energy.p;
@@ -1371,6 +1374,8 @@ void upload_topology(rs_bh *h) {
   RSG_CUDA("upload", cudaMemsetAsync(h->refit_count.p, 0, nn * sizeof(uint32_t), s));
   h->leaf_bu.alloc(nl);
   h->energy.alloc(1);
+  h->energy_part.alloc(1024), h->energy_ticket.alloc(1);
+  RSG_CUDA("upload", cudaMemsetAsync(h->energy_ticket.p, 0, sizeof(unsigned), s));
   h->dE.alloc(3 * (size_t)h->nv);
   h->pos.alloc(3 * (size_t)h->nv);
   h->ticket.alloc(1);
@@ -1641,9 +1646,10 @@ void evaluate(rs_bh *h, const Pow &pw, bool fast, bool grad, double *energy_dev,
     node_sums_kernel<<<blocks(nn, 256), 256, 0, s>>>(d);
     RSG_LAUNCHED(h->ctx, "node_sums");
     P.end(s);
-    P.begin(s, "downward_and_partners");
+    P.begin(s, "downward_partners_energy");
     const unsigned n_down = blocks(nl, kWalkThreads);
-    walks_kernel<<<n_down + blocks((size_t)h->n_fchunks * 32, kWalkThreads), kWalkThreads, 0, s>>>(d, n_down);
+    const unsigned n_sums = blocks((size_t)h->n_fchunks * 32, kWalkThreads);
+    walks_kernel<<<kEnergyBlocks + n_down + n_sums, kWalkThreads, 0, s>>>(d, n_down, energy_dev);
     RSG_LAUNCHED(h->ctx, "downward");
     P.end(s);
     P.begin(s, "final");
@@ -1658,10 +1664,12 @@ void evaluate(rs_bh *h, const Pow &pw, bool fast, bool grad, double *energy_dev,
       P.end(s);
     }
   }
-  P.begin(s, "energy_reduce");
-  energy_reduce_kernel<<<kEnergyBlocks, kEnergyThreads, 0, s>>>(h->item_energy.p, (int)h->n_items, energy_dev);
-  RSG_LAUNCHED(h->ctx, "energy_reduce");
-  P.end(s);
+  if (!grad) {
+    P.begin(s, "energy_reduce");
+    energy_reduce_kernel<<<kEnergyBlocks, kWalkThreads, 0, s>>>(d, energy_dev);
+    RSG_LAUNCHED(h->ctx, "energy_reduce");
+    P.end(s);
+  }
 }
 
 void find_culprit(rs_bh *h, const Pow &pw, bool fast) {

@@ -66,6 +66,8 @@ struct BhDev {
   float4 *leaf_bu;   // per leaf: (beta, U) of the downward pass
   float4 *partials;  // 2 per face (by face id): (d_a, d_x), (d_n, 0)
   double *item_energy;
+  double *energy_part;           // 1024 partial sums of the energy, and the ticket of their blocks
+  unsigned int *energy_ticket;
   unsigned int *ticket;
 };
 
