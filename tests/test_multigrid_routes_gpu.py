@@ -37,3 +37,30 @@ def test_columns_do_not_depend_on_the_batch(ctx, mesh, vcycles):
     for nb in (2, 3, 4):
         assert np.array_equal(S.precondition(r[:nb]), one[:nb]), nb
     assert np.array_equal(S.precondition(r), S.precondition(r))
+
+
+@pytest.mark.parametrize("mesh", [(66, 66), (140, 100)])
+def test_two_threads_solve_at_once(mesh):
+    """Two contexts, a thread each: their solves (each a kernel whose blocks wait for one another) run beside
+    one another on the device and give what they give alone."""
+    import threading
+
+    P, F = gen.noisy_torus(*mesh, 1.0, 0.35, 0.002, 5)
+    S = [R.SaddleSolver(F, P, R.Exponents(), R.solver_options(), R.Context(0)) for _ in range(2)]
+    r = np.random.default_rng(9).standard_normal((3, S[0].n))
+    r[:, S[0].n_dofs:] = 0.0
+    want = {nb: S[0].precondition(r[:nb]) for nb in (1, 3)}
+    bad = []
+
+    def work(i):
+        for k in range(40):
+            nb = 1 if (i + k) % 2 else 3
+            if not np.array_equal(S[i].precondition(r[:nb]), want[nb]):
+                bad.append((i, k))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
