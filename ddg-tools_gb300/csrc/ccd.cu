@@ -53,17 +53,21 @@ __device__ __forceinline__ double clamp01(double x) {
   return x;
 }
 
-__device__ double point_segment_distance(double3 p, double3 a, double3 b) {  // RC/src/ccd.rs:237-247
+// The distances of RC/src/ccd.rs:237-319. The correctly rounded square root does not decrease, so the least of
+// several distances is the root of the least square, bit for bit: one root (a long chain of FP64 instructions)
+// instead of three to five.
+__device__ double point_segment_square(double3 p, double3 a, double3 b) {  // RC/src/ccd.rs:237-247
   const double3 ab = sub3(b, a), ap = sub3(p, a);
   const double e = dot3(ab, ab);
   const double t = e > 0.0 ? clamp01(dot3(ap, ab) / e) : 0.0;
-  return norm3(sub3(ap, scale3(ab, t)));
+  const double3 d = sub3(ap, scale3(ab, t));
+  return dot3(d, d);
 }
 
 __device__ double segment_segment_distance(double3 p1, double3 q1, double3 p2, double3 q2) {  // ccd.rs:266-291
-  double best = fmin(fmin(fmin(point_segment_distance(p1, p2, q2), point_segment_distance(q1, p2, q2)),
-                          point_segment_distance(p2, p1, q1)),
-                     point_segment_distance(q2, p1, q1));
+  double best = fmin(fmin(fmin(point_segment_square(p1, p2, q2), point_segment_square(q1, p2, q2)),
+                          point_segment_square(p2, p1, q1)),
+                     point_segment_square(q2, p1, q1));
   const double3 d1 = sub3(q1, p1), d2 = sub3(q2, p2);
   const double a = dot3(d1, d1), e = dot3(d2, d2);
   const double3 n = cross3(d1, d2);
@@ -74,14 +78,15 @@ __device__ double segment_segment_distance(double3 p1, double3 q1, double3 p2, d
     double s = clamp01(dot3(cross3(sub3(p2, p1), d2), n) / nn);
     const double t = clamp01((b * s + f) / e);
     s = clamp01((b * t - c) / a);
-    best = fmin(best, norm3(sub3(add3(p1, scale3(d1, s)), add3(p2, scale3(d2, t)))));
+    const double3 d = sub3(add3(p1, scale3(d1, s)), add3(p2, scale3(d2, t)));
+    best = fmin(best, dot3(d, d));
   }
-  return best;
+  return sqrt(best);
 }
 
 __device__ double point_triangle_distance(double3 p, double3 a, double3 b, double3 c) {  // ccd.rs:298-319
   const double edges =
-      fmin(fmin(point_segment_distance(p, a, b), point_segment_distance(p, b, c)), point_segment_distance(p, c, a));
+      sqrt(fmin(fmin(point_segment_square(p, a, b), point_segment_square(p, b, c)), point_segment_square(p, c, a)));
   const double3 ab = sub3(b, a), ac = sub3(c, a);
   const double3 n = cross3(ab, ac);
   const double nn = dot3(n, n);
