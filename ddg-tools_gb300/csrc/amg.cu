@@ -295,8 +295,8 @@ __global__ void __launch_bounds__(kMaxThreads<C, CLUSTER>, 1) pcg_kernel(const _
     if (l == 0) {
       o = (unsigned)j / (unsigned)(kDotBlocks / kCluster * chunk), r0 = o * (kDotBlocks / kCluster * chunk);
     } else {
-      o = (unsigned)j * kCluster / n;
-      if ((unsigned long long)n * (o + 1) / kCluster <= (unsigned)j) ++o;
+      // the last block that begins at row j or before (below 16 rows some blocks own none)
+      o = (kCluster * ((unsigned)j + 1) - 1) / n;
       r0 = (unsigned)((unsigned long long)n * o / kCluster);
     }
     unsigned a;
