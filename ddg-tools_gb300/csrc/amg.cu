@@ -32,7 +32,6 @@ namespace {
 constexpr int kDotBlocks = 304;  // fixed split of the column dot products (deterministic)
 constexpr int kMaxLevels = 12;
 constexpr int kCluster = 16;     // blocks of a solve in one cluster
-constexpr unsigned kBarrierPolls = 1u << 22;  // about two seconds
 
 // floats from row to row of a vector of C columns
 template <int C>
@@ -59,6 +58,7 @@ struct CgArgs {
   double *part;                 // kDotBlocks x C partial sums, two sets used in turn
   unsigned long long *counter;  // arrivals at the grid barrier, a multiple of the grid between solves
   int *error;                   // set when a barrier gave up
+  unsigned polls;               // after this many
   int smem_bytes;
 };
 
@@ -140,6 +140,7 @@ template <bool CLUSTER>
 struct SolveBarrier {
   unsigned long long *counter;
   int *error;
+  unsigned polls_max;
   unsigned long long target;  // the count that ends the next barrier (thread 0)
   bool dead = false;
   __device__ __forceinline__ void sync() {
@@ -156,7 +157,7 @@ struct SolveBarrier {
       while (!dead) {
         asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(counter) : "memory");
         if (v >= target) break;
-        if (++polls >= kBarrierPolls || ((polls & 4095u) == 0u && *(volatile int *)error)) {
+        if (++polls >= polls_max || ((polls & 4095u) == 0u && *(volatile int *)error)) {
           *(volatile int *)error = 1;
           dead = true;
         }
@@ -365,7 +366,7 @@ __global__ void __launch_bounds__(kMaxThreads<C, CLUSTER>, 1) pcg_kernel(const _
   }
   // the counter stands at a multiple of the grid plus the blocks that arrived already, at most all
   // but this one
-  SolveBarrier<CLUSTER> bar{A.counter, A.error, 0ull};
+  SolveBarrier<CLUSTER> bar{A.counter, A.error, A.polls, 0ull};
   if (!CLUSTER) bar.target = (*(volatile unsigned long long *)A.counter / gridDim.x + 1) * gridDim.x;
 
   // out = x + dinv (b - A x)
@@ -746,8 +747,10 @@ cudaLaunchConfig_t AmgDevice::cluster_config(cudaStream_t s, cudaLaunchAttribute
   return cfg;
 }
 
-void AmgDevice::check() const {
-  if (error && *(volatile int *)error) fail(RS_GPU, "Gpu", "preconditioner", "a multigrid solve gave up waiting for its blocks");
+void AmgDevice::check() {
+  if (!error || *(volatile int *)error == 0) return;
+  *(volatile int *)error = 0;  // every block still arrived at every barrier: the next solve starts clean
+  fail(RS_GPU, "Gpu", "preconditioner", "a multigrid solve gave up waiting for its blocks");
 }
 
 template <int C>
@@ -761,7 +764,7 @@ void AmgDevice::launch(rs_ctx *ctx, const mgreal *b, mgreal *x, int iters) {
   }
   A.cinv = cinv.p, A.rhs = b, A.sol = x;
   A.p = cg_p.p, A.q = cg_q.p, A.part = cg_part.p, A.counter = counter.p;
-  A.error = error_dev, A.smem_bytes = smem_bytes;
+  A.error = error_dev, A.polls = wait_polls, A.smem_bytes = smem_bytes;
   if (C == 3 && cluster_smem > 0) {
     A.smem_bytes = cluster_smem;
     cudaLaunchAttribute at;

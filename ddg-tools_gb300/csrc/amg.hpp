@@ -64,8 +64,10 @@ struct AmgDevice {
   // scalars stay on the device (no host synchronization); a fixed number of steps makes it a
   // nonlinear map of b, which flexible GMRES (the stored preconditioned vectors) allows.
   void pcg(rs_ctx *ctx, const mgreal *b, mgreal *x, int C, int iters);
-  // fails when an earlier solve gave up at a barrier (to be called once the stream has been waited for)
-  void check() const;
+  // Fails when an earlier solve gave up at a barrier, once for every such report (to be called when the stream
+  // has been waited for; pcg calls it too, for the solves that nothing waited for).
+  void check();
+  unsigned wait_polls = 1u << 22;  // a wait across the grid gives up after that many polls (about two seconds)
   AmgDevice() = default;
   AmgDevice(const AmgDevice &) = delete;
   AmgDevice &operator=(const AmgDevice &) = delete;

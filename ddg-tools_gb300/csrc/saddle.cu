@@ -497,15 +497,25 @@ struct rs_solver {
   }
 
   // GMRES with the learned preconditioner when one is set (capped at l_cap iterations), the
-  // plain preconditioner otherwise or when the learned solve does not converge
+  // plain preconditioner otherwise or when the learned solve does not converge. A multigrid solve that
+  // gave up waiting fails the call it belongs to, whatever became of the GMRES around it.
   void solve(int nb, const double *b, double *x, const GmresOptions &o) {
+    auto run = [&](const Operator *P, const GmresOptions &go) {
+      try {
+        gmres_batch(ctx, inner_plain ? op_inner : op, P, nb, b, x, go, last, inner_plain ? &op : nullptr);
+      } catch (const Error &) {
+        amg.check();
+        throw;
+      }
+      amg.check();
+    };
     if (lmodel && use_prec) {
       GmresOptions ol = o;
       if (l_cap > 0) ol.max_iterations = l_cap;
       l_solves++;
       bool ok = true;
       try {
-        gmres_batch(ctx, inner_plain ? op_inner : op, &lprec, nb, b, x, ol, last, inner_plain ? &op : nullptr);
+        run(&lprec, ol);
         for (auto &r : last) ok = ok && r.converged;
       } catch (const Error &e) {
         if (e.code != RS_SOLVER_DIVERGED) throw;
@@ -514,9 +524,7 @@ struct rs_solver {
       if (ok) return;
       l_fallbacks++;
     }
-    gmres_batch(ctx, inner_plain ? op_inner : op, use_prec ? &prec : nullptr, nb, b, x, o, last,
-                inner_plain ? &op : nullptr);
-    amg.check();
+    run(use_prec ? &prec : nullptr, o);
   }
 };
 

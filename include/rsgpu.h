@@ -287,7 +287,9 @@ int rs_solver_profile(rs_solver *s, int nb, const double *rhs_host, char *names,
 /* LinearOperator::apply_batch (gmres.rs:32-52): ys = A' xs for nb stacked vectors. */
 int rs_solver_apply(rs_solver *s, int nb, const double *xs_host, double *ys_host);
 int rs_solver_apply_device(rs_solver *s, int nb, const double *xs_dev, double *ys_dev);
-/* Preconditioner::apply_batch (gmres.rs:55-75): zs = P^-1 rs. */
+/* Preconditioner::apply_batch (gmres.rs:55-75): zs = P^-1 rs. The device form does not wait for its work:
+ * should a multigrid solve in it give up waiting for its blocks (a wait is bounded, about two seconds), zs is
+ * meaningless and the next call on the solver that applies the preconditioner fails with RS_GPU. */
 int rs_solver_precondition(rs_solver *s, int nb, const double *rs_host, double *zs_host);
 int rs_solver_precondition_device(rs_solver *s, int nb, const double *rs_dev, double *zs_dev);
 /* SaddleSolver::solve_many (RS/src/solve/mod.rs:107-130): right-preconditioned GMRES on the
