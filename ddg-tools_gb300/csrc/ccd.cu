@@ -497,7 +497,10 @@ __global__ void count_flags_kernel(int n, const uint8_t *flag, unsigned long lon
 //   weaker. The relative positions carry 4 2^-24 M per component (M: the largest component until the
 //   horizon), a projection 25 2^-24 M between two elements, and u is at most 2^-21 too long:
 //   2^-19 M and a factor 1 - 2^-20 are taken off, and 2^-44 of the positions for the FP64 distance's own
-//   rounding. The FP64 point-plane distance loses digits on slivers: those go to FP64 at once.
+//   rounding.
+// * The FP64 point-plane distance loses digits on slivers: with edges at an angle of 2^-16 or more it is within
+//   2^-30 M of the distance. The iterates it is taken at are not the bound's, so a triangle whose angle is
+//   not known to stay above that on the whole way to the next iterate goes to FP64 (keeps_shape).
 // * The bound advanced as the reference's distance is, t <- t + (bound - gap) / l, rounded down. By
 //   induction each iterate is at most the reference's: the distance changes by at most l dt, and
 //   the margin is above its slack of 1e-9 d. So when an iterate passes the horizon within as many steps as the
@@ -544,9 +547,7 @@ __device__ __forceinline__ float triangle_bound(const F3 (&r)[3]) {
   w = foot(r[0], ac);
   if (dot(w, w) < dot(v, v)) v = w;
   const F3 n = cross(ab, ac);
-  const float nn = dot(n, n), ee = dot(ab, ab) * dot(ac, ac);
-  if (!(ee > 0x1p-110f && nn > 0x1p-30f * ee)) return __int_as_float(0x7fffffff);  // a sliver
-  const float i = __fdividef(1.f, nn), s = -dot(cross(r[0], ac), n) * i, t = -dot(cross(ab, r[0]), n) * i;
+  const float i = __fdividef(1.f, dot(n, n)), s = -dot(cross(r[0], ac), n) * i, t = -dot(cross(ab, r[0]), n) * i;
   if (s >= 0.f && t >= 0.f && s + t <= 1.f) v = (dot(r[0], n) * i) * n;
   return separation<0>(r, v);
 }
@@ -582,7 +583,7 @@ __device__ __forceinline__ void pair_vertices(const Params &P, uint2 pr, uint32_
 template <int KIND>
 struct NarrowPair {
   F3 x[3], w[3];
-  float il, err;
+  float il, err, reach;
   __device__ __forceinline__ void load(const Params &P, const uint32_t (&v)[4], double l, float hz) {
     const double3 p = P.start[v[0]], u = P.vel[v[0]];
     float M = 0.f, W = 0.f;
@@ -592,7 +593,9 @@ struct NarrowPair {
       M = fmaxf(M, largest(x[k])), W = fmaxf(W, largest(w[k]));
     }
     il = __fdiv_rd(1.f, __double2float_ru(l));
-    err = 0x1p-19f * (M + hz * W) + 0x1p-43f * (largest(p) + M + hz * (largest(u) + W));
+    const float far = largest(p) + M + hz * (largest(u) + W);
+    err = 0x1p-19f * (M + hz * W) + 0x1p-43f * far;
+    reach = M + hz * W + 0x1p-32f * far;
   }
   __device__ __forceinline__ float bound(float t) const {
     F3 r[3];
@@ -600,13 +603,28 @@ struct NarrowPair {
     for (int k = 0; k < 3; ++k) r[k] = x[k] + t * w[k];
     return (1.f - 0x1p-20f) * (KIND == 0 ? triangle_bound(r) : segment_bound(r)) - err;
   }
+  // Whether the edges ab and ac of the triangle keep an angle of 2^-16 on [t, s]: the normal n(t + u) = n + u n1 +
+  // u^2 n2 has, along n, at least |n| + min(0, u n1.n / |n|) + min(0, u^2 n2.n / |n|). The edges carry an error of
+  // 2^-20 M, and in FP64 one of 2^-50 of the positions: these parts less than 2^-17 reach (|ab| + |ac|) in all;
+  // their own rounding is far below the 2^-16 |ab| |ac| that 2^-15 leaves.
+  __device__ __forceinline__ bool keeps_shape(float t, float s) const {
+    const float h = s - t;
+    const F3 da = w[1] - w[0], dc = w[2] - w[0];
+    const F3 ab = (x[1] + t * w[1]) - (x[0] + t * w[0]), ac = (x[2] + t * w[2]) - (x[0] + t * w[0]);
+    const F3 n = cross(ab, ac), eb = ab + h * da, ec = ac + h * dc;
+    const float nn = dot(n, n), n1 = h * dot(cross(ab, dc) + cross(da, ac), n), n2 = h * h * dot(cross(da, dc), n);
+    const float b = sqrtf(fmaxf(dot(ab, ab), dot(eb, eb))), c = sqrtf(fmaxf(dot(ac, ac), dot(ec, ec)));
+    return nn > 0x1p-110f && nn + fminf(n1, 0.f) + fminf(n2, 0.f) > sqrtf(nn) * (0x1p-15f * b * c + 0x1p-17f * reach * (b + c));
+  }
   // From t with the bound d towards `target`: true when an iterate passes hz within `steps`; else
   // t is the last iterate.
   __device__ __forceinline__ bool passes(float &t, float d, float target, float hz, int steps, Tally &tally) const {
     for (int it = 0; it < steps && d > target; ++it) {
       const float next = __fadd_rd(t, __fmul_rd(__fsub_rd(d, target), il));
-      if (next >= hz) return true;
-      if (!(next > t + 0x1p-18f * t)) break;
+      const bool past = next >= hz;
+      if (!past && !(next > t + 0x1p-18f * t)) break;
+      if (KIND == 0 && !keeps_shape(t, past ? hz : next)) break;
+      if (past) return true;
       t = next;
       d = bound(t);
       tally.evals += 1;
@@ -631,7 +649,7 @@ __global__ void __launch_bounds__(128) filter_kernel(Params P, const uint2 *pair
     q.load(P, v, l, hz);
     float d = q.bound(0.f);
     tally.evals += 1;
-    if (d > gap) {  // neither touching nor close at the start
+    if (d > gap && (KIND == 1 || P.lo == 0.0 || q.keeps_shape(0.f, 0.f))) {  // neither touching nor close at the start
       if (P.lo != 0.0) t = __double2float_rd(P.lo), d = q.bound(t);
       left = !q.passes(t, d, gap, hz, min(kFilterSteps, P.max_iterations), tally);
     }
