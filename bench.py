@@ -717,7 +717,9 @@ def bench_ccd(args, rank, world, local):
                    "parallelism": "replicas" if world > 1 else "single GPU"},
         "e2e": {"value": value, "unit": "calls/s", "h2d_bytes_per_step": int(P.nbytes + V.nbytes),
                 "d2h_bytes_per_step": 64 * int(r["windows"])},
+        # evaluations: FP64 distances and the FP32 bounds that decide most pairs, together
         "pairs_per_s": r["pairs_tested"] * value, "evaluations_per_s": r["evaluations"] * value,
+        "evaluations_of": "FP64 distances and FP32 bounds of distances",
         "roofline": None,
         "roofline_note": ("bound by latency: the longest chain of FP64 distances of a pair (41 % of the GPU "
                           "time) and the tree walks (41 %) (profiles/ccd_first_contact.md); no FP64 peak is "

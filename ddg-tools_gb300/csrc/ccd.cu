@@ -134,7 +134,7 @@ struct Params {
   int nv, ne, nf, max_iterations;
   double gap_abs, close_factor, h, lo, hi;
   unsigned long long *best;   // bits of the earliest contact time (+inf: none)
-  unsigned long long *tally;  // pairs, close, touching, evaluations, exempt
+  unsigned long long *tally;  // pairs, close, touching, evaluations (FP64 distances, FP32 bounds), exempt
   int *overflow;
 };
 

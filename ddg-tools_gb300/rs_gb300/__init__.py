@@ -831,7 +831,8 @@ def ccd_options(**kw) -> CcdOptions:
 class CcdSurface:
     """Continuous collision detection of one surface against itself (first_contact,
     RS/src/ccd.rs:762-884, without obstacles and without the exempt band): the topology lives
-    on the device, each ``first_contact`` call sweeps one linear motion."""
+    on the device, each ``first_contact`` call sweeps one linear motion. Its ``evaluations`` count FP64
+    distances and FP32 bounds of them together."""
 
     REPORT_KEYS = ["contact", "windows", "pairs_tested", "close_pairs", "touching_pairs", "exempt_pairs",
                    "evaluations"]

@@ -430,8 +430,9 @@ void rs_ccd_free(rs_ccd *c);
  * touching pairs unconstrained). With a band set (rs_ccd_set_band) a pair whose two elements
  * both have a vertex in the band is exempt (first_contact_with_band, ccd.rs:781-884). No
  * obstacles. tau_max is bitwise the crate's. report7 (may be NULL): contact found (0/1),
- * windows, candidate pairs tested, close pairs, touching pairs, exempt pairs, distance
- * evaluations (the last depends on the order pairs are met and is not the crate's count). */
+ * windows, candidate pairs tested, close pairs, touching pairs, exempt pairs, evaluations (the
+ * pairs' distances in FP64 and the lower bounds of them in FP32 that decide most pairs, together;
+ * the number depends on the order pairs are met and is not the crate's count). */
 int rs_ccd_first_contact(rs_ccd *c, const double *start, const double *velocity, double tau_end,
                          const rs_ccd_options *o, double *tau_max, int64_t *report7);
 /* IntersectionBand::new (ccd.rs:1292-1319) of `positions` (V x 3, host), kept for the following
