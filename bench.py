@@ -721,8 +721,8 @@ def bench_ccd(args, rank, world, local):
         "pairs_per_s": r["pairs_tested"] * value, "evaluations_per_s": r["evaluations"] * value,
         "evaluations_of": "FP64 distances and FP32 bounds of distances",
         "roofline": None,
-        "roofline_note": ("bound by latency: the longest chain of FP64 distances of a pair (41 % of the GPU "
-                          "time) and the tree walks (41 %) (profiles/ccd_first_contact.md); no FP64 peak is "
+        "roofline_note": ("bound by latency: the longest chain of FP64 distances of a pair (37 % of the GPU "
+                          "time) and the tree walks (44 %) (profiles/ccd_first_contact.md); no FP64 peak is "
                           "measured, so no fraction is reported"),
         "gpu_launches": launches,
         "clocks": clk.summary(),

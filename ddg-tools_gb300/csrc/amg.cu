@@ -679,7 +679,9 @@ void AmgDevice::upload(const AmgHost &h, cudaStream_t s) {
   // The blocks: one cluster of 16 when their shared memory holds all the matrices and vectors, else one
   // block per SM with the vectors in global memory, shared memory for the block's share of the
   // matrices with a tenth to spare for uneven rows. As many threads as the largest level gives lanes
-  // per block.
+  // per block. A preconditioner application on the grid, three vectors, with 256 threads / as many as the nine
+  // columns' registers allow: 8,000 rows 0.78 / 0.78 ms, 25,600 rows 1.29 / 1.17, 102,400 rows 2.54 / 2.28; in the
+  // cluster, one vector, with 256 / 512 / 1,024: 900 rows 0.43 / 0.43 / 0.43, 4,356 rows 0.73 / 0.65 / 0.62.
   int dev = 0, most = 0, sms = 0;
   RSG_CUDA("preconditioner", cudaGetDevice(&dev));
   RSG_CUDA("preconditioner", cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

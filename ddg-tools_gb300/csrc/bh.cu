@@ -1600,6 +1600,10 @@ void check_positions_host(rs_bh *h, const double *pos) {
         fail(RS_NONFINITE_POSITION, "NonFinitePosition", "energy", "vertex " + std::to_string(v));
 }
 
+// Work items per SM up to which four warps share an item. The pair kernel with the differential, a warp per
+// item / four, exponents (6, 12): 458 items (1,280 faces) 41 / 28 us, 1,119 items 56 / 43, 2,114 items 81 / 77, 3,089
+// items 96 / 109, 10,280 items 246 / 361; exponents (4.5, 9): 88 / 45, 123 / 79, 174 / 159, 218 / 242, 675 / 885. The
+// line, 608 items, lies well on the near side of the crossing at about 2,500.
 constexpr size_t kCoopItems = 4;
 using PairKernel = void (*)(BhDev, Pow);
 PairKernel pair_kernel(bool grad, bool fast, bool coop) {
