@@ -538,10 +538,10 @@ __device__ __forceinline__ void pair_diff(const float4 &ah, const float4 &al, co
 }
 
 constexpr int kBatch = 64;
-// the float of component c of source e in src
-__device__ __forceinline__ int src_at(int e, int G, float rG, int c) {
-  const int i = (int)(((float)e + 0.5f) * rG);  // e / G: exact for these sizes
-  return ((c >> 1) * (kBatch / 2) + (i >> 1) * G + (e - i * G)) * 4 + (c & 1) * 2 + (i & 1);
+// the first float of source e in src
+__device__ __forceinline__ int src_at(int e, int G) {
+  const int i = e / G;
+  return ((i >> 1) * G + (e - i * G)) * 4 + (i & 1);
 }
 
 // Per-warp staging of the pair kernel in shared memory (one batch of up to kBatch sources).
@@ -584,12 +584,18 @@ struct PairStage {
 // side; only the sums, whose order is kept, take them one by one. Value alone at 640,000 faces
 // 5.15 to 4.64 ms, with the differential at 81,920 faces 0.745 to 0.714 ms.
 //
+// General exponents (two powf a pair): unrolled over two pairs of sources, both loops outgrow the instruction
+// cache. At 204,800 faces and exponents (4.5, 9) / (3, 6), with the differential 8.13 / 5.48 ms unrolled and 5.25 /
+// 3.68 not (5.40 / 3.70 with a source at a time). The value alone has room for the lumped loop unrolled, and gains
+// from six blocks per SM: whole calls 4.53 / 2.53 ms with both loops unrolled and four blocks, 3.88 / 2.34 with five, 3.72 /
+// 2.24 with six (3.64 / 2.40 with a source at a time).
+//
 // COOP: a block's four warps share a work item, a batch each in turn (every warp finds the
 // batches by itself); the batches' sums go through shared memory and are added in batch order, two of
 // the eight accumulators per warp, so the result is the same bits. For meshes of few items,
 // whose time is that of one item: 1,280 faces 55 us with a warp per item.
 template <bool GRAD, bool FAST, bool COOP>
-__global__ void __launch_bounds__(128, 4) bh_pair_kernel(BhDev d, Pow pw) {
+__global__ void __launch_bounds__(128, FAST || GRAD || COOP ? 4 : 6) bh_pair_kernel(BhDev d, Pow pw) {
   __shared__ PairStage stage[4];
   __shared__ float sums[COOP ? 2 : 1][COOP ? 4 : 1][COOP ? 8 : 1][32];
   __shared__ unsigned int next;
@@ -623,7 +629,8 @@ __global__ void __launch_bounds__(128, 4) bh_pair_kernel(BhDev d, Pow pw) {
     const float4 nL = act ? d.fnl[s0 + s] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 xsl = act ? d.fol[s0 + s] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 cLh = d.nch[leaf], cLl = d.ncl[leaf];
-    const float a_s = xs.w, rG = 1.f / (float)G;
+    const float a_s = xs.w;
+    const int at0 = src_at(lane, G), at1 = src_at(lane + 32, G);  // a lane stages sources lane and lane + 32
     float *const src = reinterpret_cast<float *>(st.src);
     const f32x2 Xh[3] = {f2_dup(xs.x), f2_dup(xs.y), f2_dup(xs.z)}, Xl[3] = {f2_dup(xsl.x), f2_dup(xsl.y), f2_dup(xsl.z)};
     const f32x2 Nh[3] = {f2_dup(nS.x), f2_dup(nS.y), f2_dup(nS.z)}, Nl[3] = {f2_dup(nL.x), f2_dup(nL.y), f2_dup(nL.z)};
@@ -670,13 +677,13 @@ __global__ void __launch_bounds__(128, 4) bh_pair_kernel(BhDev d, Pow pw) {
         const float4 ch = d.nch[c], cl = d.ncl[c];
         float h[3], l[3];
         pair_diff(cLh, cLl, ch, cl, h, l);
-        const int at = src_at(e, G, rG, 0);  // components 0 and 1, then 2 and 3 in the next plane
+        const int at = e < 32 ? at0 : at1;  // components 0 and 1, then 2 and 3 in the next plane
         src[at] = h[0] + l[0], src[at + 2] = h[1] + l[1];
         src[at + 2 * kBatch] = h[2] + l[2], src[at + 2 * kBatch + 2] = ch.w;
       }
       __syncwarp();
       float bda = 0.f, be = 0.f, bx0 = 0.f, bx1 = 0.f, bx2 = 0.f, bn0 = 0.f, bn1 = 0.f, bn2 = 0.f;
-#pragma unroll 2
+#pragma unroll (FAST || !GRAD ? 2 : 1)
       for (int i = 0; i < 4; ++i) {  // sources e and e + G
         const int e = g + 2 * G * i;
         if (!act || e >= cnt) continue;
@@ -772,7 +779,7 @@ __global__ void __launch_bounds__(128, 4) bh_pair_kernel(BhDev d, Pow pw) {
           two_sum(xt.x, -hh.x, y0, e0);
           two_sum(xt.y, -hh.y, y1, e1);
           two_sum(xt.z, -hh.z, y2, e2);
-          const int at = src_at(f, G, rG, 0);  // a plane per two components
+          const int at = f < 32 ? at0 : at1;  // a plane per two components
           src[at] = y0, src[at + 2] = y1;
           src[at + 2 * kBatch] = y2, src[at + 2 * kBatch + 2] = xt.w;
           src[at + 4 * kBatch] = e0 + (xl.x - ll.x), src[at + 4 * kBatch + 2] = e1 + (xl.y - ll.y);
@@ -782,7 +789,7 @@ __global__ void __launch_bounds__(128, 4) bh_pair_kernel(BhDev d, Pow pw) {
         }
         __syncwarp();
         float row = 0.f, rx0 = 0.f, rx1 = 0.f, rx2 = 0.f, rn0 = 0.f, rn1 = 0.f, rn2 = 0.f;
-#pragma unroll 2
+#pragma unroll (FAST ? 2 : 1)
         for (int i = 0; i < 4; ++i) {  // sources f and f + G
           const int f = g + 2 * G * i;
           if (!act || f >= cnt) continue;
@@ -1267,6 +1274,7 @@ Pow make_pow(double alpha, double beta) {
   p.alpha = (float)alpha;
   p.beta = (float)beta;
   p.a_int = (alpha == std::trunc(alpha) && alpha >= 2 && alpha <= 64) ? (int)alpha : -1;
+  p.q_exp = 0.5f * p.alpha - 1.f, p.r_exp = 0.5f * (p.alpha - p.beta);
   double ab = beta - alpha;
   p.ab_int = (ab == std::trunc(ab) && ab >= 0 && ab <= 128) ? (int)ab : -1;
   return p;
