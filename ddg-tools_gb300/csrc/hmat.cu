@@ -979,9 +979,16 @@ __global__ void item_key_kernel(uint32_t n_items, const uint4 *__restrict__ item
   key[i] = ((end[leaf] - start[leaf]) << 16) | (0xffffu - (it.z - it.y));
   idx[i] = i;
 }
-// off[i] = the first of the sorted keys of more than i rows, i = 0 .. 8
-__global__ void sched_off_kernel(uint32_t n, const uint32_t *__restrict__ key, uint32_t *off) {
+// What the host needs of the work items: off[i] = the first of the sorted keys of more than i rows, i = 0 .. 8; the
+// weights' blocks and the near entries.
+struct ItemTotals {
+  unsigned long long weights, entries;
+  uint32_t off[9];
+};
+__global__ void item_totals_kernel(uint32_t n, const uint32_t *__restrict__ key, const unsigned long long *weights,
+                                   const unsigned long long *entries, ItemTotals *out) {
   const uint32_t i = threadIdx.x;
+  if (i == 9) out->weights = *weights, out->entries = *entries;
   if (i > 8) return;
   uint32_t a = 0, b = n;
   while (a < b) {
@@ -989,7 +996,7 @@ __global__ void sched_off_kernel(uint32_t n, const uint32_t *__restrict__ key, u
     if (key[c] >> 16 > i) b = c;
     else a = c + 1;
   }
-  off[i] = a;
+  out->off[i] = a;
 }
 __global__ void item_base_kernel(uint32_t n_items, const unsigned long long *__restrict__ base, uint4 *items) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1036,13 +1043,14 @@ struct HMat {
   double neg_s = 0;
   DevBuf<uint32_t> start, end, right, parent, leaves, chain_off, chain, item_off;
   DevBuf<uint32_t> far_item_off, leaf_of;
-  // the groups of the upward sums: the bottom ones, and the levels above (see hm_upward_kernel)
+  // the groups of the upward sums: the bottom ones, and the levels above (see hm_upward_kernel); the bottom
+  // ones' depths, then every level's ext, inner and child
   DevBuf<uint4> grp;
-  DevBuf<uint32_t> grp_depth;
+  DevBuf<uint32_t> grp_words;
+  size_t n_bottom = 0;
   struct Level {
-    DevBuf<uint4> groups;
-    DevBuf<uint32_t> ext, inner;
-    DevBuf<uint2> child;
+    size_t first, count;        // its groups
+    size_t ext, inner, child;  // its lists, in words
   };
   std::vector<Level> levels;
   // the far passes run on the context's second stream beside the near field
@@ -1086,7 +1094,7 @@ struct HMat {
     d.sched = sched.p;
     std::copy(sched_off, sched_off + 9, d.sched_off);
     d.up = up.p, d.up2 = up2.p, d.part = part.p, d.leafsum = leafsum.p;
-    d.leaf_of = leaf_of.p, d.grp = grp.p, d.grp_depth = grp_depth.p, d.n_grp = (int)grp.n;
+    d.leaf_of = leaf_of.p, d.grp = grp.p, d.grp_depth = grp_words.p, d.n_grp = (int)n_bottom;
     d.m = reinterpret_cast<const float *>(m.p), d.z = z.p;
     d.n_nodes = (int)tree.n_nodes(), d.n_leaves = (int)tree.leaves.size(), d.n_el = (int)n_el;
     d.n_items = (int)n_items;
@@ -1129,7 +1137,9 @@ struct HMat {
     hm_upward_kernel<SEL><<<dim3((unsigned)d.n_grp, gy), 192, 0, s>>>(d);
     RSG_LAUNCHED(ctx, "hm_upward");
     for (const Level &l : levels) {
-      hm_upward_level_kernel<CC><<<dim3((unsigned)l.groups.n, gy), 128, 0, s>>>(d, l.groups.p, l.ext.p, l.inner.p, l.child.p);
+      const uint32_t *w = grp_words.p;
+      hm_upward_level_kernel<CC><<<dim3((unsigned)l.count, gy), 128, 0, s>>>(d, grp.p + l.first, w + l.ext, w + l.inner,
+                                                                             reinterpret_cast<const uint2 *>(w + l.child));
       RSG_LAUNCHED(ctx, "hm_upward");
     }
     prof.end(s);
@@ -1143,16 +1153,14 @@ struct HMat {
     prof.end(s);
   }
 
-  // The groups of the upward sums (see hm_upward_kernel), from the tree.
-  void build_groups() {
+  // The groups of the upward sums (see hm_upward_kernel), from the tree: g, the groups (bottom, then level by
+  // level), and words, their depths and lists.
+  void build_groups(std::vector<uint4> &g, std::vector<uint32_t> &words) {
     const Tree &T = tree;
     const size_t nn = T.n_nodes();
-    cudaStream_t s = st();
     std::vector<uint32_t> size(nn, 1);
     for (size_t i = nn; i-- > 0;)
       if (T.right[i]) size[i] = 1 + size[i + 1] + size[T.right[i]];
-    std::vector<uint4> g;
-    std::vector<uint32_t> depth;
     // the nodes not yet inside a group in preorder, each with whether it is a root of one
     std::vector<std::pair<uint32_t, bool>> cur, next;
     std::vector<uint32_t> ends;  // ends of the subtrees of the current node's ancestors
@@ -1161,7 +1169,7 @@ struct HMat {
       if ((size[n] + 1) / 2 <= (uint32_t)kGrpLeaves) {
         const uint32_t nl = (size[n] + 1) / 2;
         g.push_back(make_uint4(n, size[n], k, nl));
-        depth.push_back((uint32_t)ends.size());
+        words.push_back((uint32_t)ends.size());
         cur.push_back({n, true});
         k += nl, n += size[n];
       } else {
@@ -1170,15 +1178,15 @@ struct HMat {
         ++n;
       }
     }
-    up_vec(grp, g, s), up_vec(grp_depth, depth, s);
+    n_bottom = g.size();
     levels.clear();
     while (cur.size() > 1) {
       const size_t m = cur.size();
       std::vector<uint32_t> roots(m + 1, 0);  // roots before each entry
       for (size_t i = 0; i < m; ++i) roots[i + 1] = roots[i] + (cur[i].second ? 1u : 0u);
-      std::vector<uint4> groups;
-      std::vector<uint32_t> ext, inner, slot(nn);
-      std::vector<uint2> child;
+      Level l;
+      l.first = g.size();
+      std::vector<uint32_t> ext, inner, child, slot(nn);
       next.clear();
       for (size_t i = 0; i < m;) {
         const uint32_t n = cur[i].first;
@@ -1194,20 +1202,23 @@ struct HMat {
           if (!cur[a].second) {
             const uint32_t v = cur[a].first;
             inner.push_back(v);
-            child.push_back(make_uint2(slot[v + 1], slot[T.right[v]]));
+            child.push_back(slot[v + 1]), child.push_back(slot[T.right[v]]);
             slot[v] = gr.y + gr.w++;
           }
-        groups.push_back(gr);
+        g.push_back(gr);
         next.push_back({n, true});
         i = j;
       }
-      levels.emplace_back();
-      Level &l = levels.back();
-      up_vec(l.groups, groups, s), up_vec(l.ext, ext, s), up_vec(l.inner, inner, s), up_vec(l.child, child, s);
-      RSG_CUDA("upload", cudaStreamSynchronize(s));  // before the staging vectors go
+      l.count = g.size() - l.first;
+      auto add = [&](const std::vector<uint32_t> &v) {
+        words.resize((words.size() + 1) & ~size_t(1));  // pairs lie on 8 bytes
+        words.insert(words.end(), v.begin(), v.end());
+        return words.size() - v.size();
+      };
+      l.ext = add(ext), l.inner = add(inner), l.child = add(child);
+      levels.push_back(l);
       cur.swap(next);
     }
-    RSG_CUDA("upload", cudaStreamSynchronize(s));
   }
 
   // Uploads the tree, the near column ranges split into work items, the element records and
@@ -1272,36 +1283,35 @@ struct HMat {
     lap(setup_times[0]);
     // weight base of every item
     {
-      DevBuf<unsigned long long> w(n_items + 1), base(n_items + 1), entries(1);
-      RSG_CUDA("upload", cudaMemsetAsync(w.p + n_items, 0, sizeof(unsigned long long), s));
-      RSG_CUDA("upload", cudaMemsetAsync(entries.p, 0, sizeof(unsigned long long), s));
+      DevBuf<unsigned long long> w(n_items + 2), base(n_items + 1);  // w: zero past the items, then the entries
+      unsigned long long *entries = w.p + n_items + 1;
+      RSG_CUDA("upload", cudaMemsetAsync(w.p + n_items, 0, 2 * sizeof(unsigned long long), s));
       if (kind == FACE)
         item_weights_kernel<FACE><<<nblk(n_items, 256), 256, 0, s>>>((uint32_t)n_items, items.p, leaves.p, start.p,
-                                                                     end.p, w.p, entries.p);
+                                                                     end.p, w.p, entries);
       else
         item_weights_kernel<VERTEX><<<nblk(n_items, 256), 256, 0, s>>>((uint32_t)n_items, items.p, leaves.p, start.p,
-                                                                       end.p, w.p, entries.p);
+                                                                       end.p, w.p, entries);
       RSG_LAUNCHED(ctx, "hm_item_weights");
       scan(w.p, base.p, n_items + 1);
-      DevBuf<uint32_t> key(2 * n_items), idx(n_items), off(9);
-      item_key_kernel<<<nblk(n_items, 256), 256, 0, s>>>((uint32_t)n_items, items.p, leaves.p, start.p, end.p, key.p,
-                                                          idx.p);
+      DevBuf<uint32_t> sort(3 * n_items);  // keys, sorted keys, items
+      uint32_t *key = sort.p, *sorted = key + n_items, *idx = sorted + n_items;
+      item_key_kernel<<<nblk(n_items, 256), 256, 0, s>>>((uint32_t)n_items, items.p, leaves.p, start.p, end.p, key, idx);
       RSG_LAUNCHED(ctx, "hm_item_key");
       sched.alloc(n_items);
       size_t bytes = 0;
-      RSG_CUDA("upload", cub::DeviceRadixSort::SortPairs(nullptr, bytes, key.p, key.p + n_items, idx.p, sched.p,
-                                                         (int)n_items, 0, 20, s));
+      RSG_CUDA("upload", cub::DeviceRadixSort::SortPairs(nullptr, bytes, key, sorted, idx, sched.p, (int)n_items, 0, 20, s));
       if (bytes > tmp.n) tmp.alloc(bytes);
-      RSG_CUDA("upload", cub::DeviceRadixSort::SortPairs(tmp.p, bytes, key.p, key.p + n_items, idx.p, sched.p,
-                                                         (int)n_items, 0, 20, s));
-      sched_off_kernel<<<1, 32, 0, s>>>((uint32_t)n_items, key.p + n_items, off.p);
-      RSG_LAUNCHED(ctx, "hm_sched_off");
-      off.download(sched_off, 9, s);
-      unsigned long long tot = 0, n_entries = 0;
-      RSG_CUDA("upload", copy_async(&tot, base.p + n_items, sizeof(tot), cudaMemcpyDeviceToHost, s));
-      RSG_CUDA("upload", copy_async(&n_entries, entries.p, sizeof(n_entries), cudaMemcpyDeviceToHost, s));
+      RSG_CUDA("upload", cub::DeviceRadixSort::SortPairs(tmp.p, bytes, key, sorted, idx, sched.p, (int)n_items, 0, 20, s));
+      DevBuf<ItemTotals> totals(1);
+      item_totals_kernel<<<1, 32, 0, s>>>((uint32_t)n_items, sorted, base.p + n_items, entries, totals.p);
+      RSG_LAUNCHED(ctx, "hm_item_totals");
+      ItemTotals t;
+      totals.download(&t, 1, s);
       RSG_CUDA("upload", cudaStreamSynchronize(s));
-      if (n_entries > UINT32_MAX || tot > UINT32_MAX)
+      std::copy(t.off, t.off + 9, sched_off);
+      const unsigned long long tot = t.weights;
+      if (t.entries > UINT32_MAX || tot > UINT32_MAX)
         fail(RS_INVALID_OPTION, "InvalidOption", "upload", "near field too large");
       n_wts = 8 * (size_t)tot;
       item_base_kernel<<<nblk(n_items, 256), 256, 0, s>>>((uint32_t)n_items, base.p, items.p);
@@ -1326,7 +1336,10 @@ struct HMat {
     leaf_of.alloc(n_el);
     leaf_of_kernel<<<nblk(nl, 128), 128, 0, s>>>((uint32_t)nl, leaves.p, start.p, end.p, leaf_of.p);
     RSG_LAUNCHED(ctx, "hm_leaf_of");
-    build_groups();
+    std::vector<uint4> groups;
+    std::vector<uint32_t> group_words;  // both live until the stream is waited for below
+    build_groups(groups, group_words);
+    up_vec(grp, groups, s), up_vec(grp_words, group_words, s);
     RSG_CUDA("upload", cudaEventCreateWithFlags(&ev_fork.e, cudaEventDisableTiming));
     RSG_CUDA("upload", cudaEventCreateWithFlags(&ev_join.e, cudaEventDisableTiming));
     // far coefficients (kernel.far, hierarchical.rs:210-220 / 980-984) in FP64 on the device
