@@ -784,6 +784,7 @@ void AmgDevice::launch(rs_ctx *ctx, const mgreal *b, mgreal *x, int iters) {
 
 void AmgDevice::pcg(rs_ctx *ctx, const mgreal *b, mgreal *x, int C, int iters) {
   check();
+  if (C > 12) fail(RS_INTERNAL, "Internal", "preconditioner", "at most 12 multigrid columns");
   switch (C) {
     case 3: launch<3>(ctx, b, x, iters); break;
     case 6: launch<6>(ctx, b, x, iters); break;

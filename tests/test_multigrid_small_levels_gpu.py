@@ -42,3 +42,11 @@ def test_fewer_coarse_rows_than_blocks(ctx, m, k, per_component):
     assert np.isfinite(one).all() and not one[2].any()
     for nb in (2, 3, 4):
         assert np.array_equal(S.precondition(r[:nb]), one[:nb]), nb
+
+
+def test_more_columns_than_the_widest_batch(ctx):
+    P, F = fans(5, 60)
+    S = R.SaddleSolver(F, P, R.Exponents(), R.solver_options(coarse=0), ctx)
+    with pytest.raises(R.RsError) as e:
+        S.precondition(np.zeros((5, S.n)))
+    assert (e.value.kind, e.value.operation, e.value.detail) == ("Internal", "preconditioner", "at most 12 multigrid columns")
