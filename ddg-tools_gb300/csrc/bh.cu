@@ -480,31 +480,60 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &t) {
   t = (a - (s - bv)) + (b - bv);
 }
 
-// Packed FP32: two sources at once. The contractions of these and of the pair terms below are fixed:
-// the energies of earlier builds keep their bits.
-__device__ __forceinline__ f32x2 f2_neg(f32x2 a) { return a ^ kF2Sign; }
-__device__ __forceinline__ void two_sum2(f32x2 a, f32x2 b, f32x2 &s, f32x2 &t) {
+// The terms of a source (T = float) or of two at once in packed FP32 (T = f32x2). The contractions of these and
+// of the pair terms below are fixed: the energies of earlier builds keep their bits.
+template <class T>
+__device__ __forceinline__ void two_sum2(T a, T b, T &s, T &t) {
   s = f2_add(a, b);
-  const f32x2 bv = f2_sub(s, a);
+  const T bv = f2_sub(s, a);
   t = f2_add(f2_sub(a, f2_sub(s, bv)), f2_sub(b, bv));
 }
-template <bool SECOND = false>  // the product that is rounded alone: the first or the second
-__device__ __forceinline__ f32x2 dot3x2(f32x2 a, f32x2 x, f32x2 b, f32x2 y, f32x2 c, f32x2 z) {
+template <bool SECOND = false, class T>  // SECOND: the product that is rounded alone, the first or the second
+__device__ __forceinline__ T dot3x2(T a, T x, T b, T y, T c, T z) {
   return f2_fma(c, z, SECOND ? f2_fma(a, x, f2_mul(b, y)) : f2_fma(b, y, f2_mul(a, x)));
 }
 // N . o for a unit normal and an offset both held as float pairs (hi + lo), compensated
 // (the Dot2 scheme of Ogita, Rump and Oishi, 2005): the sum of the three products carries its
 // rounding errors, which matters because it nearly cancels for a smooth surface.
 // The result is left unrounded as u + lo.
-__device__ __forceinline__ void dot2x2(const f32x2 (&n)[3], const f32x2 (&l)[3], const f32x2 (&o)[3], const f32x2 (&p)[3],
-                                       f32x2 &u, f32x2 &lo) {
-  f32x2 q[3], e[3], s, t0, t1;
+template <class T>
+__device__ __forceinline__ void dot2x2(const T (&n)[3], const T (&l)[3], const T (&o)[3], const T (&p)[3], T &u, T &lo) {
+  T q[3], e[3], s, t0, t1;
 #pragma unroll
   for (int k = 0; k < 3; ++k) q[k] = f2_mul(n[k], o[k]), e[k] = f2_fma(n[k], o[k], f2_neg(q[k]));
   two_sum2(q[0], q[1], s, t0);
   two_sum2(s, q[2], u, t1);
   lo = f2_add(f2_add(f2_add(e[0], e[1]), f2_add(e[2], t0)), t1);
   lo = f2_add(lo, f2_add(dot3x2(n[0], p[0], n[1], p[1], n[2], p[2]), dot3x2(l[0], o[0], l[1], o[1], l[2], o[2])));
+}
+// A lane's target face: X_S - X_L, N_S and alpha_S as float pairs (h + l).
+template <class T>
+struct Target {
+  T Xh[3], Xl[3], Nh[3], Nl[3], ah, al;
+};
+// v, nu and |v|^2 of a target and a lumped node at nd = X_L - X_C
+template <class T>
+__device__ __forceinline__ void lumped_terms(const Target<T> &S, const T (&nd)[3], T (&v)[3], T &nu, T &r2) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) v[k] = f2_add(S.Xh[k], nd[k]);
+  const T u = f2_fma(S.Nh[2], nd[2], f2_fma(S.Nh[1], nd[1], f2_mul(S.Nh[0], nd[0])));
+  nu = f2_add(S.ah, f2_add(u, S.al));
+  r2 = dot3x2<true>(v[0], v[0], v[1], v[1], v[2], v[2]);
+}
+// the same of a target and a face at y = X_T - X_L, a float pair
+template <class T>
+__device__ __forceinline__ void exact_terms(const Target<T> &S, const T (&yh)[3], const T (&yl)[3], T (&v)[3], T &nu, T &r2) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    T w, e;
+    two_sum2(S.Xh[k], f2_neg(yh[k]), w, e);
+    v[k] = f2_add(w, f2_add(e, f2_sub(S.Xl[k], yl[k])));
+  }
+  r2 = dot3x2(v[0], v[0], v[1], v[1], v[2], v[2]);
+  T ph, pl, sh, se;
+  dot2x2(S.Nh, S.Nl, yh, yl, ph, pl);
+  two_sum2(S.ah, f2_neg(ph), sh, se);
+  nu = f2_add(sh, f2_add(se, f2_sub(S.al, pl)));
 }
 // K and c_n of two sources; gg = beta K / r^2
 template <bool FAST>
@@ -538,7 +567,7 @@ __device__ __forceinline__ void pair_diff(const float4 &ah, const float4 &al, co
 }
 
 constexpr int kBatch = 64;
-// the first float of source e in src
+// the first float of source e in src (sources in pairs)
 __device__ __forceinline__ int src_at(int e, int G) {
   const int i = e / G;
   return ((i >> 1) * G + (e - i * G)) * 4 + (i & 1);
@@ -549,8 +578,8 @@ struct PairStage {
   // lumped: per node entry, X_L - X_C rounded to FP32 (xyz) and A_C (w);
   // exact: per source face T, y_T = X_T - X_L as a float pair: hi (xyz) with a_T (w), lo (xyz)
   // with T's slot in the target leaf when C = L, else -1 (w, integer bits)
-  // (hi xyzw, lo xyzw), two sources e and e + G of a group side by side: plane p of pair
-  // (e / G / 2) G + e % G holds components 2 p and 2 p + 1 of both
+  // In pairs: (hi xyzw, lo xyzw), two sources e and e + G of a group side by side: plane p of pair
+  // (e / G / 2) G + e % G holds components 2 p and 2 p + 1 of both. One by one: hi of all, then lo.
   float4 src[4][kBatch / 2];
   uint32_t src_slot[kBatch];            // exact: partner slot of each staged face
   float4 ent_h[32], ent_l[32];          // exact: X_L - X_C of each entry as a float pair
@@ -585,10 +614,10 @@ struct PairStage {
 // 5.15 to 4.64 ms, with the differential at 81,920 faces 0.745 to 0.714 ms.
 //
 // General exponents (two powf a pair): unrolled over two pairs of sources, both loops outgrow the instruction
-// cache. At 204,800 faces and exponents (4.5, 9) / (3, 6), with the differential 8.13 / 5.48 ms unrolled and 5.25 /
-// 3.68 not (5.40 / 3.70 with a source at a time). The value alone has room for the lumped loop unrolled, and gains
-// from six blocks per SM: whole calls 4.53 / 2.53 ms with both loops unrolled and four blocks, 3.88 / 2.34 with five, 3.72 /
-// 2.24 with six (3.64 / 2.40 with a source at a time).
+// cache, so with the differential they are not unrolled: exponents (4.5, 9) / (3, 6), 204,800 faces, 8.13 / 5.48 ms
+// unrolled, 5.18 / 3.66 not, 5.40 / 3.70 with a source at a time. The value alone takes one source at a time with six
+// blocks per SM: whole calls 3.57 / 2.34 ms, in pairs 4.53 / 2.53 unrolled with four blocks and 3.74 / 2.25 at
+// best (lumped loop unrolled, six blocks; 0.325 against 0.311 ms at 20,000 faces).
 //
 // COOP: a block's four warps share a work item, a batch each in turn (every warp finds the
 // batches by itself); the batches' sums go through shared memory and are added in batch order, two of
@@ -596,6 +625,8 @@ struct PairStage {
 // whose time is that of one item: 1,280 faces 55 us with a warp per item.
 template <bool GRAD, bool FAST, bool COOP>
 __global__ void __launch_bounds__(128, FAST || GRAD || COOP ? 4 : 6) bh_pair_kernel(BhDev d, Pow pw) {
+  constexpr bool PAIRS = FAST || GRAD;   // two sources at once
+  constexpr int UNROLL = FAST ? 2 : 1;  // pairs
   __shared__ PairStage stage[4];
   __shared__ float sums[COOP ? 2 : 1][COOP ? 4 : 1][COOP ? 8 : 1][32];
   __shared__ unsigned int next;
@@ -630,11 +661,25 @@ __global__ void __launch_bounds__(128, FAST || GRAD || COOP ? 4 : 6) bh_pair_ker
     const float4 xsl = act ? d.fol[s0 + s] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 cLh = d.nch[leaf], cLl = d.ncl[leaf];
     const float a_s = xs.w;
-    const int at0 = src_at(lane, G), at1 = src_at(lane + 32, G);  // a lane stages sources lane and lane + 32
-    float *const src = reinterpret_cast<float *>(st.src);
-    const f32x2 Xh[3] = {f2_dup(xs.x), f2_dup(xs.y), f2_dup(xs.z)}, Xl[3] = {f2_dup(xsl.x), f2_dup(xsl.y), f2_dup(xsl.z)};
-    const f32x2 Nh[3] = {f2_dup(nS.x), f2_dup(nS.y), f2_dup(nS.z)}, Nl[3] = {f2_dup(nL.x), f2_dup(nL.y), f2_dup(nL.z)};
-    const f32x2 ah = f2_dup(nL.w), al = f2_dup(xsl.w);
+    const Target<float> one = {{xs.x, xs.y, xs.z}, {xsl.x, xsl.y, xsl.z}, {nS.x, nS.y, nS.z}, {nL.x, nL.y, nL.z}, nL.w, xsl.w};
+    Target<f32x2> two;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      two.Xh[k] = f2_dup(one.Xh[k]), two.Xl[k] = f2_dup(one.Xl[k]);
+      two.Nh[k] = f2_dup(one.Nh[k]), two.Nl[k] = f2_dup(one.Nl[k]);
+    }
+    two.ah = f2_dup(one.ah), two.al = f2_dup(one.al);
+    // a source's record into the stage, its hi part (half 0) or lo part (1)
+    float4 *const rec = reinterpret_cast<float4 *>(st.src);
+    const int at0 = src_at(lane, G), at1 = src_at(lane + 32, G);
+    auto put = [&](int e, int half, float x, float y, float z, float w) {
+      if constexpr (PAIRS) {  // a plane per two components
+        float *const o = reinterpret_cast<float *>(rec) + half * (4 * kBatch) + (e < 32 ? at0 : at1);
+        o[0] = x, o[2] = y, o[2 * kBatch] = z, o[2 * kBatch + 2] = w;
+      } else {
+        rec[half * kBatch + e] = make_float4(x, y, z, w);
+      }
+    };
     // the differential's direction of one component, c_n N - gg v
     auto dv2 = [&](f32x2 cn, f32x2 n, f32x2 gg, f32x2 v) {
       return f2_fma(cn, n, f2_neg(f2_mul(gg, v)));
@@ -677,26 +722,33 @@ __global__ void __launch_bounds__(128, FAST || GRAD || COOP ? 4 : 6) bh_pair_ker
         const float4 ch = d.nch[c], cl = d.ncl[c];
         float h[3], l[3];
         pair_diff(cLh, cLl, ch, cl, h, l);
-        const int at = e < 32 ? at0 : at1;  // components 0 and 1, then 2 and 3 in the next plane
-        src[at] = h[0] + l[0], src[at + 2] = h[1] + l[1];
-        src[at + 2 * kBatch] = h[2] + l[2], src[at + 2 * kBatch + 2] = ch.w;
+        put(e, 0, h[0] + l[0], h[1] + l[1], h[2] + l[2], ch.w);
       }
       __syncwarp();
       float bda = 0.f, be = 0.f, bx0 = 0.f, bx1 = 0.f, bx2 = 0.f, bn0 = 0.f, bn1 = 0.f, bn2 = 0.f;
-#pragma unroll (FAST || !GRAD ? 2 : 1)
-      for (int i = 0; i < 4; ++i) {  // sources e and e + G
+      if constexpr (!PAIRS) {
+#pragma unroll 2
+        for (int i = 0; i < 8; ++i) {
+          const int e = g + G * i;
+          if (!act || e >= cnt) continue;
+          const float4 n4 = rec[e];
+          const float nd[3] = {n4.x, n4.y, n4.z};
+          float v[3], nu, r2, K, cn;
+          lumped_terms(one, nd, v, nu, r2);
+          kernel_k<false>(pw, nu, r2, __fdividef(1.f, r2), K, cn);
+          be = __fmaf_rn(__fmul_rn(a_s, K), n4.w, be);
+        }
+      }
+#pragma unroll UNROLL
+      for (int i = 0; i < (PAIRS ? 4 : 0); ++i) {  // sources e and e + G
         const int e = g + 2 * G * i;
         if (!act || e >= cnt) continue;
         const bool both = e + G < cnt;
         const ulonglong2 s0_ = reinterpret_cast<const ulonglong2 *>(st.src[0])[i * G + g];
         const ulonglong2 s1_ = reinterpret_cast<const ulonglong2 *>(st.src[1])[i * G + g];
         const f32x2 nd[3] = {s0_.x, s0_.y, s1_.x}, Ac = s1_.y;
-        f32x2 v[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) v[k] = f2_add(Xh[k], nd[k]);
-        const f32x2 u = f2_fma(Nh[2], nd[2], f2_fma(Nh[1], nd[1], f2_mul(Nh[0], nd[0])));
-        const f32x2 nu = f2_add(ah, f2_add(u, al));
-        const f32x2 r2 = dot3x2<true>(v[0], v[0], v[1], v[1], v[2], v[2]);
+        f32x2 v[3], nu, r2;
+        lumped_terms(two, nd, v, nu, r2);
         f32x2 K, cn, gg;
         kernel_k2<FAST>(pw, nu, r2, K, cn, gg);
         const f32x2 A = f2_dup(a_s), aK = f2_mul(A, K);
@@ -707,7 +759,7 @@ __global__ void __launch_bounds__(128, FAST || GRAD || COOP ? 4 : 6) bh_pair_ker
           const f32x2 aa = f2_mul(A, Ac), ac = f2_mul(aa, cn);
           float2 d[3], w[3];
 #pragma unroll
-          for (int k = 0; k < 3; ++k) d[k] = f2_unpack(dv2(cn, Nh[k], gg, v[k])), w[k] = f2_unpack(v[k]);
+          for (int k = 0; k < 3; ++k) d[k] = f2_unpack(dv2(cn, two.Nh[k], gg, v[k])), w[k] = f2_unpack(v[k]);
           const float2 K_ = f2_unpack(K), aa_ = f2_unpack(aa), ac_ = f2_unpack(ac);
           bda = __fmaf_rn(K_.x, Ac_.x, bda);
           bx0 = __fmaf_rn(aa_.x, d[0].x, bx0), bx1 = __fmaf_rn(aa_.x, d[1].x, bx1), bx2 = __fmaf_rn(aa_.x, d[2].x, bx2);
@@ -779,18 +831,29 @@ __global__ void __launch_bounds__(128, FAST || GRAD || COOP ? 4 : 6) bh_pair_ker
           two_sum(xt.x, -hh.x, y0, e0);
           two_sum(xt.y, -hh.y, y1, e1);
           two_sum(xt.z, -hh.z, y2, e2);
-          const int at = f < 32 ? at0 : at1;  // a plane per two components
-          src[at] = y0, src[at + 2] = y1;
-          src[at + 2 * kBatch] = y2, src[at + 2 * kBatch + 2] = xt.w;
-          src[at + 4 * kBatch] = e0 + (xl.x - ll.x), src[at + 4 * kBatch + 2] = e1 + (xl.y - ll.y);
-          src[at + 6 * kBatch] = e2 + (xl.z - ll.z);
-          src[at + 6 * kBatch + 2] = __int_as_float(__float_as_int(ll.w) ? (int)t : -1);
+          put(f, 0, y0, y1, y2, xt.w);
+          put(f, 1, e0 + (xl.x - ll.x), e1 + (xl.y - ll.y), e2 + (xl.z - ll.z),
+              __int_as_float(__float_as_int(ll.w) ? (int)t : -1));
           st.src_slot[f] = st.ent_po[i] + t;
         }
         __syncwarp();
         float row = 0.f, rx0 = 0.f, rx1 = 0.f, rx2 = 0.f, rn0 = 0.f, rn1 = 0.f, rn2 = 0.f;
-#pragma unroll (FAST ? 2 : 1)
-        for (int i = 0; i < 4; ++i) {  // sources f and f + G
+        if constexpr (!PAIRS) {
+#pragma unroll 2
+          for (int i = 0; i < 8; ++i) {
+            const int f = g + G * i;
+            if (!act || f >= cnt) continue;
+            const float4 h4 = rec[f], l4 = rec[kBatch + f];
+            if (__float_as_int(l4.w) == s) continue;  // the face itself: no terms
+            const float yh[3] = {h4.x, h4.y, h4.z}, yl[3] = {l4.x, l4.y, l4.z};
+            float v[3], nu, r2, K, cn;
+            exact_terms(one, yh, yl, v, nu, r2);
+            kernel_k<false>(pw, nu, r2, __fdividef(1.f, r2), K, cn);
+            row = __fmaf_rn(h4.w, K, row);
+          }
+        }
+#pragma unroll UNROLL
+        for (int i = 0; i < (PAIRS ? 4 : 0); ++i) {  // sources f and f + G
           const int f = g + 2 * G * i;
           if (!act || f >= cnt) continue;
           const bool both = f + G < cnt;
@@ -798,18 +861,8 @@ __global__ void __launch_bounds__(128, FAST || GRAD || COOP ? 4 : 6) bh_pair_ker
 #pragma unroll
           for (int p = 0; p < 4; ++p) sp[p] = reinterpret_cast<const ulonglong2 *>(st.src[p])[i * G + g];
           const f32x2 yh[3] = {sp[0].x, sp[0].y, sp[1].x}, yl[3] = {sp[2].x, sp[2].y, sp[3].x}, at2 = sp[1].y;
-          f32x2 v[3];
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            f32x2 w, e;
-            two_sum2(Xh[k], f2_neg(yh[k]), w, e);
-            v[k] = f2_add(w, f2_add(e, f2_sub(Xl[k], yl[k])));
-          }
-          const f32x2 r2 = dot3x2(v[0], v[0], v[1], v[1], v[2], v[2]);
-          f32x2 ph, pl, sh, se, K, cn, gg;
-          dot2x2(Nh, Nl, yh, yl, ph, pl);
-          two_sum2(ah, f2_neg(ph), sh, se);
-          const f32x2 nu = f2_add(sh, f2_add(se, f2_sub(al, pl)));
+          f32x2 v[3], nu, r2, K, cn, gg;
+          exact_terms(two, yh, yl, v, nu, r2);
           kernel_k2<FAST>(pw, nu, r2, K, cn, gg);
           // the face itself: no terms
           const float2 slot = f2_unpack(sp[3].y);
@@ -829,7 +882,7 @@ __global__ void __launch_bounds__(128, FAST || GRAD || COOP ? 4 : 6) bh_pair_ker
             float2 d[3], w[3], b[3];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-              const f32x2 dk = dv2(cn, Nh[k], gg, v[k]);
+              const f32x2 dk = dv2(cn, two.Nh[k], gg, v[k]);
               d[k] = f2_unpack(dk), w[k] = f2_unpack(v[k]), b[k] = f2_unpack(f2_mul(aa, dk));
             }
             const float2 tc_ = f2_unpack(tc), aK = f2_unpack(f2_mul(f2_dup(a_s), K));
@@ -1274,7 +1327,6 @@ Pow make_pow(double alpha, double beta) {
   p.alpha = (float)alpha;
   p.beta = (float)beta;
   p.a_int = (alpha == std::trunc(alpha) && alpha >= 2 && alpha <= 64) ? (int)alpha : -1;
-  p.q_exp = 0.5f * p.alpha - 1.f, p.r_exp = 0.5f * (p.alpha - p.beta);
   double ab = beta - alpha;
   p.ab_int = (ab == std::trunc(ab) && ab >= 0 && ab <= 128) ? (int)ab : -1;
   return p;

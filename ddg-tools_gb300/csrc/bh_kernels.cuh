@@ -77,7 +77,6 @@ struct Pow {
   float alpha, beta;
   int a_int;   // alpha as an integer, or -1
   int ab_int;  // beta - alpha as an integer, or -1
-  float q_exp, r_exp;  // alpha / 2 - 1 and (alpha - beta) / 2
 };
 
 // q^(alpha/2 - 1): (alpha - 2)/2 = h, integer or half-integer for integer alpha.
@@ -94,7 +93,7 @@ __device__ __forceinline__ float pow_q1(const Pow &p, float q) {
     if (m & 1) acc *= sqrtf(q);
     return acc;
   }
-  return q > 0.f ? powf(q, p.q_exp) : 0.f;
+  return q > 0.f ? powf(q, 0.5f * p.alpha - 1.f) : 0.f;
 }
 
 // r2^((alpha-beta)/2) = ir2^((beta-alpha)/2)
@@ -111,7 +110,7 @@ __device__ __forceinline__ float pow_r(const Pow &p, float r2, float ir2) {
     if (m & 1) acc *= rsqrtf(r2);
     return acc;
   }
-  return powf(r2, p.r_exp);
+  return powf(r2, 0.5f * (p.alpha - p.beta));
 }
 
 // K and c_n for (alpha, beta) = (6, 12) (FAST) or the general exponents.

@@ -37,6 +37,14 @@ __device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
   return r;
 }
 constexpr f32x2 kF2Sign = 0x8000000080000000ull;  // both halves' sign bits
+__device__ __forceinline__ f32x2 f2_neg(f32x2 a) { return a ^ kF2Sign; }
+// The same on one value, for code written for either. Sums rounded to nearest are never contracted with the
+// product before them, so the product needs no such form (with __fmul_rn the energy's value takes 4 % longer).
+__device__ __forceinline__ float f2_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float f2_sub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float f2_mul(float a, float b) { return a * b; }
+__device__ __forceinline__ float f2_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float f2_neg(float a) { return -a; }
 __device__ __forceinline__ f32x2 f2_dup(float a) { return f2_pack(a, a); }
 
 }  // namespace rsg
