@@ -93,7 +93,7 @@ struct alignas(4 * V) Floats {
 // out[v][c] = mean over the one-ring of in[u][c]. A thread takes V channels (widths that are a multiple
 // of four: 16-byte loads, and the ring's offsets and indices found a quarter as often: at 102,400
 // vertices and 64 channels 52 us with a thread per channel, 19 with this).
-template <int V>
+template <int V, int UNROLL>
 __global__ void __launch_bounds__(256) ring_mean(int nv, int W, const uint32_t *__restrict__ off,
                                                  const uint32_t *__restrict__ idx, const float *__restrict__ in,
                                                  float *__restrict__ out) {
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(256) ring_mean(int nv, int W, const uint32_t *
   const int v = (int)(t / G), c = (int)(t % G) * V;
   const uint32_t a = off[v], b = off[v + 1];
   Floats<V> s = {};
-#pragma unroll 4
+#pragma unroll UNROLL
   for (uint32_t p = a; p < b; ++p) {
     const Floats<V> x = *reinterpret_cast<const Floats<V> *>(in + (size_t)idx[p] * W + c);
 #pragma unroll
@@ -115,20 +115,20 @@ __global__ void __launch_bounds__(256) ring_mean(int nv, int W, const uint32_t *
 }
 
 // dh[u][c] += sum over v in N(u) of dnb[v][c] / deg(v)   (transpose of ring_mean; the mesh
-// one-ring is symmetric), and the gradient before the activation, dpre = dh silu'(pre); four channels a thread
-// (102,400 vertices: 80 us, and 22 for the activation in a pass of its own, before; 35 together).
+// one-ring is symmetric), and the gradient before the activation, dpre = dh silu'(pre); four channels a thread,
+// or one (see rs_lgraph; 102,400 vertices: 80 us with one, and 22 for the activation in a pass of its own; 35 together).
+template <int V>
 __global__ void __launch_bounds__(256) ring_mean_bwd(int nv, int W, const uint32_t *__restrict__ off,
                                                      const uint32_t *__restrict__ idx, const float *__restrict__ dnb,
                                                      const float *__restrict__ dh, const float *__restrict__ pre,
                                                      float *__restrict__ dpre) {
-  constexpr int V = 4;
   const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const unsigned G = (unsigned)W / V;
   if (t >= (size_t)nv * G) return;
   const int u = (int)(t / G), c = (int)(t % G) * V;
   Floats<V> s = {};
   const uint32_t b = off[u + 1];
-#pragma unroll 4
+#pragma unroll (V == 1 ? 8 : 4)
   for (uint32_t p = off[u]; p < b; ++p) {
     const uint32_t v = idx[p];
     const float dv = (float)(off[v + 1] - off[v]);
@@ -483,6 +483,12 @@ struct rs_lgraph {
   int nv = 0;
   DevBuf<uint32_t> off, idx;
   DevBuf<float> stat7;
+  // Four channels a thread in the ring means, except where a long ring outlasts the rest: a thread adds its ring
+  // one after another, 37 ns a neighbour more with four channels, against 0.3 ns a vertex saved; with one it
+  // looks eight neighbours ahead.
+  // Forward, 501 vertices with a hub of 500 neighbours: 150 us with one channel, 220 with four; 40 of these side by side:
+  // 184 / 269; 102,400 vertices of six neighbours: 240 / 180.
+  bool four = true;
 };
 
 namespace rsg {
@@ -504,8 +510,9 @@ void forward(rs_learned *M, rs_lgraph *G, const double *r, const double *y, bool
   RSG_LAUNCHED(ctx, "learned_features");
   const __nv_bfloat16 *wb = M->wb.p;
   auto mean = [&](int W, const float *in, float *out) {
-    if (W % 4 == 0) ring_mean<4><<<nblk((size_t)nv * (W / 4), 256), 256, 0, s>>>(nv, W, G->off.p, G->idx.p, in, out);
-    else ring_mean<1><<<nblk((size_t)nv * W, 256), 256, 0, s>>>(nv, W, G->off.p, G->idx.p, in, out);
+    const int V = W % 4 == 0 && G->four ? 4 : 1;
+    (V == 4 ? ring_mean<4, 4> : G->four ? ring_mean<1, 4> : ring_mean<1, 8>)<<<nblk((size_t)nv * (W / V), 256), 256, 0, s>>>(
+        nv, W, G->off.p, G->idx.p, in, out);
     RSG_LAUNCHED(ctx, "learned_mean");
   };
   mean(kIn, M->X.p, M->nX.p);
@@ -653,6 +660,9 @@ int rs_lgraph_create(rs_ctx *ctx, int nv, int nf, const uint32_t *faces, const d
       off[v + 1] = off[v] + (uint32_t)l.size();
       idx.insert(idx.end(), l.begin(), l.end());
     }
+    uint32_t longest = 0;
+    for (int v = 0; v < nv; ++v) longest = std::max(longest, off[v + 1] - off[v]);
+    G->four = longest <= 64 || longest <= (uint32_t)nv / 128;
     // static features: centred / RMS-radius positions, unit area-weighted normals, dual area
     FaceGeom g = face_geometry(nf, faces, positions_host);
     std::vector<double> nrm(3 * (size_t)nv, 0.0), area(nv, 0.0);
@@ -732,18 +742,21 @@ int rs_learned_loss_and_gradient_device(rs_learned *M, rs_lgraph *G, const doubl
     dense_bwd_in<64, kOut><<<nblk(nv, 64), 128, 0, s>>>(nv, wb + M->o3s, wb + M->o3n, M->dpre.p,
                                                                       M->dself.p, M->dnb.p);
     RSG_LAUNCHED(ctx, "learned_bwd_in");
+    // the transposed ring mean of a layer's input gradient, up to its pre-activation
+    auto mean_bwd = [&](const float *pre) {
+      const int V = G->four ? 4 : 1;
+      (V == 4 ? ring_mean_bwd<4> : ring_mean_bwd<1>)<<<nblk((size_t)nv * (H / V), 256), 256, 0, s>>>(
+          nv, H, G->off.p, G->idx.p, M->dnb.p, M->dself.p, pre, M->dpre.p);
+      RSG_LAUNCHED(ctx, "learned_mean_bwd");
+    };
     // dh2 = dself + mean^T(dnb)
-    ring_mean_bwd<<<nblk((size_t)nv * (H / 4), 256), 256, 0, s>>>(nv, H, G->off.p, G->idx.p, M->dnb.p, M->dself.p, M->pre2.p,
-                                                                  M->dpre.p);
-    RSG_LAUNCHED(ctx, "learned_mean_bwd");
+    mean_bwd(M->pre2.p);
     // layer 2
     layer_grad<64, 64>(M, nv, M->h1.p, M->nh1.p, M->o2s);
     dense_bwd_in<64, 64><<<nblk(nv, 64), 128, 0, s>>>(nv, wb + M->o2s, wb + M->o2n, M->dpre.p,
                                                                     M->dself.p, M->dnb.p);
     RSG_LAUNCHED(ctx, "learned_bwd_in");
-    ring_mean_bwd<<<nblk((size_t)nv * (H / 4), 256), 256, 0, s>>>(nv, H, G->off.p, G->idx.p, M->dnb.p, M->dself.p, M->pre1.p,
-                                                                  M->dpre.p);
-    RSG_LAUNCHED(ctx, "learned_mean_bwd");
+    mean_bwd(M->pre1.p);
     // layer 1
     layer_grad<kIn, 64>(M, nv, M->X.p, M->nX.p, M->o1s);
     std::vector<double> lp(kChunks);
